@@ -1,0 +1,588 @@
+// dense_panel.cu -- dense row-major product with several right-hand sides:
+// one pass over A for up to kPanelCols of them.
+//
+// What bounds it: A streams once from HBM (k is small), but every element of A
+// meets k elements of X, so the operand path from shared memory to registers
+// and the FMA pipes run close to the HBM rate as well (20 right-hand sides:
+// 10 flop per byte of an f32 A, 5 of an f64 A).  Reading A once per block of
+// eight right-hand sides, as a gemv repeated over column blocks does, costs
+// ceil(k / 8) passes over HBM, and rows that do not start on 16 bytes went
+// through single-element loads with few of them in flight.
+//
+// Measured (us): 5003 x 3001 f64 with 20 right-hand sides 246 -> 57, f32 428 -> 47;
+// 8192^2 f32 with 20 336 -> 116, with 8 143 -> 78, with 4 61 -> 62; 4096 x 8192
+// f64 with 32 428 -> 103.
+//
+// Tiles and split.  A CTA of 16 warps owns a tile of BM rows and walks along the
+// columns in chunks of KC; the chunks of A and of X come through a
+// STAGES-deep cp.async ring in 16-byte pieces.  Where rows of A or columns of X
+// do not start on 16 bytes (odd sizes), a row is copied from the boundary below
+// its start and read from its own offset in shared memory: copies of single
+// elements ran at a third of the speed.  All chunks of all tiles form one list
+// that is cut into equal consecutive shares, one per CTA, so the chip is full
+// whatever the shape; a tile cut between CTAs leaves one partial per CTA, and
+// panel_sum adds them in chunk order (deterministic).
+//
+//   f32: a warp has R rows; a lane takes every 16th column of A and one half of
+//        the right-hand sides: R x C/2 sums per lane (an X value read from shared
+//        memory serves R rows, an A value C/2 right-hand sides), so the FMA pipes
+//        and the shared-memory path are about equally busy.  The lanes' sums
+//        meet in a halving tree at the end of a tile.  Scalar fused multiply-adds:
+//        the packed f32x2 form kept the pipe busy for four cycles each, half the
+//        scalar rate.
+//   f64: mma.sync m8n8k4: a warp has 16 rows x 8 NT right-hand sides and one
+//        half of each chunk's columns (the halves meet in shared memory at the
+//        end of a tile): 16 warps keep the tensor pipe fed where 8 left it idle
+//        half the time.  CUDA cores would need 2 (R + C) shared-memory cycles
+//        for R C fused multiply-adds at half rate, and 4 R C registers.
+#include <algorithm>
+
+#include "drb_internal.cuh"
+
+namespace drb {
+namespace {
+
+constexpr int kNT = 512;
+constexpr int kWarps = kNT / 32;
+constexpr int kPanelCols = 32; // right-hand sides of one pass
+constexpr int64_t kTurnElems = (int64_t)1 << 21; // A above this: row-major X is transposed first
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+// BYTES from global to shared memory, the last BYTES - n of them zeros.
+template <int BYTES>
+__device__ __forceinline__ void cp_zfill(uint32_t dst, const void *src, int n = BYTES) {
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n)
+                 : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(n),
+                 "n"(BYTES)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N> __device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+struct PanelArgs {
+  const void *A;
+  const void *x;
+  void *y;
+  void *part; // [CTA][2][BM][CP] partial sums of cut tiles
+  int64_t m, n, lda;
+  int64_t x_cs, x_js; // address of X(c, j): c * x_cs + j * x_js
+  int64_t y_ld, y_js; // address of Y(r, j): r * y_ld + j * y_js
+  int k;
+  int64_t cpt, chunks, share; // chunks per tile, in all, per CTA
+};
+
+// Tile shapes: BM rows, KC columns a chunk, AS / XS elements between the rows of
+// a staged A / X chunk: a 16-byte multiple with room for the offset of a
+// shifted row.  The rows of one shared-memory load hit different banks: f32
+// right-hand sides of the two half-warps are 64 bytes apart modulo 128, f64 rows
+// 64 bytes for the 16-byte fragment loads of aligned rows and 32 bytes for the
+// 8-byte loads of shifted ones.
+template <class V, int P, bool SH> struct Shape;
+template <int C, bool SH> struct Shape<float, C, SH> { // C right-hand sides
+  static constexpr int R = C <= 20 ? 8 : 4;
+  static constexpr int BM = kWarps * R, KC = 64, AS = KC + 4, XS = KC + 16, CP = C;
+  static constexpr int STAGES = 4, MERGE = 0;
+};
+template <int NT, bool SH> struct Shape<double, NT, SH> { // 8 NT right-hand sides
+  static constexpr int R = 16;
+  static constexpr int BM = kWarps / 2 * R, KC = 32, AS = KC + (SH ? 4 : 8), XS = AS, CP = 8 * NT;
+  static constexpr int STAGES = NT == 4 && !SH ? 3 : 4;
+  static constexpr int MERGE = BM * CP; // the second half's sums of a tile
+};
+template <class V, int P, bool SH> constexpr size_t panel_smem() {
+  using S = Shape<V, P, SH>;
+  return ((size_t)S::STAGES * (S::BM * S::AS + S::CP * S::XS) + S::MERGE) * sizeof(V);
+}
+
+// Elements from the 16-byte boundary at or below p to p.
+template <class V> __device__ __forceinline__ int shift_of(const V *p) {
+  return (int)((reinterpret_cast<uintptr_t>(p) & 15) / sizeof(V));
+}
+
+// One 16-byte piece of a shifted row: element e0 of the row (kb - its offset +
+// a multiple of a piece) lands at dst.  Zeros from element n on; elements below
+// kb are not wanted.  [lo, hi) is the whole array: a piece that reaches
+// outside it is copied element by element.
+template <class V>
+__device__ __forceinline__ void copy_edge_piece(uint32_t dst, const V *row, int64_t e0, int64_t kb,
+                                                int64_t n, const V *lo, const V *hi) {
+  constexpr int PER = 16 / (int)sizeof(V);
+  const V *src = row + e0;
+  if (e0 >= n) {
+    // (nothing is read, but the address has to be a piece's)
+    cp_zfill<16>(dst, reinterpret_cast<const void *>(reinterpret_cast<uintptr_t>(lo) & ~(uintptr_t)15),
+                 0);
+  } else if (src >= lo && src + PER <= hi) {
+    cp_zfill<16>(dst, src, (int)min((int64_t)PER, n - e0) * (int)sizeof(V));
+  } else {
+    for (int i = 0; i < PER; i++)
+      if (e0 + i >= kb)
+        cp_zfill<sizeof(V)>(dst + i * (uint32_t)sizeof(V), e0 + i < n ? src + i : lo,
+                            e0 + i < n ? (int)sizeof(V) : 0);
+  }
+}
+
+template <class V, int P, bool SH>
+__global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
+  using S = Shape<V, P, SH>;
+  constexpr int BM = S::BM, KC = S::KC, AS = S::AS, XS = S::XS, CP = S::CP, ST = S::STAGES;
+  constexpr int PER = 16 / (int)sizeof(V), GR = KC / PER, RP = kNT / GR;
+  extern __shared__ __align__(16) unsigned char panel_mem[];
+  V *sa = reinterpret_cast<V *>(panel_mem);
+  V *sx = sa + (size_t)ST * BM * AS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const V *A = static_cast<const V *>(a.A);
+  const V *X = static_cast<const V *>(a.x);
+  const V *Aend = A + (a.m - 1) * a.lda + a.n;
+  const V *Xend = X + (a.k - 1) * a.x_js + a.n;
+  const int64_t c0 = (int64_t)blockIdx.x * a.share, c1 = min(a.chunks, c0 + a.share);
+  const int cpt = (int)a.cpt;
+
+  // The next chunk of the share -> ring slot st.  A thread's piece column is
+  // fixed and its rows step by a constant, so a whole chunk costs one address
+  // addition per piece.
+  const int ar = tid / GR, ag = (tid % GR) * PER; // first row, piece column
+  int64_t lt = c0 / cpt;                           // tile and chunk of the next load
+  int lc = (int)(c0 - lt * cpt);
+  auto load = [&](int st) {
+    const int64_t kb = (int64_t)lc * KC, r0 = lt * BM;
+    // every piece lies in A (shifted rows: also what precedes the first one
+    // and follows the last)
+    const bool inside =
+        kb + KC <= a.n && r0 + BM <= a.m &&
+        (!SH || ((lt > 0 || lc > 0) && (r0 + BM < a.m || kb + KC + PER <= a.n)));
+    if (++lc == cpt) {
+      lc = 0;
+      lt++;
+    }
+    const uint32_t s0 = smem_u32(sa + (size_t)st * BM * AS);
+    const uint32_t da = s0 + (uint32_t)((ar * AS + ag) * sizeof(V));
+    const V *row = A + (r0 + ar) * a.lda;
+    const int64_t step = RP * a.lda;
+    if (inside) {
+      const V *src = row + kb + ag;
+#pragma unroll
+      for (int p = 0; p < BM / RP; p++, src += step)
+        cp_zfill<16>(da + (uint32_t)(p * RP * AS * sizeof(V)), SH ? src - shift_of(src) : src);
+    } else {
+#pragma unroll 1
+      for (int p = 0; p < BM / RP; p++, row += step)
+        if (r0 + ar + p * RP < a.m)
+          copy_edge_piece<V>(da + (uint32_t)(p * RP * AS * sizeof(V)), row,
+                             kb + ag - (SH ? shift_of(row) : 0), kb, a.n, A, Aend);
+    }
+    if (SH && tid < BM && r0 + tid < a.m) { // the piece past the chunk
+      const V *rw = A + (r0 + tid) * a.lda;
+      const int sh = shift_of(rw);
+      if (sh > 0) {
+        const uint32_t d = s0 + (uint32_t)((tid * AS + KC) * sizeof(V));
+        if (inside)
+          cp_zfill<16>(d, rw + kb + KC - sh);
+        else
+          copy_edge_piece<V>(d, rw, kb + KC - sh, kb, a.n, A, Aend);
+      }
+    }
+    const uint32_t dx = smem_u32(sx + (size_t)st * CP * XS);
+    if (a.x_cs == 1) {
+      const bool xin = SH ? kb > 0 && kb + KC + PER <= a.n : kb + KC <= a.n;
+      for (int j = ar; j < a.k; j += RP) {
+        const V *xc = X + j * a.x_js;
+        const int64_t e0 = kb + ag - (SH ? shift_of(xc) : 0);
+        const uint32_t d = dx + (uint32_t)((j * XS + ag) * sizeof(V));
+        if (xin)
+          cp_zfill<16>(d, xc + e0);
+        else
+          copy_edge_piece<V>(d, xc, e0, kb, a.n, X, Xend);
+      }
+      if (SH && tid < a.k) {
+        const V *xc = X + tid * a.x_js;
+        const int sh = shift_of(xc);
+        const uint32_t d = dx + (uint32_t)((tid * XS + KC) * sizeof(V));
+        if (sh > 0 && xin)
+          cp_zfill<16>(d, xc + kb + KC - sh);
+        else if (sh > 0)
+          copy_edge_piece<V>(d, xc, kb + KC - sh, kb, a.n, X, Xend);
+      }
+    } else { // row-major X: 32-byte runs of right-hand sides, few bank conflicts
+      constexpr int JL = 32 / (int)sizeof(V), CL = 32 / JL; // lanes over j, over c
+      const int kn = (int)min((int64_t)KC, a.n - kb);
+      const int jl = lane % JL;
+      for (int c = warp * CL + lane / JL; c < KC; c += kWarps * CL)
+        for (int j = jl; j < a.k; j += JL)
+          cp_zfill<sizeof(V)>(dx + (uint32_t)((j * XS + c) * sizeof(V)),
+                              c < kn ? X + (kb + c) * a.x_cs + j : X,
+                              c < kn ? (int)sizeof(V) : 0);
+    }
+  };
+  // offset of column j of a staged X chunk (columns PER apart share it)
+  auto xshift = [&](int j) { return SH && a.x_cs == 1 ? shift_of(X + j * a.x_js) : 0; };
+
+  // first row of this warp; f64: its half of a chunk's columns
+  const int wr = (sizeof(V) == 4 ? warp : warp % (kWarps / 2)) * S::R;
+  const int kh = sizeof(V) == 4 ? 0 : warp / (kWarps / 2) * (KC / 2);
+  // this thread's sums of the current tile
+  constexpr int R = S::R;
+  constexpr int NACC = sizeof(V) == 4 ? R * CP / 2 : 2 * (CP / 8);
+  float accf[sizeof(V) == 4 ? NACC : 1];
+  double accd[sizeof(V) == 8 ? NACC : 1][2];
+  auto clear = [&]() {
+    if constexpr (sizeof(V) == 4) {
+#pragma unroll
+      for (int i = 0; i < NACC; i++)
+        accf[i] = 0.0f;
+    } else {
+#pragma unroll
+      for (int i = 0; i < NACC; i++)
+        accd[i][0] = accd[i][1] = 0.0;
+    }
+  };
+  auto compute = [&](int st, int64_t tile) {
+    const V *As = sa + (size_t)st * BM * AS + wr * AS;
+    const V *Xs = sx + (size_t)st * CP * XS;
+    if constexpr (sizeof(V) == 4) {
+      constexpr int CH = CP / 2;
+      const int cg = lane >> 4; // the lane has right-hand sides cg, cg + 2, ...
+      int ra[R], xj[2];         // where its rows and columns start
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        ra[r] = r * AS + (SH ? shift_of(A + (tile * BM + wr + r) * a.lda) : 0);
+#pragma unroll
+      for (int q = 0; q < 2; q++)
+        xj[q] = cg * XS + xshift(cg + 2 * q); // (columns four apart share an offset)
+#pragma unroll 2
+      for (int c = lane & 15; c < KC; c += 16) {
+        float av[R];
+#pragma unroll
+        for (int r = 0; r < R; r++)
+          av[r] = As[ra[r] + c];
+#pragma unroll
+        for (int j = 0; j < CH; j++) {
+          const float xv = Xs[2 * j * XS + xj[j % 2] + c];
+#pragma unroll
+          for (int r = 0; r < R; r++)
+            accf[r * CH + j] = fmaf(av[r], xv, accf[r * CH + j]);
+        }
+      }
+    } else {
+      constexpr int NT = CP / 8;
+      const int fr = lane >> 2;
+      // k order inside a step of eight: a lane's pair (aligned rows) or the
+      // lane's column of either half (shifted rows); the same for A and X
+      const int fk = SH ? (lane & 3) : 2 * (lane & 3);
+      const V *Ap[2], *Xp = Xs + fr * XS + fk + xshift(fr) + kh; // 8 columns on: the same offset
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+        Ap[i] = As + (i * 8 + fr) * AS + fk + kh +
+                (SH ? shift_of(A + (tile * BM + wr + i * 8 + fr) * a.lda) : 0);
+#pragma unroll
+      for (int c = 0; c < KC / 2; c += 8) {
+        double2 av[2], bv[NT];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          if constexpr (SH)
+            av[i] = make_double2(Ap[i][c], Ap[i][c + 4]);
+          else
+            av[i] = *reinterpret_cast<const double2 *>(Ap[i] + c);
+        }
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          if constexpr (SH)
+            bv[t] = make_double2(Xp[t * 8 * XS + c], Xp[t * 8 * XS + c + 4]);
+          else
+            bv[t] = *reinterpret_cast<const double2 *>(Xp + t * 8 * XS + c);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int t = 0; t < NT; t++)
+            dmma(accd[i * NT + t], av[i].x, bv[t].x);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int t = 0; t < NT; t++)
+            dmma(accd[i * NT + t], av[i].y, bv[t].y);
+      }
+    }
+  };
+  // the tile's sums to Y (all its chunks were this CTA's) or to the partials
+  auto emit = [&](int64_t tile) {
+    const int64_t t0 = tile * cpt, t1 = t0 + cpt;
+    const bool whole = t0 >= c0 && t1 <= c1;
+    V *P0 = static_cast<V *>(a.part) +
+            ((int64_t)blockIdx.x * 2 + (tile == c0 / cpt ? 0 : 1)) * BM * CP;
+    V *Y = static_cast<V *>(a.y);
+    auto put = [&](int r, int j, V v) {
+      if (!whole)
+        P0[r * CP + j] = v;
+      else if (tile * BM + r < a.m && j < a.k)
+        Y[(tile * BM + r) * a.y_ld + j * a.y_js] = v;
+    };
+    if constexpr (sizeof(V) == 4) {
+      constexpr int CH = CP / 2, N = R * CH;
+      static_assert(N % 16 == 0, "the halving tree needs a multiple of 16 sums");
+      // each step a lane keeps one half of its sums and passes the other on
+#pragma unroll
+      for (int s = 0; s < 4; s++) {
+        const int off = 8 >> s, h = N >> (s + 1);
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < N / 2; i++)
+          if (i < h) {
+            const float keep = up ? accf[i + h] : accf[i], send = up ? accf[i] : accf[i + h];
+            accf[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+          }
+      }
+      int f0 = 0;
+#pragma unroll
+      for (int s = 0; s < 4; s++)
+        if (lane & (8 >> s))
+          f0 += N >> (s + 1);
+#pragma unroll
+      for (int i = 0; i < N / 16; i++)
+        put(wr + (f0 + i) / CH, (lane >> 4) + 2 * ((f0 + i) % CH), accf[i]);
+    } else {
+      // the second half's warps hand their sums over
+      constexpr int NT = CP / 8;
+      double *mine = sx + (size_t)ST * CP * XS + wr * CP;
+      auto at = [&](int i, int t, int e) {
+        return (i * 8 + (lane >> 2)) * CP + t * 8 + 2 * (lane & 3) + e;
+      };
+      if (kh) {
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int t = 0; t < NT; t++)
+            *reinterpret_cast<double2 *>(mine + at(i, t, 0)) =
+                make_double2(accd[i * NT + t][0], accd[i * NT + t][1]);
+      }
+      __syncthreads();
+      if (!kh) {
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int t = 0; t < NT; t++)
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+              put(wr + i * 8 + (lane >> 2), t * 8 + 2 * (lane & 3) + e,
+                  accd[i * NT + t][e] + mine[at(i, t, e)]);
+      }
+    }
+  };
+
+#pragma unroll
+  for (int s = 0; s < ST - 1; s++) {
+    if (c0 + s < c1)
+      load(s);
+    cp_commit();
+  }
+  clear();
+  int st = 0;
+  int64_t ct = c0 / cpt;                      // current tile
+  int left = cpt - (int)(c0 - ct * cpt);      // chunks left in it
+  for (int64_t q = c0; q < c1; q++) {
+    cp_wait<ST - 2>();
+    __syncthreads(); // chunk q landed; slot st - 1 is free
+    const int fill = st == 0 ? ST - 1 : st - 1;
+    if (q + ST - 1 < c1)
+      load(fill);
+    cp_commit();
+    compute(st, ct);
+    if (--left == 0 || q + 1 == c1) {
+      emit(ct);
+      clear();
+      left = cpt;
+      ct++;
+    }
+    st = st + 1 == ST ? 0 : st + 1;
+  }
+  cp_wait<0>();
+}
+
+// Y of the tiles cut between CTAs: their partials added in chunk order.
+template <class V>
+__global__ void panel_sum(const PanelArgs a, int BM, int CP) {
+  const V *part = static_cast<const V *>(a.part);
+  V *Y = static_cast<V *>(a.y);
+  const int64_t nth = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.m * a.k; i += nth) {
+    int64_t r;
+    int j;
+    if (a.y_ld == 1) { // consecutive threads write consecutive addresses
+      j = (int)(i / a.m);
+      r = i - (int64_t)j * a.m;
+    } else {
+      r = i / a.k;
+      j = (int)(i - r * a.k);
+    }
+    const int64_t tile = r / BM;
+    const int64_t b0 = tile * a.cpt / a.share, b1 = ((tile + 1) * a.cpt - 1) / a.share;
+    if (b0 == b1)
+      continue; // one CTA had the whole tile
+    V s = 0;
+    for (int64_t b = b0; b <= b1; b++) {
+      const int slot = tile == b * a.share / a.cpt ? 0 : 1;
+      s += part[((b * 2 + slot) * BM + (r - tile * BM)) * CP + j];
+    }
+    Y[r * a.y_ld + j * a.y_js] = s;
+  }
+}
+
+template <class V, int P, bool SH> drb_status panel_run(PanelArgs a, cudaStream_t s) {
+  using S = Shape<V, P, SH>;
+  constexpr size_t smem = panel_smem<V, P, SH>();
+  static int sm_count[64] = {0}; // 0: this device has not run the kernel yet
+  int dev = 0;
+  DRB_CUDA_TRY(cudaGetDevice(&dev));
+  int &sms = sm_count[dev < 64 ? dev : 0];
+  if (sms == 0 || dev >= 64) {
+    DRB_CUDA_TRY(cudaFuncSetAttribute(dense_panel<V, P, SH>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DRB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  const int64_t tiles = (a.m + S::BM - 1) / S::BM;
+  a.cpt = (a.n + S::KC - 1) / S::KC;
+  a.chunks = tiles * a.cpt;
+  // Equal shares over the SMs (one CTA each), of at least kMinShare chunks: a
+  // shorter share is over before the ring is full, and a tile cut into more
+  // pieces only adds partials.
+  constexpr int64_t kMinShare = 4;
+  a.share = std::max((a.chunks + sms - 1) / sms, std::min(kMinShare, a.cpt));
+  // Shares of many tiles end on a tile: the rounding costs under 1/16, the
+  // partials and their pass are saved.
+  if (a.share >= 16 * a.cpt)
+    a.share = (a.share + a.cpt - 1) / a.cpt * a.cpt;
+  const int64_t grid = (a.chunks + a.share - 1) / a.share;
+  const bool cut = a.share % a.cpt != 0;
+  a.part = nullptr;
+  if (cut)
+    DRB_TRY(scratch_alloc(&a.part, sizeof(V) * 2 * (size_t)grid * S::BM * S::CP, s));
+  dense_panel<V, P, SH><<<(unsigned)grid, kNT, smem, s>>>(a);
+  note_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && cut) {
+    const unsigned g = (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>(148 * 8, (a.m * a.k + 255) / 256));
+    panel_sum<V><<<g, 256, 0, s>>>(a, S::BM, S::CP);
+    note_launch();
+    e = cudaGetLastError();
+  }
+  if (a.part)
+    scratch_free(a.part, s);
+  if (e != cudaSuccess) {
+    set_error("dense gemv launch: %s", cudaGetErrorString(e));
+    return DRB_ERR_CUDA;
+  }
+  return DRB_OK;
+}
+
+template <class V, int P> drb_status panel_align(const PanelArgs &a, cudaStream_t s) {
+  const bool aligned = reinterpret_cast<uintptr_t>(a.A) % 16 == 0 &&
+                       a.lda * sizeof(V) % 16 == 0 &&
+                       (a.x_cs != 1 || (reinterpret_cast<uintptr_t>(a.x) % 16 == 0 &&
+                                        a.x_js * sizeof(V) % 16 == 0));
+  return aligned ? panel_run<V, P, false>(a, s) : panel_run<V, P, true>(a, s);
+}
+
+drb_status panel_cols(const PanelArgs &a, float, cudaStream_t s) {
+  if (a.k <= 4)
+    return panel_align<float, 4>(a, s);
+  if (a.k <= 8)
+    return panel_align<float, 8>(a, s);
+  if (a.k <= 12)
+    return panel_align<float, 12>(a, s);
+  if (a.k <= 16)
+    return panel_align<float, 16>(a, s);
+  if (a.k <= 20)
+    return panel_align<float, 20>(a, s);
+  if (a.k <= 24)
+    return panel_align<float, 24>(a, s);
+  return panel_align<float, 32>(a, s);
+}
+drb_status panel_cols(const PanelArgs &a, double, cudaStream_t s) {
+  if (a.k <= 8)
+    return panel_align<double, 1>(a, s);
+  if (a.k <= 16)
+    return panel_align<double, 2>(a, s);
+  if (a.k <= 24)
+    return panel_align<double, 3>(a, s);
+  return panel_align<double, 4>(a, s);
+}
+
+template <class V>
+drb_status panel_typed(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, V *y,
+                       int64_t k, drb_layout layout, cudaStream_t s) {
+  const bool rm = layout == DRB_ROW_MAJOR;
+  if (rm && (n + 31) / 32 > 65535) { // the limit of the layout transposes
+    set_error("transpose: %lld rows exceed the grid limit", (long long)n);
+    return DRB_ERR_UNSUPPORTED;
+  }
+  // Row-major X is gathered element by element in every chunk, which a large A
+  // pays for more than one transpose of X (a launch) costs.
+  const bool turn = rm && m * n > kTurnElems;
+  void *xt = nullptr;
+  if (turn) {
+    DRB_TRY(scratch_alloc(&xt, sizeof(V) * (size_t)n * k, s));
+    const drb_status st = transpose_launch(x, xt, n, k, sizeof(V), s);
+    if (st != DRB_OK) {
+      scratch_free(xt, s);
+      return st;
+    }
+    x = static_cast<const V *>(xt);
+  }
+  PanelArgs a{};
+  a.A = A;
+  a.m = m;
+  a.n = n;
+  a.lda = lda;
+  a.x_cs = rm && !turn ? k : 1;
+  a.x_js = rm && !turn ? 1 : n;
+  a.y_ld = rm ? k : 1;
+  a.y_js = rm ? 1 : m;
+  // more right-hand sides than one pass takes: equal blocks
+  const int64_t nb = (k + kPanelCols - 1) / kPanelCols, kb = (k + nb - 1) / nb;
+  for (int64_t j = 0; j < k; j += kb) {
+    a.k = (int)std::min(kb, k - j);
+    a.x = x + j * a.x_js;
+    a.y = y + j * a.y_js;
+    const drb_status st = panel_cols(a, V(0), s);
+    if (st != DRB_OK) {
+      if (xt)
+        scratch_free(xt, s);
+      return st;
+    }
+  }
+  if (xt)
+    scratch_free(xt, s);
+  return DRB_OK;
+}
+
+} // namespace
+
+drb_status dense_panel_launch(int64_t m, int64_t n, const void *A, int64_t lda, const void *x,
+                              void *y, int64_t k, drb_layout layout, drb_dtype dt,
+                              cudaStream_t s) {
+  if (dt == DRB_F32)
+    return panel_typed<float>(m, n, static_cast<const float *>(A), lda,
+                              static_cast<const float *>(x), static_cast<float *>(y), k, layout,
+                              s);
+  return panel_typed<double>(m, n, static_cast<const double *>(A), lda,
+                             static_cast<const double *>(x), static_cast<double *>(y), k, layout,
+                             s);
+}
+
+} // namespace drb

@@ -1,5 +1,5 @@
-// dense_reduce.cu -- dense row-major gemv and the deterministic dot/norm
-// reduction.
+// dense_reduce.cu -- dense row-major gemv (one right-hand side; several:
+// dense_panel.cu) and the deterministic dot/norm reduction.
 //
 // Dense gemv has no dr::mp counterpart (dr::mp::gemv only takes
 // distributed_sparse_matrix, include/dr/mp/algorithms/matrix/gemv.hpp:16-71);
@@ -29,288 +29,195 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
   return v;
 }
 
-// One warp owns RPW consecutive rows at a time and streams them with 16-byte
-// loads (evict-first); x is read through L1 once per column step and reused
-// for the RPW rows and KB right-hand sides.  x is column-major (x[c + j*n]).
-template <class V, int KB, int RPW, bool VEC>
-__global__ void __launch_bounds__(kDenseNT)
-    dense_gemv_kernel(int64_t m, int64_t n, const V *__restrict__ A,
-                      int64_t lda, const V *__restrict__ x,
-                      V *__restrict__ y, int64_t kb_count, int64_t y_ld,
-                      int64_t y_js) {
-  constexpr int PER = 16 / sizeof(V);
-  const uint64_t pol_s = ptx::policy_evict_first();
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * kDenseNT + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * kDenseNT) >> 5;
-  const int64_t nvec = VEC ? (n / PER) * PER : 0;
-  for (int64_t row0 = warp * RPW; row0 < m; row0 += nwarps * RPW) {
-    V acc[RPW][KB];
-#pragma unroll
-    for (int r = 0; r < RPW; r++)
-#pragma unroll
-      for (int j = 0; j < KB; j++)
-        acc[r][j] = 0;
-    if (VEC) {
-      for (int64_t c = (int64_t)lane * PER; c < nvec; c += 32 * PER) {
-        V a[RPW][PER];
-#pragma unroll
-        for (int r = 0; r < RPW; r++) {
-          union {
-            uint4 u;
-            V t[PER];
-          } w;
-          w.u = make_uint4(0, 0, 0, 0);
-          if (row0 + r < m)
-            w.u = ptx::ld_stream16(A + (row0 + r) * lda + c, pol_s);
-#pragma unroll
-          for (int i = 0; i < PER; i++)
-            a[r][i] = w.t[i];
-        }
-#pragma unroll
-        for (int j = 0; j < KB; j++) {
-          union {
-            uint4 u;
-            V t[PER];
-          } xv;
-          xv.u = __ldg(reinterpret_cast<const uint4 *>(x + j * n + c));
-#pragma unroll
-          for (int r = 0; r < RPW; r++)
-#pragma unroll
-            for (int i = 0; i < PER; i++)
-              acc[r][j] += a[r][i] * xv.t[i];
-        }
-      }
-    }
-    for (int64_t c = nvec + lane; c < n; c += 32) {
-#pragma unroll
-      for (int j = 0; j < KB; j++) {
-        const V xv = __ldg(x + j * n + c);
-#pragma unroll
-        for (int r = 0; r < RPW; r++)
-          if (row0 + r < m)
-            acc[r][j] += A[(row0 + r) * lda + c] * xv;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < RPW; r++)
-#pragma unroll
-      for (int j = 0; j < KB; j++) {
-        const V s = warp_sum_d(acc[r][j]);
-        if (lane == 0 && row0 + r < m && j < kb_count)
-          y[(row0 + r) * y_ld + j * y_js] = s;
-      }
+// One right-hand side: HBM-bound, A streamed once.  The work is cut into
+// steps of one row x 32 * U pieces (16 bytes, or single elements where A's rows
+// or x do not start on 16 bytes), 2 KB to 8 KB of a row, so a warp reads long
+// contiguous runs (page locality decides: one row per warp with 2 KB steps
+// streams at 6.9 TB/s on 32768^2 f32, four rows of 512 bytes at 4.9).
+// Warps take equal consecutive shares of the steps; a row that falls to one
+// warp goes straight to y, the pieces of a row cut between warps to frag
+// (slot 0: the piece does not start its row; slot 1: it does), added in step
+// order.  With LOCAL a CTA owns whole rows, its warps share them, and the
+// pieces meet in shared memory; else the steps are shared over the whole grid
+// and dense_row_join adds the pieces.  (Whole 32 KB row slabs per warp, the
+// earlier unit, left 8192 rows on 7104 warps: some did two while the others
+// had finished one.  8192^2 f32 53.8 -> 46.8 us = 0.89 of the measured HBM
+// rate, 4001^2 f32, whose rows are not aligned, 73 -> 32.)
+template <class V, bool VEC> constexpr int row_unroll() {
+  return VEC ? (sizeof(V) == 4 ? 4 : 8) : 16;
+}
+
+struct RowShare { // the steps [s0, s1) of warp w of W over `steps`, from `base`
+  int64_t s0, s1;
+  __device__ RowShare(int64_t base, int64_t steps, int64_t w, int64_t W)
+      : s0(base + steps * w / W), s1(base + steps * (w + 1) / W) {}
+};
+
+// The row that warp w started and did not finish: its pieces in step order.
+template <class V>
+__device__ __forceinline__ void join_cut_row(int64_t base, int64_t steps, int64_t spr, int64_t w,
+                                             int64_t W, const V *frag, V *y) {
+  const RowShare me(base, steps, w, W);
+  const int64_t row = me.s1 / spr;
+  if (me.s1 % spr == 0 || row * spr < me.s0)
+    return;
+  V s = frag[2 * w + 1];
+  for (int64_t v = w + 1;; v++) {
+    const RowShare o(base, steps, v, W);
+    if (o.s0 >= (row + 1) * spr)
+      break;
+    if (o.s1 > o.s0)
+      s += frag[2 * v];
+    if (v + 1 == W)
+      break;
   }
+  y[row] = s;
 }
 
-// Balanced 16-byte path.  The work is cut into units of one row x one column
-// slab (slab_groups<V>() 16-byte groups: 32 KB of an f32 row, 16 KB of an
-// f64 row); warp w of W takes the contiguous unit range
-// [units*w/W, units*(w+1)/W), so every warp gets the same number of units
-// (+-1) whatever the shape -- tall, square or wide.  A unit's sums go to y
-// directly when a row is one slab, else to part[(row * ns + slab) * KB + j],
-// which dense_slab_sum adds in slab order (deterministic).  Each lane keeps
-// U consecutive 16-byte groups of its row in flight, so a warp reads
-// 512*U contiguous bytes per step: one row per warp with U = 4 (f32) / 16
-// (f64) measured 6.9 TB/s on 32768^2, against 4.9 TB/s (f32) for four rows
-// per warp with one group each (page locality, not occupancy, decides).
-template <class V> constexpr int64_t slab_groups() { return sizeof(V) == 4 ? 2048 : 1024; }
-template <class V, int KB> constexpr int slab_unroll() {
-  return KB == 1 ? (sizeof(V) == 4 ? 4 : 16) : (KB <= 4 ? 2 : 1);
-}
-
-template <class V, int KB>
+template <class V, bool VEC, bool LOCAL>
 __global__ void __launch_bounds__(kDenseNT)
-    dense_slab_kernel(int64_t m, int64_t ng, const V *__restrict__ A, int64_t lda,
-                      const V *__restrict__ x, int64_t n, V *__restrict__ y, int64_t kbc,
-                      int64_t y_ld, int64_t y_js, V *__restrict__ part, int64_t ns,
-                      int64_t units) {
-  constexpr int PER = 16 / sizeof(V);
-  constexpr int U = slab_unroll<V, KB>();
-  constexpr int64_t SG = slab_groups<V>();
+    dense_row_kernel(int64_t m, int64_t n, const V *__restrict__ A, int64_t lda,
+                     const V *__restrict__ x, V *__restrict__ y, int64_t spr, V *frag) {
+  constexpr int PER = VEC ? 16 / (int)sizeof(V) : 1;
+  constexpr int U = row_unroll<V, VEC>();
+  constexpr int NW = kDenseNT / 32;
+  __shared__ V s_frag[2 * NW];
   const uint64_t pol_s = ptx::policy_evict_first();
-  const int lane = threadIdx.x & 31;
-  const int64_t w = ((int64_t)blockIdx.x * kDenseNT + threadIdx.x) >> 5;
-  const int64_t W = ((int64_t)gridDim.x * kDenseNT) >> 5;
-  // units * W stays far below 2^63 (units <= m * n / 1024, W < 2^17)
-  const int64_t u0 = units * w / W;
-  const int64_t u1 = units * (w + 1) / W;
-  for (int64_t u = u0; u < u1; u++) {
-    const int64_t row = u / ns, sl = u - row * ns;
-    const int64_t g0 = sl * SG;
-    const int64_t g1 = min(g0 + SG, ng);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t r0 = LOCAL ? m * blockIdx.x / gridDim.x : 0;
+  const int64_t r1 = LOCAL ? m * (blockIdx.x + 1) / gridDim.x : m;
+  const int64_t base = r0 * spr, steps = (r1 - r0) * spr;
+  const int64_t w = LOCAL ? warp : (int64_t)blockIdx.x * NW + warp;
+  const int64_t W = LOCAL ? NW : (int64_t)gridDim.x * NW;
+  const RowShare me(base, steps, w, W);
+  V *fr = LOCAL ? s_frag : frag;
+  const int64_t ng = n / PER; // whole pieces of a row
+  int64_t row = me.s0 / spr, q = me.s0 - row * spr;
+  bool inside = q != 0; // the current piece does not start its row
+  V acc = 0;
+  for (int64_t s = me.s0; s < me.s1; s++) {
     const V *Ar = A + row * lda;
-    V acc[KB];
-#pragma unroll
-    for (int j = 0; j < KB; j++)
-      acc[j] = 0;
-    for (int64_t gb = g0 + lane; gb < g1; gb += 32 * U) {
+    const int64_t g0 = q * (32 * U) + lane;
+    if constexpr (VEC) {
       union G16 {
         uint4 u;
         V t[PER];
       };
       G16 a[U];
 #pragma unroll
-      for (int q = 0; q < U; q++) {
-        a[q].u = make_uint4(0, 0, 0, 0);
-        if (gb + 32 * q < g1)
-          a[q].u = ptx::ld_stream16(Ar + (gb + 32 * q) * PER, pol_s);
+      for (int i = 0; i < U; i++) {
+        a[i].u = make_uint4(0, 0, 0, 0);
+        if (g0 + 32 * i < ng)
+          a[i].u = ptx::ld_stream16(Ar + (g0 + 32 * i) * PER, pol_s);
       }
 #pragma unroll
-      for (int q = 0; q < U; q++) {
-        const int64_t g = gb + 32 * q;
-        if (g < g1) {
+      for (int i = 0; i < U; i++)
+        if (g0 + 32 * i < ng) {
+          G16 xv;
+          xv.u = __ldg(reinterpret_cast<const uint4 *>(x) + g0 + 32 * i);
 #pragma unroll
-          for (int j = 0; j < KB; j++) {
-            G16 xv;
-            xv.u = __ldg(reinterpret_cast<const uint4 *>(x + j * n) + g);
-#pragma unroll
-            for (int i = 0; i < PER; i++)
-              acc[j] += a[q].t[i] * xv.t[i];
-          }
+          for (int e = 0; e < PER; e++)
+            acc += a[i].t[e] * xv.t[e];
         }
-      }
-    }
+      if (q + 1 == spr && ng * PER + lane < n) // the elements after the last piece
+        acc += Ar[ng * PER + lane] * __ldg(x + ng * PER + lane);
+    } else {
+      V a[U];
 #pragma unroll
-    for (int j = 0; j < KB; j++) {
-      const V t = warp_sum_d(acc[j]);
-      if (lane == 0 && j < kbc) {
-        if (ns == 1)
-          y[row * y_ld + j * y_js] = t;
+      for (int i = 0; i < U; i++)
+        a[i] = g0 + 32 * i < ng ? __ldcs(Ar + g0 + 32 * i) : V(0);
+#pragma unroll
+      for (int i = 0; i < U; i++)
+        if (g0 + 32 * i < ng)
+          acc += a[i] * __ldg(x + g0 + 32 * i);
+    }
+    q++;
+    if (q == spr || s + 1 == me.s1) {
+      const V t = warp_sum_d(acc);
+      if (lane == 0) {
+        if (q == spr && !inside)
+          y[row] = t;
         else
-          part[(row * ns + sl) * KB + j] = t;
+          fr[2 * w + (inside ? 0 : 1)] = t;
       }
+      acc = 0;
+      row++;
+      q = 0;
+      inside = false;
     }
   }
-}
-
-// y[r, j] = sum over slabs of part[(r * ns + s) * KB + j], in slab order.
-template <class V, int KB>
-__global__ void dense_slab_sum(int64_t m, int64_t ns, const V *__restrict__ part,
-                               V *__restrict__ y, int64_t kbc, int64_t y_ld, int64_t y_js) {
-  const int64_t nth = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m * kbc; t += nth) {
-    const int64_t r = t / kbc, j = t - r * kbc;
-    const V *p = part + r * ns * KB + j;
-    V s = 0;
-    for (int64_t q = 0; q < ns; q++)
-      s += p[q * KB];
-    y[r * y_ld + j * y_js] = s;
+  if (LOCAL) {
+    __syncthreads();
+    if (threadIdx.x < NW)
+      join_cut_row<V>(base, steps, spr, threadIdx.x, NW, s_frag, y);
   }
 }
 
-template <class V, int KB>
-drb_status dense_slab_call(cudaStream_t s, int64_t m, int64_t n, const V *A, int64_t lda,
-                           const V *x, V *y, int64_t kbc, int64_t y_ld, int64_t y_js) {
-  constexpr int PER = 16 / sizeof(V);
-  constexpr int64_t SG = slab_groups<V>();
+template <class V>
+__global__ void dense_row_join(int64_t steps, int64_t spr, int64_t W, const V *frag, V *y) {
+  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (w < W)
+    join_cut_row<V>(0, steps, spr, w, W, frag, y);
+}
+
+template <class V, bool VEC>
+drb_status dense_row_call(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, V *y,
+                          cudaStream_t s) {
+  constexpr int PER = VEC ? 16 / (int)sizeof(V) : 1;
+  constexpr int64_t STEP = 32 * row_unroll<V, VEC>(); // pieces per step
   static int grid_cache[64] = {0};
   int dev = 0;
   DRB_CUDA_TRY(cudaGetDevice(&dev));
-  int &grid = grid_cache[dev < 64 ? dev : 0];
-  if (grid == 0) {
+  int &full = grid_cache[dev < 64 ? dev : 0];
+  if (full == 0) {
     int occ = 0, sms = 0;
     DRB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &occ, dense_slab_kernel<V, KB>, kDenseNT, 0));
+        &occ, dense_row_kernel<V, VEC, true>, kDenseNT, 0));
     DRB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    grid = std::max(1, occ) * sms;
+    full = std::max(1, occ) * sms;
   }
-  const int64_t ng = n / PER;
-  const int64_t ns = std::max<int64_t>(1, (ng + SG - 1) / SG);
-  const int64_t units = m * ns;
-  V *part = nullptr;
-  if (ns > 1)
-    DRB_TRY(scratch_alloc(reinterpret_cast<void **>(&part), sizeof(V) * (size_t)m * ns * KB, s));
-  const int64_t need = (units + 7) / 8; // 8 warps per CTA
-  const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid, need));
-  dense_slab_kernel<V, KB><<<g, kDenseNT, 0, s>>>(m, ng, A, lda, x, n, y, kbc, y_ld, y_js,
-                                                  part, ns, units);
-  note_launch();
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess && ns > 1) {
-    const unsigned sg = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(148 * 16, (m * kbc + 255) / 256));
-    dense_slab_sum<V, KB><<<sg, 256, 0, s>>>(m, ns, part, y, kbc, y_ld, y_js);
+  const int64_t spr = std::max<int64_t>(1, (n / PER + STEP - 1) / STEP);
+  const int64_t steps = m * spr;
+  constexpr int NW = kDenseNT / 32;
+  // Whole rows per CTA, unless there are so few of them per CTA (under 4) that
+  // the rounding idles warps for longer than the second launch takes (A over
+  // 16 MB).
+  const bool local = m >= 4 * (int64_t)full || m * n * (int64_t)sizeof(V) < ((int64_t)16 << 20);
+  cudaError_t e;
+  if (local) {
+    const unsigned g = (unsigned)std::min<int64_t>(full, m);
+    dense_row_kernel<V, VEC, true><<<g, kDenseNT, 0, s>>>(m, n, A, lda, x, y, spr, nullptr);
     note_launch();
     e = cudaGetLastError();
+  } else {
+    const unsigned g = (unsigned)std::min<int64_t>(full, (steps + NW - 1) / NW);
+    const int64_t W = (int64_t)g * NW;
+    V *frag = nullptr;
+    DRB_TRY(scratch_alloc(reinterpret_cast<void **>(&frag), sizeof(V) * 2 * (size_t)W, s));
+    dense_row_kernel<V, VEC, false><<<g, kDenseNT, 0, s>>>(m, n, A, lda, x, y, spr, frag);
+    note_launch();
+    e = cudaGetLastError();
+    if (e == cudaSuccess) {
+      dense_row_join<V><<<(unsigned)((W + 255) / 256), 256, 0, s>>>(steps, spr, W, frag, y);
+      note_launch();
+      e = cudaGetLastError();
+    }
+    scratch_free(frag, s);
   }
-  if (part)
-    scratch_free(part, s);
   if (e != cudaSuccess) {
     set_error("dense gemv launch: %s", cudaGetErrorString(e));
     return DRB_ERR_CUDA;
   }
-  return DRB_OK;
-}
-
-template <class V, int KB, int RPW>
-drb_status dense_call(bool vec, unsigned grid, cudaStream_t s, int64_t m, int64_t n,
-                      const V *A, int64_t lda, const V *x, V *y, int64_t kbc,
-                      int64_t y_ld, int64_t y_js) {
-  if (vec)
-    return dense_slab_call<V, KB>(s, m, n, A, lda, x, y, kbc, y_ld, y_js);
-  dense_gemv_kernel<V, KB, RPW, false><<<grid, kDenseNT, 0, s>>>(
-      m, n, A, lda, x, y, kbc, y_ld, y_js);
-  note_launch();
   return DRB_OK;
 }
 
 template <class V>
-drb_status dense_typed(int64_t m, int64_t n, const V *A, int64_t lda,
-                       const V *x, V *y, int64_t k, drb_layout layout,
-                       cudaStream_t s) {
-  constexpr int PER = 16 / sizeof(V);
-  // x as column-major: a row-major k > 1 block is transposed first.
-  const V *xc = x;
-  void *tmp = nullptr;
-  if (layout == DRB_ROW_MAJOR && k > 1) {
-    DRB_TRY(scratch_alloc(&tmp, sizeof(V) * n * k, s));
-    drb_status st = transpose_launch(x, tmp, n, k, sizeof(V), s);
-    if (st != DRB_OK) {
-      scratch_free(tmp, s);
-      return st;
-    }
-    xc = static_cast<const V *>(tmp);
-  }
-  const bool vec = (reinterpret_cast<uintptr_t>(A) % 16 == 0) &&
-                   (reinterpret_cast<uintptr_t>(xc) % 16 == 0) &&
-                   (lda % PER == 0) && (n % PER == 0);
-  const unsigned grid = 148 * 8;
-  // y address of (row r, rhs j): r*y_ld + j*y_js
-  const int64_t y_ld = layout == DRB_ROW_MAJOR ? k : 1;
-  const int64_t y_js = layout == DRB_ROW_MAJOR ? 1 : m;
-  for (int64_t jb = 0; jb < k;) {
-    const int64_t left = k - jb;
-    const V *xj = xc + jb * n;
-    V *yj = y + jb * y_js;
-    drb_status st;
-    if (left >= 8) {
-      st = dense_call<V, 8, 1>(vec, grid, s, m, n, A, lda, xj, yj, 8, y_ld, y_js);
-      jb += 8;
-    } else if (left >= 4) {
-      st = dense_call<V, 4, 2>(vec, grid, s, m, n, A, lda, xj, yj, 4, y_ld, y_js);
-      jb += 4;
-    } else if (left >= 2) {
-      st = dense_call<V, 2, 2>(vec, grid, s, m, n, A, lda, xj, yj, 2, y_ld, y_js);
-      jb += 2;
-    } else {
-      st = dense_call<V, 1, 4>(vec, grid, s, m, n, A, lda, xj, yj, 1, y_ld, y_js);
-      jb += 1;
-    }
-    if (st != DRB_OK) {
-      if (tmp)
-        scratch_free(tmp, s);
-      return st;
-    }
-  }
-  cudaError_t e = cudaGetLastError();
-  if (tmp)
-    scratch_free(tmp, s);
-  if (e != cudaSuccess) {
-    set_error("dense gemv launch: %s", cudaGetErrorString(e));
-    return DRB_ERR_CUDA;
-  }
-  return DRB_OK;
+drb_status dense_row(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, V *y,
+                     cudaStream_t s) {
+  const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(x) % 16 == 0 && lda * sizeof(V) % 16 == 0;
+  return vec ? dense_row_call<V, true>(m, n, A, lda, x, y, s)
+             : dense_row_call<V, false>(m, n, A, lda, x, y, s);
 }
 
 // ---- dot -------------------------------------------------------------------------
@@ -524,12 +431,13 @@ drb_status dense_launch(int64_t m, int64_t n, const void *A, int64_t lda,
     DRB_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)dtype_bytes(dt) * m * k, s));
     return DRB_OK;
   }
-  if (dt == DRB_F32)
-    return dense_typed<float>(m, n, (const float *)A, lda, (const float *)x,
-                              (float *)y, k, layout, s);
-  if (dt == DRB_F64)
-    return dense_typed<double>(m, n, (const double *)A, lda, (const double *)x,
-                               (double *)y, k, layout, s);
+  if (dt == DRB_F32 || dt == DRB_F64) {
+    if (k > 1)
+      return dense_panel_launch(m, n, A, lda, x, y, k, layout, dt, s);
+    if (dt == DRB_F32)
+      return dense_row<float>(m, n, (const float *)A, lda, (const float *)x, (float *)y, s);
+    return dense_row<double>(m, n, (const double *)A, lda, (const double *)x, (double *)y, s);
+  }
   set_error("dense gemv: dtype %d not supported", (int)dt);
   return DRB_ERR_UNSUPPORTED;
 }

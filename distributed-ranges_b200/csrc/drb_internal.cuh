@@ -301,6 +301,10 @@ drb_status adjoint_refresh_values(Csr &A, cudaStream_t s);
 drb_status dense_launch(int64_t m, int64_t n, const void *A, int64_t lda,
                         const void *x, void *y, int64_t k, drb_layout layout,
                         drb_dtype dt, cudaStream_t s);
+// k > 1 right-hand sides, F32 or F64 (dense_panel.cu)
+drb_status dense_panel_launch(int64_t m, int64_t n, const void *A, int64_t lda, const void *x,
+                              void *y, int64_t k, drb_layout layout, drb_dtype dt,
+                              cudaStream_t s);
 drb_status dot_launch(int64_t n, const void *a, const void *b, drb_dtype dt,
                       double *out, cudaStream_t s);
 drb_status dot_noalloc_launch(int64_t n, const void *a, const void *b,

@@ -1,0 +1,84 @@
+"""Dense gemv paths against the oracle at the edges of their tiles: the multi-RHS
+panel kernel (tiles of 64 or 32 rows x 128 columns in FP32, 128 x 32 in FP64,
+tiles cut between CTAs, 16-byte and single-element loads, blocks of at most 32
+right-hand sides) and the one-RHS row kernel (rows cut between warps and CTAs)."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def mp():
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from drb import mp as _mp
+    return _mp
+
+
+def check(mp, dtype, m, n, k, lda, layout, offset=0):
+    g = torch.Generator().manual_seed(1000 * m + 10 * n + k)
+    buf = torch.full((m * lda + offset,), float("nan"), dtype=dtype)
+    A = buf[offset:].view(m, lda)[:, :n]
+    A.copy_(torch.randn(m, n, generator=g, dtype=torch.float64))
+    X = torch.randn(n, k, generator=g, dtype=torch.float64).to(dtype)
+    dev = buf.cuda()
+    Ad = dev[offset:].view(m, lda)[:, :n]
+    xin = (X.t().contiguous() if layout == 0 else X.contiguous()).cuda()
+    y = torch.full((m * k,), float("nan"), dtype=dtype, device="cuda")
+    mp.dense_gemv(Ad, xin, y, k, layout)
+    y2 = torch.empty_like(y)
+    mp.dense_gemv(Ad, xin, y2, k, layout)
+    assert torch.equal(y, y2)  # repeatable bit for bit
+    Y = (y.cpu().view(k, m).t() if layout == 0 else y.cpu().view(m, k)).double().numpy()
+    ref = oracle.dense_gemv(A.double().contiguous().numpy(),
+                            X.double().t().contiguous().numpy().ravel(), k,
+                            oracle.ACC_LD).reshape(k, m).T
+    u = 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -53
+    # every output is a sum of n products in some order: at most n roundings each
+    bound = (n + 8) * u * (A.double().abs() @ X.double().abs()).numpy()
+    assert np.all(np.abs(Y - ref) <= bound)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("m,n,k,lda,layout", [
+    (1, 1, 2, 1, 0), (31, 33, 2, 33, 1), (33, 127, 4, 128, 0), (63, 128, 5, 128, 1),
+    (64, 129, 8, 132, 0), (65, 31, 9, 31, 1), (127, 32, 12, 32, 0), (128, 640, 13, 643, 0),
+    (129, 1000, 16, 1000, 1), (257, 4111, 17, 4111, 0), (300, 2050, 20, 2052, 1),
+    (1000, 777, 21, 777, 0), (2000, 515, 24, 516, 1), (95, 6000, 25, 6000, 0),
+    (4099, 100, 32, 100, 1), (130, 1500, 33, 1501, 0), (70, 300, 67, 300, 1)])
+def test_panel(mp, dtype, m, n, k, lda, layout):
+    check(mp, dtype, m, n, k, lda, layout)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", [1, 6])
+def test_misaligned_base(mp, dtype, k):
+    check(mp, dtype, 200, 1024, k, 1024, 0, offset=1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("m,n,lda", [
+    (1, 3, 3), (2, 511, 512), (3, 513, 513), (100, 2049, 2052), (889, 1000, 1000),
+    # over 16 MB with few rows per CTA: rows cut between CTAs
+    (5, 1_000_003, 1_000_004), (40, 131_073, 131_073), (1500, 3001, 3001),
+    # whole rows per CTA
+    (5003, 1001, 1001), (9000, 130, 132)])
+def test_one_rhs(mp, dtype, m, n, lda):
+    check(mp, dtype, m, n, 1, lda, 0)
+
+
+def test_nan_stays_in_its_row_and_column(mp):
+    A = torch.randn(70, 200, device="cuda")
+    x = torch.randn(3 * 200, device="cuda")
+    A[5, 7], x[200 + 11] = float("nan"), float("inf")
+    y = torch.empty(3 * 70, device="cuda")
+    mp.dense_gemv(A, x, y, 3, 0)
+    bad = ~torch.isfinite(y.view(3, 70)).cpu()
+    want = torch.zeros(3, 70, dtype=torch.bool)
+    want[:, 5] = True
+    want[1, :] = True
+    assert torch.equal(bad, want)
