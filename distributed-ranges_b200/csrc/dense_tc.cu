@@ -7,8 +7,10 @@
 // 18-62: a naive M x K x N loop with atomics or oneMKL gemm); this is the
 // multi-RHS dense form of dr::mp::gemv for a batch of matrices.
 //
-// One CTA computes one 128-row tile of one matrix over the whole K range
-// (tiles of all matrices in one grid, longest K first).  Six warps:
+// One CTA computes one unit: a 128-row tile of one matrix over its whole K range
+// (units of all matrices in one grid, longest K first), or, when the tiles
+// alone leave SMs idle, over one of several equal parts of it; the parts'
+// partial tiles are then added in K order by a second small kernel.  Six warps:
 //   warp 0    : TMA producer -- for each 64-wide K step, the 128 x 64 tile
 //               of A and the N x 64 tile of X (K-major, 128-byte swizzle)
 //               into a STAGES-deep ring, completion counted on an mbarrier;
@@ -54,6 +56,17 @@ constexpr int kVarStages[kNumVariants] = {4, 5, 8, 2, 4};
 constexpr int kVarBoxes[kNumVariants] = {1, 1, 1, 2, 2};
 constexpr int kDefaultVariant = 1; // fastest on the 64-matrix, k = 32 batch
 
+// A CTA's work: rows [row, row + 128) of matrix mat, K steps [s0, s1) of
+// kUnitK columns; slot >= 0: the partial tile it writes (else Y).
+constexpr int kUnitK = 2 * kTileK; // a whole number of steps of every ring variant
+struct DUnit {
+  int mat, row, s0, s1, slot, tile;
+  int pad0, pad1;
+};
+struct DSplit { // a tile summed from parts [slot, slot + count)
+  int mat, row, slot, count;
+};
+
 struct DMat {
   const CUtensorMap *tma; // A map
   const CUtensorMap *tmx; // X map (K-major: rows = right-hand sides)
@@ -64,14 +77,15 @@ struct DMat {
 
 struct DArgs {
   const DMat *mats;
-  const int2 *tiles; // {matrix, first row}
+  const DUnit *units;
+  float *part; // [slot][k][128] partial tiles
   int k;             // right-hand sides
   int N;             // k rounded up to 16 (UMMA N)
   int tmem_cols;     // power of two >= max(32, N)
   int row_major;
   int *err;
   uint64_t wait_ns; // limit of every mbarrier wait
-  int stall_tile;   // failure-detection hook: this CTA issues no loads (-1: none)
+  int stall_tile;   // failure-detection hook: this tile's CTAs issue no loads (-1: none)
 };
 
 // ---- tcgen05 / TMA PTX wrappers --------------------------------------------
@@ -187,9 +201,13 @@ __global__ void __launch_bounds__(kThreads, 1) dense_tc(const DArgs a) {
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int2 tile = a.tiles[blockIdx.x];
-  const DMat mt = a.mats[tile.x];
-  const int nk = (int)((mt.n + kBoxes * kTileK - 1) / (kBoxes * kTileK));
+  const DUnit unit = a.units[blockIdx.x];
+  const DMat mt = a.mats[unit.mat];
+  // stages of this unit, from column k0
+  constexpr int kStageK = kBoxes * kTileK;
+  const int k0 = unit.s0 * kUnitK;
+  const int64_t kend = min(mt.n, (int64_t)unit.s1 * kUnitK);
+  const int nk = (int)((kend - k0 + kStageK - 1) / kStageK);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; s++) {
@@ -219,8 +237,25 @@ __global__ void __launch_bounds__(kThreads, 1) dense_tc(const DArgs a) {
     if (lane == 0) {
       const uint32_t tx = (uint32_t)(kStageA + stage_b);
       int issued = 0; // stages whose loads were issued
-      if ((int)blockIdx.x != a.stall_tile) {
-        for (int s = 0; s < nk; s++) {
+      if (unit.tile != a.stall_tile) {
+        // A does not depend on the kernel that packs X: its first boxes go out
+        // before that kernel is waited for
+        const int ahead = min(nk, kStages);
+        for (int s = 0; s < ahead; s++) {
+          tma::mbar_arrive_expect_tx(&full[s], tx);
+#pragma unroll
+          for (int b = 0; b < kBoxes; b++)
+            tma_load_2d(sa + s * kStageA + b * kABytes, mt.tma, k0 + (s * kBoxes + b) * kTileK,
+                        unit.row, &full[s]);
+        }
+        ptx::grid_dependency_wait();
+        for (int s = 0; s < ahead; s++)
+#pragma unroll
+          for (int b = 0; b < kBoxes; b++)
+            tma_load_2d(sb + s * stage_b + b * bbytes, mt.tmx, k0 + (s * kBoxes + b) * kTileK, 0,
+                        &full[s]);
+        issued = ahead;
+        for (int s = ahead; s < nk; s++) {
           const int slot = s % kStages;
           const uint32_t ph = (uint32_t)((s / kStages) & 1);
           if (aborted(a.err, abort_flag))
@@ -230,8 +265,8 @@ __global__ void __launch_bounds__(kThreads, 1) dense_tc(const DArgs a) {
           tma::mbar_arrive_expect_tx(&full[slot], tx);
 #pragma unroll
           for (int b = 0; b < kBoxes; b++) {
-            const int kx = (s * kBoxes + b) * kTileK;
-            tma_load_2d(sa + slot * kStageA + b * kABytes, mt.tma, kx, tile.y,
+            const int kx = k0 + (s * kBoxes + b) * kTileK;
+            tma_load_2d(sa + slot * kStageA + b * kABytes, mt.tma, kx, unit.row,
                         &full[slot]);
             tma_load_2d(sb + slot * stage_b + b * bbytes, mt.tmx, kx, 0,
                         &full[slot]);
@@ -287,7 +322,9 @@ __global__ void __launch_bounds__(kThreads, 1) dense_tc(const DArgs a) {
     }
     tc_fence_after();
     if (ok && !aborted(a.err, abort_flag)) {
-      const int64_t r = (int64_t)tile.y + q * 32 + lane;
+      const int64_t r = (int64_t)unit.row + q * 32 + lane;
+      float *pt = unit.slot >= 0 ? a.part + (int64_t)unit.slot * a.k * kTileM + q * 32 + lane
+                                 : nullptr;
       for (int c0 = 0; c0 < a.N; c0 += 32) {
         uint32_t v[32];
         tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
@@ -296,7 +333,9 @@ __global__ void __launch_bounds__(kThreads, 1) dense_tc(const DArgs a) {
           for (int j = 0; j < 32; j++) {
             const int c = c0 + j;
             if (c < a.k) {
-              if (a.row_major)
+              if (pt)
+                pt[c * kTileM] = __uint_as_float(v[j]);
+              else if (a.row_major)
                 mt.y[r * a.k + c] = __uint_as_float(v[j]);
               else
                 mt.y[r + (int64_t)c * mt.m] = __uint_as_float(v[j]);
@@ -322,22 +361,74 @@ __global__ void __launch_bounds__(kThreads, 1) dense_tc(const DArgs a) {
   }
 }
 
-// Xp[j*ldp + c] = X(c, j) for c < n: the right-hand sides of every matrix
-// as K-major rows, in one launch (blockIdx.y = matrix; a few blocks per
-// matrix loop over its k right-hand sides).
+// Xp[j*ldp + c] = X(c, j) for c < n: the right-hand sides of a matrix as K-major
+// rows that a tensor map can read (ldp a multiple of 64), one CTA per 64
+// columns of one matrix, all matrices in one launch.  A thread writes 16 bytes
+// of a row at a time; row-major X turns through shared memory.  (A grid of
+// eight CTAs per matrix walking over all right-hand sides one element per
+// thread took 62 of 198 us for 16 matrices of up to 8192 columns and k = 32;
+// the call now takes 140, 0.91 of the measured HBM rate for its A.)
+// Column-major X whose columns start on 16 bytes is not packed at all: the
+// tensor map reads it in place.
 struct RhsPack {
   const uint16_t *x;
   uint16_t *xp;
   int64_t n, ldp;
 };
+constexpr int kPackCols = 64;
 
-__global__ void pack_rhs_bf16(const RhsPack *__restrict__ packs, int k,
-                              int row_major) {
-  const RhsPack p = packs[blockIdx.y];
-  for (int j = 0; j < k; j++)
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < p.n;
-         c += (int64_t)gridDim.x * blockDim.x)
-      p.xp[j * p.ldp + c] = row_major ? p.x[c * k + j] : p.x[c + j * p.n];
+__global__ void __launch_bounds__(256) pack_rhs_bf16(const RhsPack *__restrict__ packs,
+                                                     const int2 *__restrict__ tiles, int k,
+                                                     int row_major) {
+  __shared__ uint16_t s_x[kPackCols * 256 + 8];
+  ptx::grid_dependents_start();
+  const int2 t = tiles[blockIdx.x]; // {matrix, first column}
+  const RhsPack p = packs[t.x];
+  const int64_t c0 = t.y;
+  const int nc = (int)min((int64_t)kPackCols, p.n - c0);
+  if (row_major) {
+    const uint16_t *src = p.x + c0 * k;
+    for (int i = threadIdx.x; i < nc * k; i += 256)
+      s_x[i] = src[i];
+    __syncthreads();
+  }
+  const int g = (threadIdx.x & 7) * 8; // 8 columns of the tile
+  if (g >= nc)
+    return;
+  for (int j = threadIdx.x >> 3; j < k; j += 32) {
+    union {
+      uint4 u;
+      uint16_t w[8];
+    } v;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      v.w[i] = g + i >= nc ? (uint16_t)0
+               : row_major ? s_x[(g + i) * k + j]
+                           : __ldg(p.x + c0 + g + i + j * p.n);
+    *reinterpret_cast<uint4 *>(p.xp + j * p.ldp + c0 + g) = v.u;
+  }
+}
+
+// Y of the tiles computed in parts: the partial tiles added in K order.
+__global__ void __launch_bounds__(kTileM) dense_tc_sum(const DArgs a,
+                                                       const DSplit *__restrict__ splits) {
+  if (*(volatile const int *)a.err)
+    return; // a part is missing: Y stays unwritten
+  const DSplit t = splits[blockIdx.x];
+  const DMat mt = a.mats[t.mat];
+  const int64_t r = (int64_t)t.row + threadIdx.x;
+  if (r >= mt.m)
+    return;
+  const float *p = a.part + (int64_t)t.slot * a.k * kTileM + threadIdx.x;
+  for (int c = blockIdx.y; c < a.k; c += gridDim.y) {
+    float s = 0.0f;
+    for (int i = 0; i < t.count; i++)
+      s += p[((int64_t)i * a.k + c) * kTileM];
+    if (a.row_major)
+      mt.y[r * a.k + c] = s;
+    else
+      mt.y[r + (int64_t)c * mt.m] = s;
+  }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -411,14 +502,12 @@ struct DenseBatch {
   int64_t k = 1;
   int N = 16, tmem_cols = 32;
   bool row_major = false;
-  int ntiles = 0;
+  int nunits = 0, nsplits = 0, npack_tiles = 0;
   size_t smem = 0;
-  int npacks = 0;
-  int64_t max_n = 0;
   std::vector<std::pair<float *, size_t>> zero; // outputs of n == 0 matrices
   uint64_t wait_ns = tma::kWaitNs;
   int stall_tile = -1;
-  DevBuf maps, mats, tiles, xp, packs, err;
+  DevBuf maps, mats, units, splits, part, xp, packs, pack_tiles, err;
 };
 
 namespace {
@@ -470,7 +559,8 @@ drb_status make_dense_batch(DenseBatch &P, int32_t count, const int64_t *m,
   P.row_major = layout == DRB_ROW_MAJOR;
   std::vector<std::pair<int64_t, int2>> order; // (K, tile)
   int64_t xp_elems = 0;
-  std::vector<int64_t> ldp(count, 0);
+  std::vector<int64_t> ldp(count, 0); // row pitch of X as the kernel reads it; 0: no tile
+  std::vector<char> packed(count, 0);
   for (int i = 0; i < count; i++) {
     if (m[i] < 0 || n[i] < 0 || m[i] >= INT32_MAX || n[i] >= INT32_MAX)
       return fail(DRB_ERR_INVALID_ARG, "invalid argument: m[%d] or n[%d]", i, i);
@@ -491,21 +581,64 @@ drb_status make_dense_batch(DenseBatch &P, int32_t count, const int64_t *m,
                   "dense batch needs lda[%d] >= n, a multiple of 8, and A 16-byte "
                   "aligned",
                   i);
-    ldp[i] = (n[i] + 63) / 64 * 64;
-    xp_elems += ldp[i] * k;
+    packed[i] = P.row_major || n[i] % 8 != 0 || reinterpret_cast<uintptr_t>(x[i]) % 16 != 0;
+    ldp[i] = packed[i] ? (n[i] + 63) / 64 * 64 : n[i];
+    if (packed[i])
+      xp_elems += ldp[i] * k;
     for (int64_t r0 = 0; r0 < m[i]; r0 += kTileM)
       order.push_back({n[i], make_int2(i, (int)r0)});
   }
   std::stable_sort(order.begin(), order.end(),
                    [](const auto &p, const auto &q) { return p.first > q.first; });
-  P.ntiles = (int)order.size();
+  const int ntiles = (int)order.size();
   DRB_TRY(P.err.alloc(sizeof(int)));
   DRB_CUDA_TRY(cudaMemset(P.err.p, 0, sizeof(int)));
-  if (P.ntiles == 0)
+  if (ntiles == 0)
     return DRB_OK;
+  // Fewer tiles than the GPU runs at once (two CTAs per SM): cut them along K
+  // into about that many units.  A unit keeps at least 512 columns (a shorter one
+  // is mostly prologue and epilogue) and 16 k (its partial tile is written and
+  // read once, 1 KB per right-hand side against 256 bytes of A per column).  One
+  // 8192^2 matrix (64 tiles on 148 SMs, k = 32): 134 -> 44 us; two of 3000^2 at
+  // k = 128: 107 -> 39.
+  const int64_t kMinUnit = std::max<int64_t>(4, k * 16 / kUnitK); // steps of kUnitK columns
+  int sms = 0;
+  DRB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t slots = 2 * (int64_t)sms;
+  int64_t total = 0;
+  for (const auto &o : order)
+    total += (o.first + kUnitK - 1) / kUnitK;
+  const int64_t target = std::max<int64_t>(kMinUnit, (total + slots - 1) / slots);
+  std::vector<DUnit> units;
+  std::vector<DSplit> splits;
+  int nslots = 0;
+  for (int t = 0; t < ntiles; t++) {
+    const int64_t steps = (order[t].first + kUnitK - 1) / kUnitK;
+    int64_t parts = 1;
+    if (ntiles < slots)
+      parts = std::max<int64_t>(1, std::min((steps + target - 1) / target, steps / kMinUnit));
+    const int2 at = order[t].second;
+    if (parts > 1)
+      splits.push_back({at.x, at.y, nslots, (int)parts});
+    for (int64_t i = 0; i < parts; i++)
+      units.push_back({at.x, at.y, (int)(steps * i / parts), (int)(steps * (i + 1) / parts),
+                       parts > 1 ? nslots++ : -1, t, 0, 0});
+  }
+  std::stable_sort(units.begin(), units.end(), [](const DUnit &p, const DUnit &q) {
+    return p.s1 - p.s0 > q.s1 - q.s0;
+  });
+  P.nunits = (int)units.size();
+  P.nsplits = (int)splits.size();
+  if (nslots > 0) {
+    DRB_TRY(P.part.alloc(sizeof(float) * (size_t)nslots * k * kTileM));
+    DRB_TRY(P.splits.alloc(sizeof(DSplit) * splits.size()));
+    DRB_CUDA_TRY(cudaMemcpy(P.splits.p, splits.data(), sizeof(DSplit) * splits.size(),
+                            cudaMemcpyHostToDevice));
+  }
   DRB_TRY(P.xp.alloc((size_t)xp_elems * 2));
   std::vector<CUtensorMap> maps(2 * (size_t)count);
-  std::vector<RhsPack> hp;
+  std::vector<RhsPack> hp(count, RhsPack{nullptr, nullptr, 0, 0});
+  std::vector<int2> ptiles;
   std::vector<DMat> dm(count);
   DRB_TRY(P.maps.alloc(sizeof(CUtensorMap) * maps.size()));
   int64_t off = 0;
@@ -513,10 +646,14 @@ drb_status make_dense_batch(DenseBatch &P, int32_t count, const int64_t *m,
     dm[i] = DMat{nullptr, nullptr, static_cast<float *>(y[i]), m[i], n[i]};
     if (ldp[i] == 0)
       continue;
-    uint16_t *xpi = P.xp.as<uint16_t>() + off;
-    off += ldp[i] * k;
-    hp.push_back({static_cast<const uint16_t *>(x[i]), xpi, n[i], ldp[i]});
-    P.max_n = std::max(P.max_n, n[i]);
+    const void *xpi = x[i];
+    if (packed[i]) {
+      hp[i] = {static_cast<const uint16_t *>(x[i]), P.xp.as<uint16_t>() + off, n[i], ldp[i]};
+      xpi = hp[i].xp;
+      off += ldp[i] * k;
+      for (int64_t c = 0; c < n[i]; c += kPackCols)
+        ptiles.push_back(make_int2(i, (int)c));
+    }
     DRB_TRY(make_map(&maps[2 * i], A[i], (uint64_t)n[i], (uint64_t)m[i],
                      (uint64_t)lda[i] * 2, kTileM));
     DRB_TRY(make_map(&maps[2 * i + 1], xpi, (uint64_t)n[i], (uint64_t)k,
@@ -524,20 +661,22 @@ drb_status make_dense_batch(DenseBatch &P, int32_t count, const int64_t *m,
     dm[i].tma = P.maps.as<CUtensorMap>() + 2 * i;
     dm[i].tmx = P.maps.as<CUtensorMap>() + 2 * i + 1;
   }
-  P.npacks = (int)hp.size();
+  P.npack_tiles = (int)ptiles.size();
   DRB_TRY(P.packs.alloc(sizeof(RhsPack) * hp.size()));
   DRB_CUDA_TRY(cudaMemcpy(P.packs.p, hp.data(), sizeof(RhsPack) * hp.size(),
                           cudaMemcpyHostToDevice));
+  if (P.npack_tiles > 0) {
+    DRB_TRY(P.pack_tiles.alloc(sizeof(int2) * ptiles.size()));
+    DRB_CUDA_TRY(cudaMemcpy(P.pack_tiles.p, ptiles.data(), sizeof(int2) * ptiles.size(),
+                            cudaMemcpyHostToDevice));
+  }
   DRB_TRY(P.mats.alloc(sizeof(DMat) * count));
-  DRB_TRY(P.tiles.alloc(sizeof(int2) * P.ntiles));
-  std::vector<int2> tl(P.ntiles);
-  for (int t = 0; t < P.ntiles; t++)
-    tl[t] = order[t].second;
+  DRB_TRY(P.units.alloc(sizeof(DUnit) * units.size()));
   DRB_CUDA_TRY(cudaMemcpy(P.maps.p, maps.data(), sizeof(CUtensorMap) * maps.size(),
                           cudaMemcpyHostToDevice));
   DRB_CUDA_TRY(cudaMemcpy(P.mats.p, dm.data(), sizeof(DMat) * count,
                           cudaMemcpyHostToDevice));
-  DRB_CUDA_TRY(cudaMemcpy(P.tiles.p, tl.data(), sizeof(int2) * P.ntiles,
+  DRB_CUDA_TRY(cudaMemcpy(P.units.p, units.data(), sizeof(DUnit) * units.size(),
                           cudaMemcpyHostToDevice));
   return set_dense_variant(P, kDefaultVariant);
 }
@@ -545,18 +684,18 @@ drb_status make_dense_batch(DenseBatch &P, int32_t count, const int64_t *m,
 drb_status dense_batch_launch(DenseBatch &P, cudaStream_t s) {
   for (auto &z : P.zero)
     DRB_CUDA_TRY(cudaMemsetAsync(z.first, 0, z.second * sizeof(float), s));
-  if (P.ntiles == 0)
+  if (P.nunits == 0)
     return DRB_OK;
-  {
-    const dim3 grid((unsigned)std::min<int64_t>((P.max_n + 255) / 256, 8),
-                    (unsigned)P.npacks);
-    pack_rhs_bf16<<<grid, 256, 0, s>>>(P.packs.as<RhsPack>(), (int)P.k,
-                                       P.row_major ? 1 : 0);
+  if (P.npack_tiles > 0) {
+    pack_rhs_bf16<<<(unsigned)P.npack_tiles, 256, 0, s>>>(
+        P.packs.as<RhsPack>(), P.pack_tiles.as<int2>(), (int)P.k, P.row_major ? 1 : 0);
     DRB_CUDA_TRY(cudaGetLastError());
+    note_launch();
   }
   DArgs a;
   a.mats = P.mats.as<DMat>();
-  a.tiles = P.tiles.as<int2>();
+  a.units = P.units.as<DUnit>();
+  a.part = P.part.as<float>();
   a.k = (int)P.k;
   a.N = P.N;
   a.tmem_cols = P.tmem_cols;
@@ -564,9 +703,23 @@ drb_status dense_batch_launch(DenseBatch &P, cudaStream_t s) {
   a.err = P.err.as<int>();
   a.wait_ns = P.wait_ns;
   a.stall_tile = P.stall_tile;
-  dense_kernel(P.variant)<<<P.ntiles, kThreads, P.smem, s>>>(a);
-  DRB_CUDA_TRY(cudaGetLastError());
-  note_launch(2);
+  // behind the pack kernel the product may start early: it prepares its ring
+  // and loads A, and waits for the packed X before it loads any of it
+  const dim3 grid((unsigned)P.nunits);
+  if (P.npack_tiles > 0) {
+    DRB_CUDA_TRY(
+        launch_overlapped(dense_kernel(P.variant), grid, dim3(kThreads), P.smem, s, a));
+  } else {
+    dense_kernel(P.variant)<<<grid, kThreads, P.smem, s>>>(a);
+    DRB_CUDA_TRY(cudaGetLastError());
+  }
+  note_launch();
+  if (P.nsplits > 0) {
+    const dim3 sum_grid((unsigned)P.nsplits, (unsigned)std::min<int64_t>(P.k, 16));
+    dense_tc_sum<<<sum_grid, kTileM, 0, s>>>(a, P.splits.as<DSplit>());
+    DRB_CUDA_TRY(cudaGetLastError());
+    note_launch();
+  }
   return DRB_OK;
 }
 

@@ -53,6 +53,25 @@ inline void note_launch(uint64_t n = 1) {
     g_launch_count.fetch_add(n);
 }
 
+// Launches `kernel` so that it may start while the previous kernel of the stream
+// finishes (programmatic dependent launch): it must execute
+// ptx::grid_dependency_wait() before it touches anything that kernel writes.
+template <class... P, class... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute early = {};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Makes `dev` current for the scope of an entry point, restoring the
 // caller's device afterwards.
 struct DeviceGuard {
@@ -336,6 +355,16 @@ struct drb_csr_matrix : public drb::Csr {};
 
 // ---- PTX helpers ---------------------------------------------------------------
 namespace drb::ptx {
+
+// Waits until the grids this launch depends on have completed (returns at once
+// for a launch without the programmatic attribute).
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Lets the next kernel of the stream start (it waits for this one's results).
+__device__ __forceinline__ void grid_dependents_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // L2 policies: streamed matrix data is evicted first, the gathered vector x
 // is kept (evict_last) so it stays L2-resident across the whole launch.
