@@ -4,7 +4,9 @@
 // The reference gives the pieces -- gemv (include/dr/mp/algorithms/matrix/
 // gemv.hpp:16-27), reduce over a distributed_vector (reduce.hpp:58-181) and
 // element-wise transforms -- and leaves the loop to the caller, who would pay
-// a host round trip per reduction.  Here one iteration is three launches:
+// a host round trip per reduction.  Matrices on their sliced-ELL copy run the
+// whole loop in one launch (cg_resident.cu).  For the others one iteration is
+// three launches:
 //
 //   1. the persistent SpMV, q = A p, with p.q summed in its row epilogue
 //      (rowdot_pipe_launch; the same deterministic per-CTA partials + last-CTA
@@ -22,6 +24,7 @@
 // the scalars are f64.
 #include <cmath>
 
+#include "cg_state.cuh"
 #include "drb_internal.cuh"
 
 namespace drb {
@@ -33,23 +36,11 @@ constexpr int kCgNT = 256;
 constexpr int kCgGrid = 148 * 3;
 constexpr int kCgMinBlocks = 3;
 constexpr int kCgBlock = 8;  // iterations per graph replay
-
-enum : int { kRunning = 0, kConverged = 1, kBreakdown = 2, kMaxIters = 3 };
-
-struct CgState {
-  double rr;   // r.r of the current residual
-  double pq;   // p.Ap of the current iteration (written by the SpMV)
-  double beta; // rr' / rr of the last update
-  double bb;   // b.b
-  double tol2; // rtol^2 * b.b
-  int64_t iters, max_iters;
-  int done; // kRunning, kConverged, kBreakdown, kMaxIters
-  int pad;
-};
 } // namespace
 
 struct CgPlan {
   DevBuf r, p, q, state, scratch; // scratch: double[2 * kCgGrid] + ticket
+  DevBuf sync;                    // exchange words of the one-launch loop
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   const void *gx = nullptr; // the x the graph was captured with
@@ -345,6 +336,45 @@ drb_status capture_block(Csr &A, CgPlan &C, T *x) {
   return DRB_OK;
 }
 
+void report(const CgState &h, drb_cg_info *info) {
+  if (!info)
+    return;
+  info->iterations = h.iters;
+  info->residual_norm = std::sqrt(h.rr);
+  info->b_norm = std::sqrt(h.bb);
+  info->converged = h.done == kConverged;
+  info->breakdown = h.done == kBreakdown;
+}
+
+// Waits for the one-launch loop, whose first launch is queued, and launches it
+// again while the solve runs.
+template <class T>
+drb_status finish_resident(Csr &A, CgPlan &C, const T *b, T *x, double rtol, int64_t max_iters,
+                           drb_cg_info *info, cudaStream_t s) {
+  auto *st = C.state.as<CgState>();
+  for (;;) {
+    // one host round trip: the state and the error word behind the launch
+    int *err = reinterpret_cast<int *>(&C.host[1]);
+    DRB_CUDA_TRY(cudaMemcpyAsync(&C.host[0], st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
+    DRB_CUDA_TRY(
+        cudaMemcpyAsync(err, A.pipe.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    DRB_CUDA_TRY(cudaStreamSynchronize(s));
+    if (*err != 0)
+      return pipe_check(A, s); // reports and clears it
+    if (C.host[0].done != kRunning)
+      break;
+    bool launched = false;
+    DRB_TRY(cg_resident_launch<T>(A, b, x, C.r.as<T>(), C.p.as<T>(), C.q.as<T>(), st, C.sync.p,
+                                  rtol, max_iters, false, &launched, s));
+    if (!launched) {
+      set_error("drb_csr_cg: the grid no longer fits the device");
+      return DRB_ERR_CUDA;
+    }
+  }
+  report(C.host[0], info);
+  return DRB_OK;
+}
+
 template <class T>
 drb_status solve(Csr &A, const T *b, T *x, int64_t max_iters, double rtol,
                  drb_cg_info *info, cudaStream_t s) {
@@ -367,10 +397,20 @@ drb_status solve(Csr &A, const T *b, T *x, int64_t max_iters, double rtol,
     for (cudaEvent_t &e : C.ev)
       DRB_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
-  DRB_TRY(fused_scratch(A)); // allocated before any capture
   auto *st = C.state.as<CgState>();
   double *partials = C.scratch.as<double>();
   int *ticket = reinterpret_cast<int *>(partials + 2 * kCgGrid);
+
+  bool resident = cg_resident_wanted(A);
+  if (resident) {
+    if (!C.sync.p)
+      DRB_TRY(C.sync.alloc(cg_resident_sync_bytes()));
+    DRB_TRY(cg_resident_launch<T>(A, b, x, C.r.as<T>(), C.p.as<T>(), C.q.as<T>(), st, C.sync.p,
+                                  rtol, max_iters, true, &resident, s));
+  }
+  if (resident)
+    return finish_resident<T>(A, C, b, x, rtol, max_iters, info, s);
+  DRB_TRY(fused_scratch(A)); // allocated before any capture
 
   // r = b - A x0, p = r
   DRB_TRY(spmv_pipe_launch(A, x, C.q.p, s));
@@ -407,13 +447,7 @@ drb_status solve(Csr &A, const T *b, T *x, int64_t max_iters, double rtol,
   CgState h;
   DRB_CUDA_TRY(cudaMemcpy(&h, st, sizeof(CgState), cudaMemcpyDeviceToHost));
   DRB_TRY(pipe_check(A, s));
-  if (info) {
-    info->iterations = h.iters;
-    info->residual_norm = std::sqrt(h.rr);
-    info->b_norm = std::sqrt(h.bb);
-    info->converged = h.done == kConverged;
-    info->breakdown = h.done == kBreakdown;
-  }
+  report(h, info);
   return DRB_OK;
 }
 
