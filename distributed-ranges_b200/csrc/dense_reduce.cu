@@ -222,16 +222,46 @@ drb_status dense_row(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, 
 
 // ---- dot -------------------------------------------------------------------------
 constexpr int kDotNT = 256;
-constexpr int kDotGrid = 592; // fixed: the summation order must not vary
+constexpr int kDotGrid = 592; // at most; a function of n only: the order must not vary
 constexpr int kDotUnroll = 4; // 16-byte loads in flight per vector per thread
 
-template <class V>
+// The CTA's sum of v, in thread 0.
+__device__ __forceinline__ double dot_cta_sum(double v) {
+  __shared__ double s_red[kDotNT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  v = warp_sum_d(v);
+  __syncthreads(); // (an earlier sum's values have been read)
+  if (lane == 0)
+    s_red[warp] = v;
+  __syncthreads();
+  double s = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kDotNT / 32; w++)
+      s += s_red[w];
+  return s;
+}
+
+// The partials of a dot in a fixed order, in thread 0.
+__device__ __forceinline__ double dot_partials_sum(const double *partials, int count) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < count; i += kDotNT)
+    s += __ldcg(&partials[i]);
+  return dot_cta_sum(s);
+}
+
+// HBM-bound (two streams, 2 n sizeof(T) bytes).  Every trip issues all its loads
+// first, the last, partial one too: left to single loads it was up to three
+// more memory latencies, a sixth of the time at 40 MB a vector.  With TICKET the
+// last CTA adds the partials; without it dot_finish does, whose launch overlaps
+// this kernel (a ticket needs a memset before every call: a launch and its gap,
+// about 2 us).  One CTA writes the result itself.
+template <class V, bool TICKET>
 __global__ void __launch_bounds__(kDotNT)
     dot_kernel(int64_t n, const V *__restrict__ a, const V *__restrict__ b,
                double *partials, int *ticket, double *out) {
-  __shared__ double s_red[kDotNT / 32];
-  __shared__ int s_last;
   constexpr int PER = 16 / sizeof(V);
+  if (!TICKET)
+    ptx::grid_dependents_start();
   const uint64_t pol_s = ptx::policy_evict_first();
   double acc = 0.0;
   const int64_t tid = (int64_t)blockIdx.x * kDotNT + threadIdx.x;
@@ -245,8 +275,14 @@ __global__ void __launch_bounds__(kDotNT)
       V t[PER];
     };
     const int64_t nv = n / PER;
+    auto add = [&](const W (&wa)[kDotUnroll], const W (&wb)[kDotUnroll]) {
+#pragma unroll
+      for (int u = 0; u < kDotUnroll; u++)
+#pragma unroll
+        for (int q = 0; q < PER; q++)
+          acc += (double)wa[u].t[q] * (double)wb[u].t[q];
+    };
     int64_t i = tid;
-    // kDotUnroll grid-strided vectors per trip, all loads issued first
     for (; i + (kDotUnroll - 1) * nth < nv; i += kDotUnroll * nth) {
       W wa[kDotUnroll], wb[kDotUnroll];
 #pragma unroll
@@ -255,58 +291,55 @@ __global__ void __launch_bounds__(kDotNT)
 #pragma unroll
       for (int u = 0; u < kDotUnroll; u++)
         wb[u].u = (a == b) ? wa[u].u : ptx::ld_stream16(b + (i + u * nth) * PER, pol_s);
-#pragma unroll
-      for (int u = 0; u < kDotUnroll; u++)
-#pragma unroll
-        for (int q = 0; q < PER; q++)
-          acc += (double)wa[u].t[q] * (double)wb[u].t[q];
+      add(wa, wb);
     }
-    for (; i < nv; i += nth) {
-      W wa, wb;
-      wa.u = ptx::ld_stream16(a + i * PER, pol_s);
-      wb.u = (a == b) ? wa.u : ptx::ld_stream16(b + i * PER, pol_s);
+    if (i < nv) { // the last trip: places past the end count as 0
+      W wa[kDotUnroll], wb[kDotUnroll];
 #pragma unroll
-      for (int q = 0; q < PER; q++)
-        acc += (double)wa.t[q] * (double)wb.t[q];
+      for (int u = 0; u < kDotUnroll; u++) {
+        const int64_t at = i + u * nth < nv ? i + u * nth : i;
+        wa[u].u = ptx::ld_stream16(a + at * PER, pol_s);
+        wb[u].u = ptx::ld_stream16(b + at * PER, pol_s);
+      }
+#pragma unroll
+      for (int u = 1; u < kDotUnroll; u++)
+        if (i + u * nth >= nv)
+          wa[u].u = wb[u].u = make_uint4(0, 0, 0, 0);
+      add(wa, wb);
     }
     done = nv * PER;
   }
   for (int64_t i = done + tid; i < n; i += nth)
     acc += (double)a[i] * (double)b[i];
-  // block reduction
-  acc = warp_sum_d(acc);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-    s_red[warp] = acc;
-  __syncthreads();
+  const double cta = dot_cta_sum(acc);
+  if (gridDim.x == 1 || !TICKET) {
+    if (threadIdx.x == 0)
+      *(gridDim.x == 1 ? out : partials + blockIdx.x) = cta;
+    return;
+  }
+  __shared__ int s_last;
   if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < kDotNT / 32; w++)
-      s += s_red[w];
-    partials[blockIdx.x] = s;
+    partials[blockIdx.x] = cta;
     __threadfence();
     s_last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
   }
   __syncthreads();
-  if (s_last) {
-    // the last CTA adds the partials with all threads in a fixed order
-    __threadfence();
-    double s = 0.0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += kDotNT)
-      s += __ldcg(&partials[i]);
-    s = warp_sum_d(s);
-    __syncthreads();
-    if (lane == 0)
-      s_red[warp] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < kDotNT / 32; w++)
-        t += s_red[w];
-      *out = t;
-      *ticket = 0;
-    }
+  if (!s_last)
+    return;
+  __threadfence();
+  const double t = dot_partials_sum(partials, (int)gridDim.x);
+  if (threadIdx.x == 0) {
+    *out = t;
+    *ticket = 0;
   }
+}
+
+__global__ void __launch_bounds__(kDotNT)
+    dot_finish(const double *partials, int count, double *out) {
+  ptx::grid_dependency_wait();
+  const double t = dot_partials_sum(partials, count);
+  if (threadIdx.x == 0)
+    *out = t;
 }
 
 // ---- dot without allocation --------------------------------------------------
@@ -412,10 +445,10 @@ drb_status dot_noalloc_launch(int64_t n, const void *a, const void *b,
   DRB_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(int), s));
   const int64_t grid = std::max<int64_t>(1, (n + kNoAllocBlock - 1) / kNoAllocBlock);
   if (dt == DRB_F32)
-    dot_kernel<float><<<(unsigned)grid, kDotNT, 0, s>>>(
+    dot_kernel<float, true><<<(unsigned)grid, kDotNT, 0, s>>>(
         n, (const float *)a, (const float *)b, scratch, ticket, out);
   else
-    dot_kernel<double><<<(unsigned)grid, kDotNT, 0, s>>>(
+    dot_kernel<double, true><<<(unsigned)grid, kDotNT, 0, s>>>(
         n, (const double *)a, (const double *)b, scratch, ticket, out);
   note_launch();
   DRB_CUDA_TRY(cudaGetLastError());
@@ -448,23 +481,28 @@ drb_status dot_launch(int64_t n, const void *a, const void *b, drb_dtype dt,
     set_error("dot: dtype %d not supported", (int)dt);
     return DRB_ERR_UNSUPPORTED;
   }
+  // one CTA up to 16384 elements (its result needs no scratch and no second
+  // pass), then one per 4096 up to four per SM
+  const int grid = (int)(n <= 16384 ? 1 : std::min<int64_t>(kDotGrid, (n + 4095) / 4096));
   void *scratch = nullptr;
-  const size_t bytes = sizeof(double) * kDotGrid + 16;
-  DRB_TRY(scratch_alloc(&scratch, bytes, s));
+  if (grid > 1)
+    DRB_TRY(scratch_alloc(&scratch, sizeof(double) * kDotGrid, s));
   double *partials = static_cast<double *>(scratch);
-  int *ticket = reinterpret_cast<int *>(partials + kDotGrid);
-  cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(int), s);
-  if (e == cudaSuccess) {
-    if (dt == DRB_F32)
-      dot_kernel<float><<<kDotGrid, kDotNT, 0, s>>>(
-          n, (const float *)a, (const float *)b, partials, ticket, out);
-    else
-      dot_kernel<double><<<kDotGrid, kDotNT, 0, s>>>(
-          n, (const double *)a, (const double *)b, partials, ticket, out);
+  if (dt == DRB_F32)
+    dot_kernel<float, false><<<grid, kDotNT, 0, s>>>(n, (const float *)a, (const float *)b,
+                                                     partials, nullptr, out);
+  else
+    dot_kernel<double, false><<<grid, kDotNT, 0, s>>>(n, (const double *)a, (const double *)b,
+                                                      partials, nullptr, out);
+  note_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && grid > 1) {
+    e = launch_overlapped(dot_finish, dim3(1), dim3(kDotNT), 0, s,
+                          (const double *)partials, grid, out);
     note_launch();
-    e = cudaGetLastError();
   }
-  scratch_free(scratch, s);
+  if (scratch)
+    scratch_free(scratch, s);
   if (e != cudaSuccess) {
     set_error("dot launch: %s", cudaGetErrorString(e));
     return DRB_ERR_CUDA;

@@ -6,10 +6,11 @@
 // (or on every rank), then applies `init` last: binary_op(init, reduce(r))
 // (reduce.hpp:110-120); an empty range gives init, or value_type{} without
 // one (reduce.hpp:63-65).  Here every segment is on one GPU, so the reduce is
-// one launch: a fixed grid of kRedGrid CTAs, each thread striding over the
-// vector with 16-byte loads, a per-CTA tree, and the last CTA (completion
-// ticket) combining the per-CTA partials in index order.  The grouping
-// depends only on n and x's address modulo 16, so results are deterministic.
+// one launch: a grid of at most kRedGrid CTAs, each thread striding over the
+// vector with 16-byte loads, a per-CTA tree, and a one-CTA kernel, whose launch
+// overlaps, combining the per-CTA partials in index order (one CTA writes the
+// result itself).  The grouping depends only on n and x's address modulo 16, so
+// results are deterministic.
 //
 // Accumulation: integer sums wrap modulo 2^32 / 2^64 (two's-complement
 // addition is associative, so the result equals the sequential loop's
@@ -81,15 +82,33 @@ template <class A> __device__ __forceinline__ A shfl_down(A v, int o) {
   return __shfl_down_sync(0xffffffffu, v, o);
 }
 
+// The CTA's reduction of acc, in thread 0.
+template <class R> __device__ __forceinline__ typename R::A cta_reduce(typename R::A acc) {
+  using A = typename R::A;
+  __shared__ A s_red[kRedNT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int o = 16; o > 0; o >>= 1)
+    acc = R::f(acc, shfl_down(acc, o));
+  if (lane == 0)
+    s_red[warp] = acc;
+  __syncthreads();
+  A s = R::id();
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kRedNT / 32; w++)
+      s = R::f(s, s_red[w]);
+  return s;
+}
+
+// HBM-bound: one stream.  Every trip issues its loads first, the partial last
+// one too (single loads there were up to three more memory latencies).
 template <class T, int OP>
 __global__ void __launch_bounds__(kRedNT)
     reduce_kernel(int64_t n, const T *__restrict__ x, bool has_init, T init,
-                  typename ROp<T, OP>::A *partials, int *ticket, T *out) {
+                  typename ROp<T, OP>::A *partials, T *out) {
   using R = ROp<T, OP>;
   using A = typename R::A;
-  __shared__ A s_red[kRedNT / 32];
-  __shared__ int s_last;
   constexpr int PER = 16 / sizeof(T);
+  ptx::grid_dependents_start();
   const uint64_t pol = ptx::policy_evict_first();
   A acc = R::id();
   const int64_t tid = (int64_t)blockIdx.x * kRedNT + threadIdx.x;
@@ -106,7 +125,6 @@ __global__ void __launch_bounds__(kRedNT)
       T t[PER];
     };
     int64_t i = tid;
-    // kRedUnroll grid-strided vectors per trip, all loads issued first
     for (; i + (kRedUnroll - 1) * nth < nv; i += kRedUnroll * nth) {
       W w[kRedUnroll];
 #pragma unroll
@@ -118,12 +136,16 @@ __global__ void __launch_bounds__(kRedNT)
         for (int q = 0; q < PER; q++)
           acc = R::f(acc, R::lift(w[u].t[q]));
     }
-    for (; i < nv; i += nth) {
-      W w;
-      w.u = ptx::ld_stream16(xa + i * PER, pol);
+    if (i < nv) { // the last trip: places past the end read the first one again
+      W w[kRedUnroll];
 #pragma unroll
-      for (int q = 0; q < PER; q++)
-        acc = R::f(acc, R::lift(w.t[q]));
+      for (int u = 0; u < kRedUnroll; u++)
+        w[u].u = ptx::ld_stream16(xa + (i + u * nth < nv ? i + u * nth : i) * PER, pol);
+#pragma unroll
+      for (int u = 0; u < kRedUnroll; u++)
+#pragma unroll
+        for (int q = 0; q < PER; q++)
+          acc = R::f(acc, i + u * nth < nv ? R::lift(w[u].t[q]) : R::id());
     }
     for (int64_t i = head + nv * PER + tid; i < n; i += nth)
       acc = R::f(acc, R::lift(x[i]));
@@ -133,40 +155,28 @@ __global__ void __launch_bounds__(kRedNT)
     for (int64_t i = tid; i < n; i += nth)
       acc = R::f(acc, R::lift(x[i]));
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1)
-    acc = R::f(acc, shfl_down(acc, o));
-  if (lane == 0)
-    s_red[warp] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    A s = R::id();
-    for (int w = 0; w < kRedNT / 32; w++)
-      s = R::f(s, s_red[w]);
-    partials[blockIdx.x] = s;
-    __threadfence();
-    s_last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!s_last)
+  const A s = cta_reduce<R>(acc);
+  if (threadIdx.x != 0)
     return;
-  __threadfence();
-  A s = R::id();
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kRedNT)
+  if (gridDim.x > 1)
+    partials[blockIdx.x] = s;
+  else
+    *out = n > 0 ? R::out(s, has_init, init) : (has_init ? init : T(0));
+}
+
+// The partials (of a non-empty vector) in index order.
+template <class T, int OP>
+__global__ void __launch_bounds__(kRedNT)
+    reduce_finish(const typename ROp<T, OP>::A *partials, int count, bool has_init, T init,
+                  T *out) {
+  using R = ROp<T, OP>;
+  ptx::grid_dependency_wait();
+  typename R::A s = R::id();
+  for (int i = threadIdx.x; i < count; i += kRedNT)
     s = R::f(s, __ldcg(&partials[i]));
-  for (int o = 16; o > 0; o >>= 1)
-    s = R::f(s, shfl_down(s, o));
-  __syncthreads();
-  if (lane == 0)
-    s_red[warp] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    A t = R::id();
-    for (int w = 0; w < kRedNT / 32; w++)
-      t = R::f(t, s_red[w]);
-    *out = n > 0 ? R::out(t, has_init, init) : (has_init ? init : T(0));
-    *ticket = 0;
-  }
+  s = cta_reduce<R>(s);
+  if (threadIdx.x == 0)
+    *out = R::out(s, has_init, init);
 }
 
 template <class T, int OP>
@@ -176,22 +186,25 @@ drb_status reduce_typed(int64_t n, const void *x, const void *init, void *out,
   T iv{};
   if (init)
     std::memcpy(&iv, init, sizeof(T));
+  // one CTA up to 16384 elements (no scratch, no second pass), then one per 4096
+  // up to four per SM: a function of n only
+  const int grid =
+      (int)(n <= 16384 ? 1 : std::min<int64_t>(kRedGrid, (n + kRedNT * 16 - 1) / (kRedNT * 16)));
   void *scratch = nullptr;
-  const size_t bytes = sizeof(A) * kRedGrid + 16;
-  DRB_TRY(scratch_alloc(&scratch, bytes, s));
+  if (grid > 1)
+    DRB_TRY(scratch_alloc(&scratch, sizeof(A) * kRedGrid, s));
   A *partials = static_cast<A *>(scratch);
-  int *ticket = reinterpret_cast<int *>(partials + kRedGrid);
-  cudaError_t e = cudaMemsetAsync(ticket, 0, sizeof(int), s);
-  if (e == cudaSuccess) {
-    // small inputs take fewer CTAs; the grid is still a function of n only
-    const int64_t want = (n + kRedNT * 16 - 1) / (kRedNT * 16);
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(kRedGrid, want));
-    reduce_kernel<T, OP><<<grid, kRedNT, 0, s>>>(n, static_cast<const T *>(x), init != nullptr,
-                                                 iv, partials, ticket, static_cast<T *>(out));
+  reduce_kernel<T, OP><<<grid, kRedNT, 0, s>>>(n, static_cast<const T *>(x), init != nullptr, iv,
+                                               partials, static_cast<T *>(out));
+  note_launch();
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && grid > 1) {
+    e = launch_overlapped(reduce_finish<T, OP>, dim3(1), dim3(kRedNT), 0, s,
+                          (const A *)partials, grid, init != nullptr, iv, static_cast<T *>(out));
     note_launch();
-    e = cudaGetLastError();
   }
-  scratch_free(scratch, s);
+  if (scratch)
+    scratch_free(scratch, s);
   if (e != cudaSuccess) {
     set_error("reduce launch: %s", cudaGetErrorString(e));
     return DRB_ERR_CUDA;
