@@ -371,7 +371,8 @@ drb_status build_typed(Csr &A, cudaStream_t s) {
   DRB_TRY(build_plan(T.plan, T.m, cp.data(), sizeof(RI),
                      plan_group(dtype_bytes(T.storage), T.cbytes), 0, 0, 0));
   DRB_TRY(build_pipe_plan(T.pipe, T.m, cp.data(), sizeof(RI),
-                          plan_group(dtype_bytes(T.storage), T.cbytes), 0, 0));
+                          plan_group(dtype_bytes(T.storage), T.cbytes),
+                          default_pipe_variant(T), 0));
   // A^T of a short-row matrix (a stencil) has short rows too: x-bar then
   // runs on its sliced-ELL copy, as the forward product does
   DRB_TRY(sell_build(T, cp.data(), sizeof(RI), s));

@@ -177,8 +177,12 @@ struct PipePlan {
   uint64_t gen = 0; // bumped by every (re)build
 };
 
+struct Csr;
 drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
                            int rbytes, int group, int tile, int rows);
+// The kernel variant (tile | 2 two-slot | 1 skewed) of a plan for A that was not
+// autotuned.
+int default_pipe_variant(const Csr &A);
 // Elements per 16-byte vector group of a plan over values of vbytes and
 // column indices of cbytes.
 int plan_group(int vbytes, int cbytes);

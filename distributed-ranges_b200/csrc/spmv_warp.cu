@@ -20,15 +20,22 @@ using warpk::WarpResid;
 // argument (0 = choose).  The choice does not change results beyond the
 // summation order of a chunked row, which is the same for both layouts.
 //
-// Default (measured on B200, random columns, 336M nonzeros, 64 MB x):
-// 256-nonzero items with the skewed layout are fastest or tied at every row
-// length (fixed rows of 16..4096 nonzeros: 1.33-1.49 ms; the bench's
-// power-law: 1.61 ms against 1.97 ms for 512-nonzero items) once chunked
-// rows finish in a separate pass.  The environment variable
+// Default (measured on B200, power-law rows with random columns; us per product,
+// 256- against 128-nonzero items, skewed): the smaller items keep more warps on
+// an SM and end more evenly,
+//   FP32, 0.3M / 2M / 13.4M rows (in two column blocks)  52.2 / 188 / 617
+//         against 44.6 / 184 / 539;
+//   FP64, 0.3M rows 58.9 / 53.7, 8.4M columns (64 MB x) unsplit 454 / 428, in
+//         blocks 483 / 467.
+// They cost an item descriptor twice as often, so 256 stays where x is in L2
+// and the matrix is large enough to fill the GPU either way in FP64 (1.5M rows
+// 167 / 166, 5M 490 / 505), for compensated sums (143 / 145) and for FP64 handles
+// with an adjoint, whose abar runs on the same items (1.5M rows, residual and
+// backward 525 / 537; 6M 1894 / 1990).  The environment variable
 // DRB_SPMV_VARIANT="tile,skew" (e.g. "512,0") overrides it for handles
 // created afterwards ("128,1,1": the two-slot kernel); drb_csr_autotune
 // measures them all instead.
-int choose_pipe_variant(int64_t, const void *, int) {
+int default_pipe_variant(const Csr &A) {
   if (const char *e = std::getenv("DRB_SPMV_VARIANT")) {
     const int t = std::atoi(e);
     const char *c = std::strchr(e, ',');
@@ -38,14 +45,17 @@ int choose_pipe_variant(int64_t, const void *, int) {
     if (t == 128 || t == 256 || t == 512)
       return t | (sk ? 1 : 0) | (two ? 2 : 0);
   }
+  if (A.storage == DRB_F32)
+    return (A.flags & DRB_FLAG_COMPENSATED) ? 256 | 1 : 128 | 1;
+  const bool fills = A.nnz >= 12000000, in_l2 = A.n * 8 <= (int64_t)48 << 20;
+  if (A.storage == DRB_F64 && !(A.flags & DRB_FLAG_ADJOINT) && !(fills && in_l2))
+    return 128 | 1;
   return 256 | 1;
 }
 
 drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
                            int rbytes, int group, int tile, int rows) {
   plan.gen++; // graphs captured over the old items are stale
-  if (tile == 0)
-    tile = choose_pipe_variant(m, rowptr_host, rbytes);
   plan.skew = (tile & 1) != 0;
   plan.two_slot = (tile & 2) != 0;
   tile &= ~3;
