@@ -15,7 +15,7 @@
 //
 // Measured (64 iterations on a g x g Laplacian, us, launch per step -> here):
 // f64 g = 48 787 -> 491, 512 1455 -> 801, 1024 2386 -> 1343, 1448 3672 -> 3000,
-// 1800 5462 -> 4502; f32 300 1088 -> 720, 1024 2134 -> 1417, 1800 3954 -> 3677.
+// 1800 5462 -> 4502; f32 300 1088 -> 720, 1024 2134 -> 1307, 1448 2979 -> 2353.
 // What is left at small sizes is the chain of three grid-wide steps (about 5 us
 // of 11 an iteration on all SMs), at large ones the matrix's bytes.
 //
@@ -39,8 +39,11 @@
 namespace drb {
 namespace {
 
-constexpr int kResNT = 768;
-constexpr int kResWarps = kResNT / 32;
+// Threads per CTA.  f64 needs 80 registers; f32 fits 64 and gains from more
+// warps once each has several slices a phase (64 iterations at g = 1024 1419 ->
+// 1307 us, 1448 2655 -> 2353; g = 300 726 -> 763).
+constexpr int kResNT = 768, kResNTMany = 1024;
+constexpr int kResManySlices = 64; // slices per CTA from which f32 takes 1024
 constexpr int kResMinSlices = 16;  // slices per CTA at least, for small systems
 constexpr int kResMaxCtas = 256;   // exchange slots
 constexpr int kResDirect = 32;     // CTAs that read each other's sums directly
@@ -90,11 +93,12 @@ __device__ __forceinline__ int ld_mat(const int *p, uint64_t pol) {
 }
 
 // The grid's CTAs as one group (all resident: cooperative launch).
-struct Grid {
+template <int NT> struct Grid {
+  static constexpr int W = NT / 32;
   ulonglong2 *slots;
   unsigned *count;
   int *err;
-  double *s_red;  // [kResWarps]
+  double *s_red;  // [W]
   double *s_sum;  // [kResMaxCtas / 32]
   int *s_stop;
   unsigned epoch = 0, arrived = 0; // exchanges, barrier arrivals so far
@@ -148,7 +152,7 @@ struct Grid {
     ulonglong2 *slot = slots + (epoch & 1) * kResMaxCtas;
     ulonglong2 *copies = slots + 2 * kResMaxCtas + (epoch & 1) * kResCopies * 8;
     if (warp == 0) {
-      const double t = warp_down(lane < kResWarps ? s_red[lane] : 0.0);
+      const double t = warp_down(lane < W ? s_red[lane] : 0.0);
       if (lane == 0) {
         if (G == 1)
           s_sum[0] = t;
@@ -203,10 +207,11 @@ struct Grid {
   }
 };
 
-template <class T>
-__global__ void __launch_bounds__(kResNT, 1) cg_resident(const ResArgs<T> a) {
+template <class T, int NT>
+__global__ void __launch_bounds__(NT, 1) cg_resident(const ResArgs<T> a) {
+  constexpr int W = NT / 32;
   extern __shared__ __align__(16) unsigned char res_mem[];
-  __shared__ double s_red[kResWarps], s_sum[(kResMaxCtas + 31) / 32];
+  __shared__ double s_red[W], s_sum[(kResMaxCtas + 31) / 32];
   __shared__ int s_stop;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t s0 = a.ns * blockIdx.x / gridDim.x, s1 = a.ns * (blockIdx.x + 1) / gridDim.x;
@@ -225,16 +230,16 @@ __global__ void __launch_bounds__(kResNT, 1) cg_resident(const ResArgs<T> a) {
   const int64_t obase = a.off[s0];
   if (tid == 0)
     s_stop = 0;
-  for (int i = tid; i <= nsl; i += kResNT)
+  for (int i = tid; i <= nsl; i += NT)
     soff[i] = (int)(a.off[s0 + i] - obase);
-  Grid G{a.slots, a.count, a.err, s_red, s_sum, &s_stop};
+  Grid<NT> G{a.slots, a.count, a.err, s_red, s_sum, &s_stop};
   const uint64_t pol = a.keep ? ptx::policy_evict_last() : ptx::policy_evict_first();
   __syncthreads();
 
   // The matrix runs ahead of its use: a slice's first K entries per row load
   // while the previous slice's gathers are in flight, those of the warp's first
   // slice while the CTA waits for the others' part of the vector.
-  constexpr int K = sizeof(T) == 4 ? 8 : 6;
+  constexpr int K = 6;
   struct Part {
     T e[K];
     int c[K];
@@ -271,10 +276,10 @@ __global__ void __launch_bounds__(kResNT, 1) cg_resident(const ResArgs<T> a) {
         if (s.c[k] >= 0)
           acc += s.e[k] * g[k];
     };
-    for (int i = warp; i < nsl; i += kResWarps) {
+    for (int i = warp; i < nsl; i += W) {
       Part cur = ahead;
-      if (i + kResWarps < nsl)
-        fetch(ahead, i + kResWarps, 0);
+      if (i + W < nsl)
+        fetch(ahead, i + W, 0);
       T acc = 0;
       add(cur, acc);
       const int w = (soff[i + 1] - soff[i]) >> 5;
@@ -290,15 +295,15 @@ __global__ void __launch_bounds__(kResNT, 1) cg_resident(const ResArgs<T> a) {
   // f(local row) over this CTA's rows, U at a time: load(row, u) first
   constexpr int U = sizeof(T) == 4 ? 4 : 2; // (64 registers per thread)
   auto each = [&](auto load, auto f) {
-    for (int i = tid; i < rows; i += U * kResNT) {
+    for (int i = tid; i < rows; i += U * NT) {
 #pragma unroll
       for (int u = 0; u < U; u++)
-        if (i + u * kResNT < rows)
-          load(i + u * kResNT, u);
+        if (i + u * NT < rows)
+          load(i + u * NT, u);
 #pragma unroll
       for (int u = 0; u < U; u++)
-        if (i + u * kResNT < rows)
-          f(i + u * kResNT, u);
+        if (i + u * NT < rows)
+          f(i + u * NT, u);
     }
   };
 
@@ -319,7 +324,7 @@ __global__ void __launch_bounds__(kResNT, 1) cg_resident(const ResArgs<T> a) {
       s_bb += (double)bi * (double)bi;
     });
     if (a.nres > 2)
-      for (int i = tid; i < rows; i += kResNT)
+      for (int i = tid; i < rows; i += NT)
         vx[i] = a.x[row0 + i];
     if (!G.sum(s_rr, rr) || !G.sum(s_bb, bb))
       return;
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(kResNT, 1) cg_resident(const ResArgs<T> a) {
     tol2 = a.st->tol2;
     it = a.st->iters;
     done = kRunning;
-    for (int i = tid; i < rows; i += kResNT) {
+    for (int i = tid; i < rows; i += NT) {
       if (a.nres > 0)
         vr[i] = a.r[row0 + i];
       if (a.nres > 2)
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(kResNT, 1) cg_resident(const ResArgs<T> a) {
     }
   }
 
-  for (int i = tid; i < rows; i += kResNT) {
+  for (int i = tid; i < rows; i += NT) {
     if (a.nres > 2)
       a.x[row0 + i] = vx[i];
     if (a.nres > 0 && done == kRunning)
@@ -424,11 +429,12 @@ constexpr size_t kSyncBytes =
     (2 * kResMaxCtas + 2 * kResCopies * 8) * sizeof(ulonglong2) + sizeof(unsigned);
 
 template <class T> struct ResShape {
-  int grid = 0, cap = 0, nres = 0;
+  const void *kernel = nullptr;
+  int grid = 0, threads = 0, cap = 0, nres = 0;
   size_t smem = 0;
 };
 
-template <class T> drb_status res_shape(const Csr &A, ResShape<T> &S) {
+template <class T, int NT> drb_status res_shape(const Csr &A, ResShape<T> &S) {
   static int limits[64][2]; // SMs, shared memory of a CTA (0: not read yet)
   const int d = A.device < 64 ? A.device : 0;
   if (limits[d][0] == 0 || A.device >= 64) {
@@ -437,14 +443,16 @@ template <class T> drb_status res_shape(const Csr &A, ResShape<T> &S) {
     DRB_CUDA_TRY(
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, A.device));
     cudaFuncAttributes fa;
-    DRB_CUDA_TRY(cudaFuncGetAttributes(&fa, cg_resident<T>));
+    DRB_CUDA_TRY(cudaFuncGetAttributes(&fa, cg_resident<T, NT>));
     const int dyn = optin - (int)fa.sharedSizeBytes;
-    DRB_CUDA_TRY(cudaFuncSetAttribute(cg_resident<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      dyn));
+    DRB_CUDA_TRY(cudaFuncSetAttribute(cg_resident<T, NT>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
     limits[d][1] = dyn;
     limits[d][0] = sms;
   }
   const int64_t ns = A.sell.nslices;
+  S.kernel = reinterpret_cast<const void *>(cg_resident<T, NT>);
+  S.threads = NT;
   S.grid = (int)std::max<int64_t>(
       1, std::min<int64_t>(std::min(limits[d][0], kResMaxCtas), ns / kResMinSlices));
   S.cap = (int)((ns + S.grid - 1) / S.grid);
@@ -472,7 +480,10 @@ drb_status cg_resident_launch(Csr &A, const T *b, T *x, T *r, T *p, T *q, CgStat
                               bool *launched, cudaStream_t s) {
   *launched = false;
   ResShape<T> S;
-  DRB_TRY(res_shape<T>(A, S));
+  DRB_TRY((res_shape<T, kResNT>(A, S)));
+  if constexpr (sizeof(T) == 4)
+    if (S.cap >= kResManySlices)
+      DRB_TRY((res_shape<T, kResNTMany>(A, S)));
   ResArgs<T> a;
   a.vals = A.sell.vals.as<T>();
   a.cols = A.sell.cols.as<int>();
@@ -497,8 +508,7 @@ drb_status cg_resident_launch(Csr &A, const T *b, T *x, T *r, T *p, T *q, CgStat
   DRB_CUDA_TRY(cudaMemsetAsync(sync, 0, kSyncBytes, s));
   void *args[] = {&a};
   const cudaError_t e = cudaLaunchCooperativeKernel(
-      reinterpret_cast<const void *>(cg_resident<T>), dim3((unsigned)S.grid), dim3(kResNT), args,
-      S.smem, s);
+      S.kernel, dim3((unsigned)S.grid), dim3((unsigned)S.threads), args, S.smem, s);
   if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
     cudaGetLastError(); // fewer SMs than the device reports: the graph path
     return DRB_OK;
