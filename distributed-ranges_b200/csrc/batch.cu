@@ -197,14 +197,21 @@ __device__ __forceinline__ int clog2(int x) {
   return ilog2(x) + ((x & (x - 1)) ? 1 : 0);
 }
 
-constexpr int kUnroll = 4; // X gathers in flight per lane
+// X gathers in flight per lane: 4, three CTAs per SM; with five or more lanes per
+// slot, not a power of two (at most six slots, one per row), 8, two CTAs per SM.
+// There rows are long chains of rounds in few slots, and each round waits for
+// its gathers: 0.5M rows of 8..64, f32, k = 28 502 -> 392 us, k = 33 719 -> 543,
+// f64 k = 20 795 -> 755; with fewer lanes a slot more warps do better (f32 k =
+// 12 202 -> 216, k = 16 547 -> 578, k = 8 144 -> 161).  BF16 storage keeps 4, the
+// block of its compensated sums.
+template <class V> constexpr int unroll_of(bool wide) { return wide && sizeof(V) > 2 ? 8 : 4; }
 
-// BF16 storage sums two-sum compensated, per block of the kUnroll products a
+// BF16 storage sums two-sum compensated, per block of the four products a
 // lane has in flight: the block is one chain of fused multiply-adds (at most
-// kUnroll roundings, each within u of the block's sum of |a x|), and the
+// four roundings, each within u of the block's sum of |a x|), and the
 // block sum enters the row's running sum through a two-sum whose exact error
 // goes to a compensation term, added when the row completes.  So a row's
-// error stays within about (kUnroll + 1) u of sum |a x| however long the row
+// error stays within about 5 u of sum |a x| however long the row
 // (plain f32 sums grow with its length), for about a third of the
 // arithmetic of a two-sum per product.  The operations are the _rn
 // intrinsics, which the compiler never contracts or reorders.
@@ -271,9 +278,9 @@ __device__ __forceinline__ uint64_t x_pair(const XWords<XT, VEC> &o, int p) {
 
 // The nonzeros [b, e) of one row staged at shared addresses colS/valS (byte
 // address of stage element 0), this lane's VEC sums (and, compensated, their
-// error terms cmp); the lane takes b, b + step, ... with kUnroll gathers in
+// error terms cmp); the lane takes b, b + step, ... with UN gathers in
 // flight.  f32 sums of an even VEC run on packed pairs.
-template <class V, class XT, int VEC, class A>
+template <class V, class XT, int VEC, int UN, class A>
 __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
                                          int e, const XT *Xl, int ldx,
                                          int step, A (&acc)[VEC], A (&cmp)[VEC]) {
@@ -287,12 +294,12 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
     }
     // bf16 values and bf16 X: the block's chains run on the bf16 operands
     constexpr bool kMixed = Comp<V>::value && sizeof(XT) == 2;
-    for (int q = b; q < e; q += kUnroll * step) {
-      XWords<XT, VEC> xv[kUnroll];
-      uint64_t v2[kUnroll];
-      uint16_t vb[kUnroll];
+    for (int q = b; q < e; q += UN * step) {
+      XWords<XT, VEC> xv[UN];
+      uint64_t v2[UN];
+      uint16_t vb[UN];
 #pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
+      for (int u = 0; u < UN; u++) {
         const int qq = min(q + u * step, e - 1); // in range; extra lanes masked
         const int32_t col = lds_s32(colS + 4 * qq);
         const V raw = lds_val<V>(valS + (uint32_t)sizeof(V) * qq);
@@ -312,7 +319,7 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
           float lo = fma_bf16(vb[0], (uint16_t)(xv[0].w[p] & 0xffffu), 0.0f);
           float hi = fma_bf16(vb[0], (uint16_t)(xv[0].w[p] >> 16), 0.0f);
 #pragma unroll
-          for (int u = 1; u < kUnroll; u++) {
+          for (int u = 1; u < UN; u++) {
             lo = fma_bf16(vb[u], (uint16_t)(xv[u].w[p] & 0xffffu), lo);
             hi = fma_bf16(vb[u], (uint16_t)(xv[u].w[p] >> 16), hi);
           }
@@ -328,7 +335,7 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
         for (int p = 0; p < P; p++) {
           uint64_t blk = mul2(v2[0], x_pair<XT, VEC>(xv[0], p));
 #pragma unroll
-          for (int u = 1; u < kUnroll; u++)
+          for (int u = 1; u < UN; u++)
             blk = fma2(v2[u], x_pair<XT, VEC>(xv[u], p), blk);
           // two-sum of the pair: s + err == a2 + blk exactly
           const uint64_t s = add2(a2[p], blk);
@@ -339,7 +346,7 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
         }
       } else {
 #pragma unroll
-        for (int u = 0; u < kUnroll; u++)
+        for (int u = 0; u < UN; u++)
 #pragma unroll
           for (int p = 0; p < P; p++)
             a2[p] = fma2(v2[u], x_pair<XT, VEC>(xv[u], p), a2[p]);
@@ -352,11 +359,11 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
     }
     return;
   }
-  for (int q = b; q < e; q += kUnroll * step) {
-    XWords<XT, VEC> xv[kUnroll];
-    A vv[kUnroll];
+  for (int q = b; q < e; q += UN * step) {
+    XWords<XT, VEC> xv[UN];
+    A vv[UN];
 #pragma unroll
-    for (int u = 0; u < kUnroll; u++) {
+    for (int u = 0; u < UN; u++) {
       const int qq = min(q + u * step, e - 1); // in range; extra lanes masked
       const int32_t col = lds_s32(colS + 4 * qq);
       const A v = to_acc(lds_val<V>(valS + (uint32_t)sizeof(V) * qq));
@@ -368,7 +375,7 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
       for (int t = 0; t < VEC; t++) {
         float blk = __fmul_rn(vv[0], x_at<XT, VEC, A>(xv[0], t));
 #pragma unroll
-        for (int u = 1; u < kUnroll; u++)
+        for (int u = 1; u < UN; u++)
           blk = __fmaf_rn(vv[u], x_at<XT, VEC, A>(xv[u], t), blk);
         float s, err;
         two_sum_rn(acc[t], blk, s, err);
@@ -377,7 +384,7 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
       }
     } else {
 #pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
+      for (int u = 0; u < UN; u++) {
 #pragma unroll
         for (int t = 0; t < VEC; t++)
           acc[t] = fma(vv[u], (x_at<XT, VEC, A>(xv[u], t)), acc[t]);
@@ -399,8 +406,8 @@ __device__ __forceinline__ void merge_sum(A &acc, A &cmp, A acc2, A cmp2) {
   }
 }
 
-template <class V, class XT, int VEC>
-__global__ void __launch_bounds__(256, 3) batch_spmm(const BArgs a) {
+template <class V, class XT, int VEC, int UN>
+__global__ void __launch_bounds__(256, UN == 4 ? 3 : 2) batch_spmm(const BArgs a) {
   using A = typename AccOf<V>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -491,7 +498,7 @@ __global__ void __launch_bounds__(256, 3) batch_spmm(const BArgs a) {
           acc[t] = cmp[t] = 0;
         if (con && row_on && i < nrows) {
           const int b = lds_s32(rsP + 4 * i) - p0, e = lds_s32(rsP + 4 * i + 4) - p0;
-          row_sums<V, XT, VEC, A>(colP, valP, b + gs, e, Xl, ldx, G, acc, cmp);
+          row_sums<V, XT, VEC, UN, A>(colP, valP, b + gs, e, Xl, ldx, G, acc, cmp);
         }
         for (int dd = 1; dd < G; dd <<= 1) {
 #pragma unroll
@@ -545,7 +552,7 @@ __global__ void __launch_bounds__(256, 3) batch_spmm(const BArgs a) {
         cp_wait<0>();
         __syncwarp();
         if (con)
-          row_sums<V, XT, VEC, A>(colS + 4 * (int)(lo & 3),
+          row_sums<V, XT, VEC, UN, A>(colS + 4 * (int)(lo & 3),
                                   valS + (uint32_t)sizeof(V) * (int)(lo & VOFF_MASK),
                                   slot, len, Xl, ldx, S, acc, cmp);
         __syncwarp();
@@ -722,37 +729,38 @@ PackFn pick_pack(int xbytes, bool colmajor, int lcw) {
 
 using KernelFn = void (*)(const BArgs);
 
-template <class V, class XT> KernelFn pick_vec(int vec) {
+template <class V, class XT, bool WIDE> KernelFn pick_vec(int vec) {
+  constexpr int UN = unroll_of<V>(WIDE);
   if constexpr (sizeof(XT) == 2) {
     switch (vec) {
-    case 2: return batch_spmm<V, XT, 2>;
-    case 4: return batch_spmm<V, XT, 4>;
-    case 8: return batch_spmm<V, XT, 8>;
+    case 2: return batch_spmm<V, XT, 2, UN>;
+    case 4: return batch_spmm<V, XT, 4, UN>;
+    case 8: return batch_spmm<V, XT, 8, UN>;
     }
   } else if constexpr (sizeof(XT) == 4) {
     switch (vec) {
-    case 1: return batch_spmm<V, XT, 1>;
-    case 2: return batch_spmm<V, XT, 2>;
-    case 4: return batch_spmm<V, XT, 4>;
+    case 1: return batch_spmm<V, XT, 1, UN>;
+    case 2: return batch_spmm<V, XT, 2, UN>;
+    case 4: return batch_spmm<V, XT, 4, UN>;
     }
   } else {
     switch (vec) {
-    case 1: return batch_spmm<V, XT, 1>;
-    case 2: return batch_spmm<V, XT, 2>;
+    case 1: return batch_spmm<V, XT, 1, UN>;
+    case 2: return batch_spmm<V, XT, 2, UN>;
     }
   }
   return nullptr;
 }
 
-KernelFn pick_kernel(drb_dtype storage, bool x_f32, int vec) {
+KernelFn pick_kernel(drb_dtype storage, bool x_f32, int vec, bool wide) {
   switch (storage) {
   case DRB_F32:
-    return pick_vec<float, float>(vec);
+    return wide ? pick_vec<float, float, true>(vec) : pick_vec<float, float, false>(vec);
   case DRB_F64:
-    return pick_vec<double, double>(vec);
+    return wide ? pick_vec<double, double, true>(vec) : pick_vec<double, double, false>(vec);
   case DRB_BF16:
-    return x_f32 ? pick_vec<uint16_t, float>(vec)
-                 : pick_vec<uint16_t, uint16_t>(vec);
+    return x_f32 ? pick_vec<uint16_t, float, false>(vec)
+                 : pick_vec<uint16_t, uint16_t, false>(vec);
   }
   return nullptr;
 }
@@ -1077,7 +1085,7 @@ drb_status make_batch(Batch &B, int32_t count, Csr *const *handles,
   B.KB = B.KP * B.vec;
   B.nkb = (B.ldx + B.KB - 1) / B.KB;
   B.rmax = std::min(kRmax, std::max(1, kYBudget / ((B.KB + 1) * B.abytes)));
-  B.kernel = pick_kernel(B.storage, B.x_f32, B.vec);
+  B.kernel = pick_kernel(B.storage, B.x_f32, B.vec, B.KP >= 5 && (B.KP & (B.KP - 1)));
   if (!B.kernel)
     return fail(DRB_ERR_UNSUPPORTED,
                 "no batch kernel for this type and vector width");
