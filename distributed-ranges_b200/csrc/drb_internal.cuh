@@ -181,8 +181,10 @@ struct Csr;
 drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
                            int rbytes, int group, int tile, int rows);
 // The kernel variant (tile | 2 two-slot | 1 skewed) of a plan for A that was not
-// autotuned.
+// autotuned, by its type, size and share of nonzeros in long rows.
 int default_pipe_variant(const Csr &A);
+constexpr int64_t kLongRowNnz = 256;
+int64_t long_row_nnz(int64_t m, const void *rowptr_host, int rbytes);
 // Elements per 16-byte vector group of a plan over values of vbytes and
 // column indices of cbytes.
 int plan_group(int vbytes, int cbytes);
@@ -219,6 +221,7 @@ struct Csr {
   int device = 0;
   int64_t m = 0, n = 0, nnz = 0;
   int64_t max_row = 0; // nonzeros in the longest row
+  int64_t long_nnz = 0; // nonzeros in rows longer than kLongRowNnz
   drb_dtype value_type = DRB_F32; // caller's element type
   drb_dtype storage = DRB_F32;    // device element type
   int cbytes = 4, rbytes = 4;     // stored index widths

@@ -20,18 +20,23 @@ using warpk::WarpResid;
 // argument (0 = choose).  The choice does not change results beyond the
 // summation order of a chunked row, which is the same for both layouts.
 //
-// Default (measured on B200, power-law rows with random columns; us per product,
-// 256- against 128-nonzero items, skewed): the smaller items keep more warps on
-// an SM and end more evenly,
-//   FP32, 0.3M / 2M / 13.4M rows (in two column blocks)  52.2 / 188 / 617
-//         against 44.6 / 184 / 539;
-//   FP64, 0.3M rows 58.9 / 53.7, 8.4M columns (64 MB x) unsplit 454 / 428, in
-//         blocks 483 / 467.
-// They cost an item descriptor twice as often, so 256 stays where x is in L2
-// and the matrix is large enough to fill the GPU either way in FP64 (1.5M rows
-// 167 / 166, 5M 490 / 505), for compensated sums (143 / 145) and for FP64 handles
-// with an adjoint, whose abar runs on the same items (1.5M rows, residual and
-// backward 525 / 537; 6M 1894 / 1990).  The environment variable
+// Default (measured on B200, random columns; us per product, 256- against
+// 128-nonzero items, skewed).  The smaller items take fewer registers, so more
+// warps gather, which the chunks of long rows, all gathers, want; items of whole
+// rows pay for their descriptor and row sums twice as often.
+//   power-law rows (the share of nonzeros in rows above 256 decides: FP32, 1M to 3M
+//     rows, share 0.70 / 0.37 / 0.16 / 0.10  188 / 110 / 91 / 78 against 184 / 99 /
+//     75 / 65):
+//     FP32, 0.3M / 2M / 13.4M rows (in two column blocks)  52.2 / 188 / 617
+//           against 44.6 / 184 / 539;
+//     FP64, 0.3M rows 58.9 / 53.7, 8.4M columns (64 MB x) unsplit 454 / 428, in
+//           blocks 483 / 467;
+//   rows of 1..95, FP32, 1M rows 210 / 235; rows of 1..21, FP32, 0.8M rows, residual
+//     and backward 164 / 180.
+// 256 also stays for FP64 where x is in L2 and the matrix fills the GPU either
+// way (1.5M rows 167 / 166, 5M 490 / 505), for compensated sums (143 / 145) and
+// for FP64 handles with an adjoint, whose abar runs on the same items (1.5M rows,
+// residual and backward 525 / 537; 6M 1894 / 1990).  The environment variable
 // DRB_SPMV_VARIANT="tile,skew" (e.g. "512,0") overrides it for handles
 // created afterwards ("128,1,1": the two-slot kernel); drb_csr_autotune
 // measures them all instead.
@@ -45,12 +50,26 @@ int default_pipe_variant(const Csr &A) {
     if (t == 128 || t == 256 || t == 512)
       return t | (sk ? 1 : 0) | (two ? 2 : 0);
   }
+  if (A.long_nnz < A.nnz / 32 || (A.flags & DRB_FLAG_COMPENSATED))
+    return 256 | 1;
   if (A.storage == DRB_F32)
-    return (A.flags & DRB_FLAG_COMPENSATED) ? 256 | 1 : 128 | 1;
+    return 128 | 1;
   const bool fills = A.nnz >= 12000000, in_l2 = A.n * 8 <= (int64_t)48 << 20;
   if (A.storage == DRB_F64 && !(A.flags & DRB_FLAG_ADJOINT) && !(fills && in_l2))
     return 128 | 1;
   return 256 | 1;
+}
+
+int64_t long_row_nnz(int64_t m, const void *rowptr_host, int rbytes) {
+  int64_t total = 0;
+  for (int64_t r = 0; r < m; r++) {
+    const int64_t len = rbytes == 4 ? (int64_t)((const int32_t *)rowptr_host)[r + 1] -
+                                          ((const int32_t *)rowptr_host)[r]
+                                    : ((const int64_t *)rowptr_host)[r + 1] -
+                                          ((const int64_t *)rowptr_host)[r];
+    total += len > kLongRowNnz ? len : 0;
+  }
+  return total;
 }
 
 drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
