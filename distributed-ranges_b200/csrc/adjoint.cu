@@ -106,7 +106,7 @@ template <class V, class CI, class RI, int TILE>
 __global__ void __launch_bounds__(kAbWarps * 32)
     abar_items(const RI *__restrict__ rowptr, const CI *__restrict__ colind,
                const V *__restrict__ ybar, const V *__restrict__ x, V *__restrict__ abar,
-               const Item *__restrict__ items, int64_t nitems, unsigned *counter, bool vec) {
+               const Item *__restrict__ items, int64_t nitems, int *counters, bool vec) {
   using S = AbSlot<V, CI, TILE>;
   constexpr int G = S::G, NG = S::NG;
   constexpr int VPER = 16 / sizeof(V);
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kAbWarps * 32)
   auto grab = [&]() -> int64_t {
     unsigned v = 0;
     if (lane == 0)
-      v = atomicAdd(counter, (unsigned)kBatch);
+      v = atomicAdd(reinterpret_cast<unsigned *>(counters), (unsigned)kBatch);
     return (int64_t)__shfl_sync(kFull, v, 0);
   };
   auto advance = [&]() -> int64_t {
@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(kAbWarps * 32)
     fetch(A, advance());
     step(B, xv);
   }
+  warpk::reset_counter(counters);
 }
 
 unsigned grid1(int64_t n) {
@@ -502,10 +503,9 @@ drb_status abar_tile(Csr &A, const V *ybar, const V *x, V *abar, cudaStream_t s)
   const PipePlan &P = A.pipe;
   const int g = (int)std::min<int64_t>(grid, (P.nitems + kAbWarps - 1) / kAbWarps);
   const bool vec = reinterpret_cast<uintptr_t>(abar) % 16 == 0;
-  DRB_CUDA_TRY(cudaMemsetAsync(P.counters.p, 0, sizeof(unsigned), s)); // work counter
   abar_items<V, CI, RI, TILE><<<g, kAbWarps * 32, 0, s>>>(
       A.rowptr.as<RI>(), A.colind.as<CI>(), ybar, x, abar, P.items.as<Item>(), P.nitems,
-      P.counters.as<unsigned>(), vec);
+      P.counters.as<int>(), vec);
   note_launch();
   DRB_CUDA_TRY(cudaGetLastError());
   return DRB_OK;

@@ -176,6 +176,8 @@ __device__ __forceinline__ void combine4(const Acc *__restrict__ ys, int64_t m, 
 template <class Acc>
 __global__ void split_combine(const Acc *__restrict__ ys, Acc *__restrict__ y, int64_t m,
                               int64_t r0, int64_t r1, int nblk) {
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < r1;
        r += kCombineRows * stride) {
@@ -201,6 +203,8 @@ __global__ void __launch_bounds__(256)
                         int *ticket, double *out) {
   __shared__ double s_red[8];
   __shared__ int s_last;
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   double sum = 0.0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
@@ -474,13 +478,14 @@ drb_status combine_rows(Csr &A, void *y, int64_t r0, int64_t r1, cudaStream_t s)
     return DRB_OK;
   const unsigned g = flat_grid(r1 - r0);
   if (A.storage == DRB_F64)
-    split_combine<double><<<g, 256, 0, s>>>(A.csplit_y.as<double>(), static_cast<double *>(y),
-                                            A.m, r0, r1, A.csplit_nblk);
+    DRB_CUDA_TRY(launch_overlapped(split_combine<double>, dim3(g), dim3(256), 0, s,
+                                   A.csplit_y.as<double>(), static_cast<double *>(y), A.m, r0,
+                                   r1, A.csplit_nblk));
   else
-    split_combine<float><<<g, 256, 0, s>>>(A.csplit_y.as<float>(), static_cast<float *>(y),
-                                           A.m, r0, r1, A.csplit_nblk);
+    DRB_CUDA_TRY(launch_overlapped(split_combine<float>, dim3(g), dim3(256), 0, s,
+                                   A.csplit_y.as<float>(), static_cast<float *>(y), A.m, r0, r1,
+                                   A.csplit_nblk));
   note_launch();
-  DRB_CUDA_TRY(cudaGetLastError());
   return DRB_OK;
 }
 } // namespace
@@ -502,16 +507,16 @@ drb_status colsplit_residual(Csr &A, const void *x, const void *b, void *y, doub
   double *slots = A.pipe.red.as<double>();
   int *ticket = reinterpret_cast<int *>(slots + (size_t)sms * 32);
   if (A.storage == DRB_F64)
-    split_combine_resid<double><<<g, 256, 0, s>>>(A.csplit_y.as<double>(),
-                                                  static_cast<double *>(y),
-                                                  static_cast<const double *>(b), A.m,
-                                                  A.csplit_nblk, slots, ticket, out);
+    DRB_CUDA_TRY(launch_overlapped(split_combine_resid<double>, dim3(g), dim3(256), 0, s,
+                                   A.csplit_y.as<double>(), static_cast<double *>(y),
+                                   static_cast<const double *>(b), A.m, A.csplit_nblk, slots,
+                                   ticket, out));
   else
-    split_combine_resid<float><<<g, 256, 0, s>>>(A.csplit_y.as<float>(), static_cast<float *>(y),
-                                                 static_cast<const float *>(b), A.m,
-                                                 A.csplit_nblk, slots, ticket, out);
+    DRB_CUDA_TRY(launch_overlapped(split_combine_resid<float>, dim3(g), dim3(256), 0, s,
+                                   A.csplit_y.as<float>(), static_cast<float *>(y),
+                                   static_cast<const float *>(b), A.m, A.csplit_nblk, slots,
+                                   ticket, out));
   note_launch();
-  DRB_CUDA_TRY(cudaGetLastError());
   return DRB_OK;
 }
 

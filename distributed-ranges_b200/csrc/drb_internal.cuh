@@ -163,7 +163,8 @@ struct PipePlan {
   DevBuf splits;   // int4 {row, first chunk, chunks, 0} per split row, in chunk order
   std::vector<int64_t> split_first; // host copy of each split row's first chunk
   DevBuf partials; // value type [nchunks]
-  DevBuf counters; // unsigned work counter of the persistent kernel (zeroed per launch)
+  DevBuf counters; // int[4]: the persistent kernels' work counter and CTA arrivals,
+                   // zero between launches
   DevBuf err;      // int: device-side error word (DRB_ERR_TIMEOUT)
   DevBuf red;      // double[grid] + int ticket: fused residual
   // The same items ordered by row and cut into row segments (built on the

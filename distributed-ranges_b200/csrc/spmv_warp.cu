@@ -50,7 +50,7 @@ int default_pipe_variant(const Csr &A) {
     if (t == 128 || t == 256 || t == 512)
       return t | (sk ? 1 : 0) | (two ? 2 : 0);
   }
-  if (A.long_nnz < A.nnz / 32 || (A.flags & DRB_FLAG_COMPENSATED))
+  if (A.long_nnz * 32 < A.nnz || (A.flags & DRB_FLAG_COMPENSATED))
     return 256 | 1;
   if (A.storage == DRB_F32)
     return 128 | 1;
@@ -183,7 +183,7 @@ drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
   for (size_t i = 0; i < splits.size(); i++)
     plan.split_first[i] = splits[i].y;
   DRB_TRY(plan.partials.alloc(sizeof(double) * std::max<size_t>(chunks.size(), 1)));
-  DRB_TRY(plan.counters.alloc(sizeof(int) * std::max<int64_t>(nsplit, 1)));
+  DRB_TRY(plan.counters.alloc(sizeof(int) * 4));
   DRB_CUDA_TRY(cudaMemset(plan.counters.p, 0, plan.counters.bytes));
   DRB_TRY(plan.err.alloc(sizeof(int) * 4));
   DRB_CUDA_TRY(cudaMemset(plan.err.p, 0, plan.err.bytes));

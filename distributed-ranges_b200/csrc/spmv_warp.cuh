@@ -457,6 +457,20 @@ template <class V, class XT, class CI, class RI, int TILE, bool SKEW, bool COMP>
   }
 };
 
+// The last CTA to get here leaves the work counter counters[0] (and its own
+// arrivals, counters[1]) at zero for the next launch: every warp has taken its
+// last batch by then.  (A memset before each launch was a launch of its own
+// with its gap, and kept the product from starting under its predecessor's
+// tail: power-law rows, f32, 50k rows 27.7 -> 23.1 us with the rest of the
+// launches overlapped too, 0.3M 42.7 -> 39.8, 2M 180.5 -> 178.4.)
+__device__ __forceinline__ void reset_counter(int *counters) {
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(counters + 1, 1) == (int)gridDim.x - 1) {
+    counters[0] = 0;
+    counters[1] = 0;
+  }
+}
+
 template <class V, class XT, class CI, class RI, int TILE, bool SKEW, bool RESID, bool COMP>
 __global__ void __launch_bounds__(kThreads)
     spmv_warp(const RI *__restrict__ rowptr, const CI *__restrict__ colind,
@@ -469,6 +483,8 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ __align__(16) Acc s_prod[kWarps][TILE + TILE / 32];
   __shared__ int s_rp[kWarps][kRows + 1];
 
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   if (RESID && ra.stop && *static_cast<const volatile int *>(ra.stop))
     return; // uniform: every CTA reads the same word, written by an earlier launch
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -486,7 +502,7 @@ __global__ void __launch_bounds__(kThreads)
   int *srp = s_rp[warp];
 
   // Warps take items in batches of kBatch consecutive indices from a work
-  // counter (zeroed before the launch; lane 0 takes the next index one item
+  // counter (zero between launches; lane 0 takes the next index one item
   // ahead, so the atomic's round trip overlaps the current item): a fixed
   // round-robin share was sensitive to the exact sequence of item costs (the
   // bench's power-law ran 2.23 ms against 1.61 ms for the same distribution
@@ -524,6 +540,7 @@ __global__ void __launch_bounds__(kThreads)
     cur = next;
     next = advance();
   }
+  reset_counter(counters);
 }
 
 // The plain product (no fused reduction) with two item slots per warp: the
@@ -543,6 +560,8 @@ __global__ void __launch_bounds__(kThreads, TILE == 128 ? 4 : 2)
   using Kt = Kern<V, XT, CI, RI, TILE, SKEW, COMP>;
   __shared__ __align__(16) Acc s_prod[kWarps][TILE + TILE / 32];
   __shared__ int s_rp[kWarps][kRows + 1];
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Kt K{rowptr, colind, vals, x, y, items, nitems, chunks, partials, counters,
        ptx::policy_evict_first(), ptx::policy_evict_last(),
@@ -578,6 +597,7 @@ __global__ void __launch_bounds__(kThreads, TILE == 128 ? 4 : 2)
       break;
     K.step(B, A, xg, advance(), prod, srp);
   }
+  reset_counter(counters);
 }
 
 // A split row's sum: its chunk partials pp[0, count) added in chunk order.
@@ -617,6 +637,8 @@ __device__ __forceinline__ Acc chunk_row_sum(const Acc *__restrict__ pp, int cou
 template <class Acc, bool COMP>
 __global__ void chunk_finish(const int4 *__restrict__ splits, int64_t s0, int64_t s1,
                              const Acc *__restrict__ partials, Acc *__restrict__ y) {
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   const int64_t nth = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = s0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < s1; i += nth) {
     const int4 sp = splits[i];
@@ -637,6 +659,8 @@ __global__ void __launch_bounds__(kThreads)
                  int64_t nitems) {
   __shared__ double s_red[kWarps];
   __shared__ int s_last;
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   if (ra.stop && *static_cast<const volatile int *>(ra.stop))
     return;
   const Acc *bvec = static_cast<const Acc *>(ra.b);
@@ -743,25 +767,23 @@ drb_status launch_tile(Csr &A, const void *x, void *y, const WarpResid *ra,
   WarpResid r{};
   if (ra)
     r = *ra;
-  DRB_CUDA_TRY(cudaMemsetAsync(P.counters.p, 0, sizeof(unsigned), s)); // work counter
-  kern<<<grid, kThreads, 0, s>>>(A.rowptr.as<RI>(), A.colind.as<CI>(), A.vals.as<V>(),
+  DRB_CUDA_TRY(launch_overlapped(kern, dim3(grid), dim3(kThreads), 0, s, A.rowptr.as<RI>(),
+                                 A.colind.as<CI>(), A.vals.as<V>(),
                                  static_cast<const XT *>(x), static_cast<Acc *>(y),
                                  P.items.as<Item>(), P.nitems, P.chunks.as<Chunk>(),
                                  P.partials.as<Acc>(), P.counters.as<int>(), r,
-                                 y_store_keep());
+                                 y_store_keep()));
   note_launch();
-  DRB_CUDA_TRY(cudaGetLastError());
   if (RESID) {
     // a function of the plan only, so the reduction's grouping is fixed
     const int g = (int)std::max<int64_t>(
         1, std::min<int64_t>(kResidFinishGrid,
                              std::max((P.nchunks + kThreads - 1) / kThreads,
                                       (P.nitems + 8191) / 8192)));
-    resid_finish<Acc, COMP><<<g, kThreads, 0, s>>>(P.splits.as<int4>(), P.nsplit,
-                                                   P.partials.as<Acc>(),
-                                                   static_cast<Acc *>(y), r, P.nitems);
+    DRB_CUDA_TRY(launch_overlapped(resid_finish<Acc, COMP>, dim3(g), dim3(kThreads), 0, s,
+                                   P.splits.as<int4>(), P.nsplit, P.partials.as<Acc>(),
+                                   static_cast<Acc *>(y), r, P.nitems));
     note_launch();
-    DRB_CUDA_TRY(cudaGetLastError());
   } else if (P.nsplit > 0) {
     // the split rows whose first chunk lies in [fin_c0, fin_c1) (all with -1)
     const auto &f = P.split_first;
@@ -773,10 +795,10 @@ drb_status launch_tile(Csr &A, const void *x, void *y, const WarpResid *ra,
       // one split row per thread: each is a short chain of dependent loads,
       // and a thread walking several in turn made the pass latency-bound
       const int g = (int)std::max<int64_t>(1, std::min<int64_t>(1 << 20, (s1 - s0 + 255) / 256));
-      chunk_finish<Acc, COMP><<<g, 256, 0, s>>>(P.splits.as<int4>(), s0, s1,
-                                                P.partials.as<Acc>(), static_cast<Acc *>(y));
+      DRB_CUDA_TRY(launch_overlapped(chunk_finish<Acc, COMP>, dim3(g), dim3(256), 0, s,
+                                     P.splits.as<int4>(), s0, s1, P.partials.as<Acc>(),
+                                     static_cast<Acc *>(y)));
       note_launch();
-      DRB_CUDA_TRY(cudaGetLastError());
     }
   }
   return DRB_OK;
