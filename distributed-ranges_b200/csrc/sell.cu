@@ -94,6 +94,8 @@ __global__ void __launch_bounds__(kSellNT)
   using Acc = typename AccOf<V>::type;
   __shared__ double s_red[kSellWarps];
   __shared__ int s_last;
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   if (RESID && ra.stop && *static_cast<const volatile int *>(ra.stop))
     return; // uniform: every CTA reads the same word, written by an earlier launch
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -204,18 +206,22 @@ __global__ void __launch_bounds__(kSellNT)
   }
 }
 
-template <class V, bool RESID, int NS, int K> int sell_grid(int dev) {
-  static int cache[64] = {0};
-  int &g = cache[dev < 64 ? dev : 0];
+// The grid for `need` CTAs of work: all resident, the same number on every SM (the
+// slices are shared evenly whatever the grid).  With the launch overlapped, 131072
+// rows of 16, f32, 12.3 -> 10.3 us; 256 CTAs on 148 SMs had left most of them
+// with one.
+template <class V, bool RESID, int NS, int K> int sell_grid(int dev, int64_t need) {
+  static int cache[64][2];
+  int &g = cache[dev < 64 ? dev : 0][0], &sms = cache[dev < 64 ? dev : 0][1];
   if (g == 0) {
-    int occ = 0, sms = 0;
+    int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sell_spmv<V, RESID, NS, K>, kSellNT, 0) !=
             cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return 148;
     g = std::max(1, occ) * sms;
   }
-  return g;
+  return (int)std::min<int64_t>(g, need <= 8 ? need : (need + sms - 1) / sms * sms);
 }
 
 template <class V, int NS, int K>
@@ -227,20 +233,17 @@ drb_status sell_run(Csr &A, const void *x, void *y, const WarpResid *ra, int64_t
   WarpResid r{};
   if (ra) {
     r = *ra;
-    const int g = (int)std::min<int64_t>(sell_grid<V, true, NS, K>(A.device), need);
-    sell_spmv<V, true, NS, K><<<g, kSellNT, 0, s>>>(S.vals.as<V>(), S.cols.as<int>(),
-                                                   S.off.as<int64_t>(), s0, s1, A.m,
-                                                   static_cast<const V *>(x),
-                                                   static_cast<Acc *>(y), r);
+    const int g = sell_grid<V, true, NS, K>(A.device, need);
+    DRB_CUDA_TRY(launch_overlapped(sell_spmv<V, true, NS, K>, dim3(g), dim3(kSellNT), 0, s,
+                                   S.vals.as<V>(), S.cols.as<int>(), S.off.as<int64_t>(), s0, s1,
+                                   A.m, static_cast<const V *>(x), static_cast<Acc *>(y), r));
   } else {
-    const int g = (int)std::min<int64_t>(sell_grid<V, false, NS, K>(A.device), need);
-    sell_spmv<V, false, NS, K><<<g, kSellNT, 0, s>>>(S.vals.as<V>(), S.cols.as<int>(),
-                                                    S.off.as<int64_t>(), s0, s1, A.m,
-                                                    static_cast<const V *>(x),
-                                                    static_cast<Acc *>(y), r);
+    const int g = sell_grid<V, false, NS, K>(A.device, need);
+    DRB_CUDA_TRY(launch_overlapped(sell_spmv<V, false, NS, K>, dim3(g), dim3(kSellNT), 0, s,
+                                   S.vals.as<V>(), S.cols.as<int>(), S.off.as<int64_t>(), s0, s1,
+                                   A.m, static_cast<const V *>(x), static_cast<Acc *>(y), r));
   }
   note_launch();
-  DRB_CUDA_TRY(cudaGetLastError());
   return DRB_OK;
 }
 
