@@ -9,11 +9,12 @@
 // ceil(k / 8) passes over HBM, and rows that do not start on 16 bytes went
 // through single-element loads with few of them in flight.
 //
-// Measured (us): 5003 x 3001 f64 with 20 right-hand sides 246 -> 57, f32 428 -> 47;
-// 8192^2 f32 with 20 336 -> 116, with 8 143 -> 78, with 4 61 -> 62; 4096 x 8192
-// f64 with 32 428 -> 103.
+// Measured (us): 5003 x 3001 f64 with 20 right-hand sides 246 -> 53, f32 428 -> 44;
+// 8192^2 f32 with 20 336 -> 112, with 8 143 -> 73, with 4 61 -> 57; 4096 x 8192
+// f64 with 32 428 -> 101.  (One CTA of 16 warps per SM with tiles twice as high
+// ran the f64 case in 57: all warps loaded, waited and multiplied in step.)
 //
-// Tiles and split.  A CTA of 16 warps owns a tile of BM rows and walks along the
+// Tiles and split.  A CTA of 8 warps owns a tile of BM rows and walks along the
 // columns in chunks of KC; the chunks of A and of X come through a
 // STAGES-deep cp.async ring in 16-byte pieces.  Where rows of A or columns of X
 // do not start on 16 bytes (odd sizes), a row is copied from the boundary below
@@ -32,8 +33,7 @@
 //        scalar rate.
 //   f64: mma.sync m8n8k4: a warp has 16 rows x 8 NT right-hand sides and one
 //        half of each chunk's columns (the halves meet in shared memory at the
-//        end of a tile): 16 warps keep the tensor pipe fed where 8 left it idle
-//        half the time.  CUDA cores would need 2 (R + C) shared-memory cycles
+//        end of a tile).  CUDA cores would need 2 (R + C) shared-memory cycles
 //        for R C fused multiply-adds at half rate, and 4 R C registers.
 #include <algorithm>
 
@@ -42,9 +42,11 @@
 namespace drb {
 namespace {
 
-constexpr int kNT = 512;
+constexpr int kNT = 256;
+constexpr int kCtas = 2; // per SM: one computes while the other waits for its loads
 constexpr int kWarps = kNT / 32;
 constexpr int kPanelCols = 32; // right-hand sides of one pass
+constexpr int64_t kLongShare = 6; // see Shape
 constexpr int64_t kTurnElems = (int64_t)1 << 21; // A above this: row-major X is transposed first
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -92,20 +94,30 @@ struct PanelArgs {
 // right-hand sides of the two half-warps are 64 bytes apart modulo 128, f64 rows
 // 64 bytes for the 16-byte fragment loads of aligned rows and 32 bytes for the
 // 8-byte loads of shifted ones.
-template <class V, int P, bool SH> struct Shape;
-template <int C, bool SH> struct Shape<float, C, SH> { // C right-hand sides
+// LONG chunks are twice as wide in a ring of two: half the waits and longer runs
+// of a row per copy, for shares of many chunks (a short share is over before
+// they pay, and its last chunk is mostly padding; f64 with more than 16
+// right-hand sides does not gain: its tensor pipe is as busy as the loads).
+// Measured, us, short / long: 8192^2 f32 k = 20 105 / 94, 8191^2 k = 3 83 / 69,
+// 8191 x 4095 f64 k = 5 80 / 70; 16000 x 300 f32 k = 12 9.9 / 11.1, 5003 x 3001
+// f64 k = 20 49.7 / 51.3.
+template <class V, int P, bool SH, bool LONG> struct Shape;
+template <int C, bool SH, bool LONG>
+struct Shape<float, C, SH, LONG> { // C right-hand sides
   static constexpr int R = C <= 20 ? 8 : 4;
-  static constexpr int BM = kWarps * R, KC = 64, AS = KC + 4, XS = KC + 16, CP = C;
-  static constexpr int STAGES = 4, MERGE = 0;
+  static constexpr int BM = kWarps * R, KC = LONG ? 128 : 64, AS = KC + 4, XS = KC + 16, CP = C;
+  static constexpr int STAGES = LONG ? 2 : 4, MERGE = 0;
 };
-template <int NT, bool SH> struct Shape<double, NT, SH> { // 8 NT right-hand sides
+template <int NT, bool SH, bool LONG>
+struct Shape<double, NT, SH, LONG> { // 8 NT right-hand sides
   static constexpr int R = 16;
-  static constexpr int BM = kWarps / 2 * R, KC = 32, AS = KC + (SH ? 4 : 8), XS = AS, CP = 8 * NT;
-  static constexpr int STAGES = NT == 4 && !SH ? 3 : 4;
+  static constexpr int BM = kWarps / 2 * R, KC = LONG ? 64 : 32, AS = KC + (SH ? 4 : 8), XS = AS;
+  static constexpr int CP = 8 * NT, STAGES = LONG ? 2 : 3;
   static constexpr int MERGE = BM * CP; // the second half's sums of a tile
 };
-template <class V, int P, bool SH> constexpr size_t panel_smem() {
-  using S = Shape<V, P, SH>;
+template <class V, int P> constexpr bool may_be_long() { return sizeof(V) == 4 || P <= 2; }
+template <class V, int P, bool SH, bool LONG> constexpr size_t panel_smem() {
+  using S = Shape<V, P, SH, LONG>;
   return ((size_t)S::STAGES * (S::BM * S::AS + S::CP * S::XS) + S::MERGE) * sizeof(V);
 }
 
@@ -137,12 +149,14 @@ __device__ __forceinline__ void copy_edge_piece(uint32_t dst, const V *row, int6
   }
 }
 
-template <class V, int P, bool SH>
-__global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
-  using S = Shape<V, P, SH>;
+template <class V, int P, bool SH, bool LONG>
+__global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
+  using S = Shape<V, P, SH, LONG>;
   constexpr int BM = S::BM, KC = S::KC, AS = S::AS, XS = S::XS, CP = S::CP, ST = S::STAGES;
   constexpr int PER = 16 / (int)sizeof(V), GR = KC / PER, RP = kNT / GR;
   extern __shared__ __align__(16) unsigned char panel_mem[];
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   V *sa = reinterpret_cast<V *>(panel_mem);
   V *sx = sa + (size_t)ST * BM * AS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -157,7 +171,13 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
   // fixed and its rows step by a constant, so a whole chunk costs one address
   // addition per piece.
   const int ar = tid / GR, ag = (tid % GR) * PER; // first row, piece column
-  int64_t lt = c0 / cpt;                           // tile and chunk of the next load
+  // A shifted row's offset depends on its index modulo a piece, which tiles,
+  // warps' rows and a thread's row steps are multiples of: fixed per thread.
+  const int sha = SH ? shift_of(A + ar * a.lda) : 0;
+  const int sha_end = SH ? shift_of(A + tid * a.lda) : 0;
+  const int shx = SH && a.x_cs == 1 ? shift_of(X + ar * a.x_js) : 0;
+  const int shx_end = SH && a.x_cs == 1 ? shift_of(X + tid * a.x_js) : 0;
+  int64_t lt = c0 / cpt; // tile and chunk of the next load
   int lc = (int)(c0 - lt * cpt);
   auto load = [&](int st) {
     const int64_t kb = (int64_t)lc * KC, r0 = lt * BM;
@@ -175,48 +195,44 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
     const V *row = A + (r0 + ar) * a.lda;
     const int64_t step = RP * a.lda;
     if (inside) {
-      const V *src = row + kb + ag;
+      const V *src = row + kb + ag - sha;
 #pragma unroll
       for (int p = 0; p < BM / RP; p++, src += step)
-        cp_zfill<16>(da + (uint32_t)(p * RP * AS * sizeof(V)), SH ? src - shift_of(src) : src);
+        cp_zfill<16>(da + (uint32_t)(p * RP * AS * sizeof(V)), src);
     } else {
 #pragma unroll 1
       for (int p = 0; p < BM / RP; p++, row += step)
         if (r0 + ar + p * RP < a.m)
           copy_edge_piece<V>(da + (uint32_t)(p * RP * AS * sizeof(V)), row,
-                             kb + ag - (SH ? shift_of(row) : 0), kb, a.n, A, Aend);
+                             kb + ag - sha, kb, a.n, A, Aend);
     }
-    if (SH && tid < BM && r0 + tid < a.m) { // the piece past the chunk
+    if (SH && tid < BM && sha_end > 0 && r0 + tid < a.m) { // the piece past the chunk
       const V *rw = A + (r0 + tid) * a.lda;
-      const int sh = shift_of(rw);
-      if (sh > 0) {
-        const uint32_t d = s0 + (uint32_t)((tid * AS + KC) * sizeof(V));
-        if (inside)
-          cp_zfill<16>(d, rw + kb + KC - sh);
-        else
-          copy_edge_piece<V>(d, rw, kb + KC - sh, kb, a.n, A, Aend);
-      }
+      const uint32_t d = s0 + (uint32_t)((tid * AS + KC) * sizeof(V));
+      if (inside)
+        cp_zfill<16>(d, rw + kb + KC - sha_end);
+      else
+        copy_edge_piece<V>(d, rw, kb + KC - sha_end, kb, a.n, A, Aend);
     }
     const uint32_t dx = smem_u32(sx + (size_t)st * CP * XS);
     if (a.x_cs == 1) {
       const bool xin = SH ? kb > 0 && kb + KC + PER <= a.n : kb + KC <= a.n;
       for (int j = ar; j < a.k; j += RP) {
         const V *xc = X + j * a.x_js;
-        const int64_t e0 = kb + ag - (SH ? shift_of(xc) : 0);
+        const int64_t e0 = kb + ag - shx;
         const uint32_t d = dx + (uint32_t)((j * XS + ag) * sizeof(V));
         if (xin)
           cp_zfill<16>(d, xc + e0);
         else
           copy_edge_piece<V>(d, xc, e0, kb, a.n, X, Xend);
       }
-      if (SH && tid < a.k) {
+      if (SH && tid < a.k && shx_end > 0) {
         const V *xc = X + tid * a.x_js;
-        const int sh = shift_of(xc);
         const uint32_t d = dx + (uint32_t)((tid * XS + KC) * sizeof(V));
-        if (sh > 0 && xin)
-          cp_zfill<16>(d, xc + kb + KC - sh);
-        else if (sh > 0)
-          copy_edge_piece<V>(d, xc, kb + KC - sh, kb, a.n, X, Xend);
+        if (xin)
+          cp_zfill<16>(d, xc + kb + KC - shx_end);
+        else
+          copy_edge_piece<V>(d, xc, kb + KC - shx_end, kb, a.n, X, Xend);
       }
     } else { // row-major X: 32-byte runs of right-hand sides, few bank conflicts
       constexpr int JL = 32 / (int)sizeof(V), CL = 32 / JL; // lanes over j, over c
@@ -229,12 +245,20 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
                               c < kn ? (int)sizeof(V) : 0);
     }
   };
-  // offset of column j of a staged X chunk (columns PER apart share it)
-  auto xshift = [&](int j) { return SH && a.x_cs == 1 ? shift_of(X + j * a.x_js) : 0; };
-
   // first row of this warp; f64: its half of a chunk's columns
   const int wr = (sizeof(V) == 4 ? warp : warp % (kWarps / 2)) * S::R;
   const int kh = sizeof(V) == 4 ? 0 : warp / (kWarps / 2) * (KC / 2);
+  // offsets of this lane's rows and columns in a staged chunk
+  auto ashift = [&](int r) { return SH ? shift_of(A + r * a.lda) : 0; };
+  auto xshift = [&](int j) { return SH && a.x_cs == 1 ? shift_of(X + j * a.x_js) : 0; };
+  static_assert(BM % PER == 0 && RP % PER == 0 && S::R % PER == 0, "offsets repeat");
+  int ra[PER], xj[2];
+#pragma unroll
+  for (int q = 0; q < PER; q++)
+    ra[q] = sizeof(V) == 4 ? ashift(q) : ashift(lane >> 2);
+#pragma unroll
+  for (int q = 0; q < 2; q++) // (f32: columns cg, cg + 2, ...: four apart share an offset)
+    xj[q] = sizeof(V) == 4 ? (lane >> 4) * XS + xshift((lane >> 4) + 2 * q) : xshift(lane >> 2);
   // this thread's sums of the current tile
   constexpr int R = S::R;
   constexpr int NACC = sizeof(V) == 4 ? R * CP / 2 : 2 * (CP / 8);
@@ -251,25 +275,17 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
         accd[i][0] = accd[i][1] = 0.0;
     }
   };
-  auto compute = [&](int st, int64_t tile) {
+  auto compute = [&](int st) {
     const V *As = sa + (size_t)st * BM * AS + wr * AS;
     const V *Xs = sx + (size_t)st * CP * XS;
     if constexpr (sizeof(V) == 4) {
       constexpr int CH = CP / 2;
-      const int cg = lane >> 4; // the lane has right-hand sides cg, cg + 2, ...
-      int ra[R], xj[2];         // where its rows and columns start
-#pragma unroll
-      for (int r = 0; r < R; r++)
-        ra[r] = r * AS + (SH ? shift_of(A + (tile * BM + wr + r) * a.lda) : 0);
-#pragma unroll
-      for (int q = 0; q < 2; q++)
-        xj[q] = cg * XS + xshift(cg + 2 * q); // (columns four apart share an offset)
 #pragma unroll 2
       for (int c = lane & 15; c < KC; c += 16) {
         float av[R];
 #pragma unroll
         for (int r = 0; r < R; r++)
-          av[r] = As[ra[r] + c];
+          av[r] = As[r * AS + ra[r % PER] + c];
 #pragma unroll
         for (int j = 0; j < CH; j++) {
           const float xv = Xs[2 * j * XS + xj[j % 2] + c];
@@ -284,11 +300,10 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
       // k order inside a step of eight: a lane's pair (aligned rows) or the
       // lane's column of either half (shifted rows); the same for A and X
       const int fk = SH ? (lane & 3) : 2 * (lane & 3);
-      const V *Ap[2], *Xp = Xs + fr * XS + fk + xshift(fr) + kh; // 8 columns on: the same offset
+      const V *Ap[2], *Xp = Xs + fr * XS + fk + xj[0] + kh; // 8 columns on: the same offset
 #pragma unroll
       for (int i = 0; i < 2; i++)
-        Ap[i] = As + (i * 8 + fr) * AS + fk + kh +
-                (SH ? shift_of(A + (tile * BM + wr + i * 8 + fr) * a.lda) : 0);
+        Ap[i] = As + (i * 8 + fr) * AS + fk + kh + ra[0];
 #pragma unroll
       for (int c = 0; c < KC / 2; c += 8) {
         double2 av[2], bv[NT];
@@ -384,6 +399,8 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
     }
   };
 
+  int64_t ct = c0 / cpt;                      // current tile
+  int left = cpt - (int)(c0 - ct * cpt);      // chunks left in it
 #pragma unroll
   for (int s = 0; s < ST - 1; s++) {
     if (c0 + s < c1)
@@ -392,8 +409,6 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
   }
   clear();
   int st = 0;
-  int64_t ct = c0 / cpt;                      // current tile
-  int left = cpt - (int)(c0 - ct * cpt);      // chunks left in it
   for (int64_t q = c0; q < c1; q++) {
     cp_wait<ST - 2>();
     __syncthreads(); // chunk q landed; slot st - 1 is free
@@ -401,7 +416,7 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
     if (q + ST - 1 < c1)
       load(fill);
     cp_commit();
-    compute(st, ct);
+    compute(st);
     if (--left == 0 || q + 1 == c1) {
       emit(ct);
       clear();
@@ -413,55 +428,86 @@ __global__ void __launch_bounds__(kNT, 1) dense_panel(const PanelArgs a) {
   cp_wait<0>();
 }
 
-// Y of the tiles cut between CTAs: their partials added in chunk order.
-template <class V>
-__global__ void panel_sum(const PanelArgs a, int BM, int CP) {
+// Y of the tiles cut between CTAs: their partials added in a fixed order.  A
+// group of PW threads (in different warps, so that a warp reads consecutive
+// partials) takes every PW-th piece of an output and thread 0 of the group adds
+// the groups' sums: one piece after another, a 300 x 16000 matrix's tiles, cut
+// into 59 pieces, kept the pass busy longer than the product.
+template <class V, int PW>
+__global__ void __launch_bounds__(256) panel_sum(const PanelArgs a, int BM, int CP) {
+  __shared__ V s_sum[256];
+  ptx::grid_dependency_wait();
+  constexpr int OUT = 256 / PW; // outputs per CTA
   const V *part = static_cast<const V *>(a.part);
   V *Y = static_cast<V *>(a.y);
-  const int64_t nth = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.m * a.k; i += nth) {
-    int64_t r;
-    int j;
-    if (a.y_ld == 1) { // consecutive threads write consecutive addresses
+  const int w = threadIdx.x / OUT, o = threadIdx.x % OUT;
+  for (int64_t i0 = (int64_t)blockIdx.x * OUT; i0 < a.m * a.k; i0 += (int64_t)gridDim.x * OUT) {
+    const int64_t i = i0 + o;
+    const bool in = i < a.m * a.k;
+    int64_t r = 0;
+    int j = 0;
+    if (in && a.y_ld == 1) { // consecutive threads write consecutive addresses
       j = (int)(i / a.m);
       r = i - (int64_t)j * a.m;
-    } else {
+    } else if (in) {
       r = i / a.k;
       j = (int)(i - r * a.k);
     }
     const int64_t tile = r / BM;
     const int64_t b0 = tile * a.cpt / a.share, b1 = ((tile + 1) * a.cpt - 1) / a.share;
-    if (b0 == b1)
-      continue; // one CTA had the whole tile
+    const bool cut = in && b0 != b1; // else one CTA had the whole tile
     V s = 0;
-    for (int64_t b = b0; b <= b1; b++) {
-      const int slot = tile == b * a.share / a.cpt ? 0 : 1;
-      s += part[((b * 2 + slot) * BM + (r - tile * BM)) * CP + j];
+    if (cut) {
+      // every piece but the first opens its CTA's share (slot 0)
+      const V *p = part + (r - tile * BM) * CP + j;
+      const int64_t step = 2 * (int64_t)BM * CP;
+      const int slot0 = tile == b0 * a.share / a.cpt ? 0 : 1;
+      int64_t b = b0 + w;
+      if (w == 0) {
+        s = p[b * step + slot0 * (int64_t)BM * CP];
+        b += PW;
+      }
+#pragma unroll 4
+      for (; b <= b1; b += PW)
+        s += p[b * step];
     }
-    Y[r * a.y_ld + j * a.y_js] = s;
+    if constexpr (PW > 1) {
+      __syncthreads(); // (the previous outputs' sums have been read)
+      s_sum[threadIdx.x] = s;
+      __syncthreads();
+      if (w > 0)
+        continue;
+#pragma unroll
+      for (int q = 1; q < PW; q++)
+        s += s_sum[q * OUT + o];
+    }
+    if (cut && w == 0)
+      Y[r * a.y_ld + j * a.y_js] = s;
   }
 }
 
-template <class V, int P, bool SH> drb_status panel_run(PanelArgs a, cudaStream_t s) {
-  using S = Shape<V, P, SH>;
-  constexpr size_t smem = panel_smem<V, P, SH>();
+template <class V, int P, bool SH, bool LONG>
+drb_status panel_run(PanelArgs a, cudaStream_t s) {
+  using S = Shape<V, P, SH, LONG>;
+  constexpr size_t smem = panel_smem<V, P, SH, LONG>();
   static int sm_count[64] = {0}; // 0: this device has not run the kernel yet
   int dev = 0;
   DRB_CUDA_TRY(cudaGetDevice(&dev));
   int &sms = sm_count[dev < 64 ? dev : 0];
   if (sms == 0 || dev >= 64) {
-    DRB_CUDA_TRY(cudaFuncSetAttribute(dense_panel<V, P, SH>,
+    DRB_CUDA_TRY(cudaFuncSetAttribute(dense_panel<V, P, SH, LONG>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     DRB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   }
   const int64_t tiles = (a.m + S::BM - 1) / S::BM;
   a.cpt = (a.n + S::KC - 1) / S::KC;
   a.chunks = tiles * a.cpt;
-  // Equal shares over the SMs (one CTA each), of at least kMinShare chunks: a
+  // Equal shares over the resident CTAs, of at least kMinShare chunks: a
   // shorter share is over before the ring is full, and a tile cut into more
   // pieces only adds partials.
   constexpr int64_t kMinShare = 4;
-  a.share = std::max((a.chunks + sms - 1) / sms, std::min(kMinShare, a.cpt));
+  const int64_t ctas = (int64_t)kCtas * sms;
+  a.share = std::max((a.chunks + ctas - 1) / ctas, std::min(kMinShare, a.cpt));
   // Shares of many tiles end on a tile: the rounding costs under 1/16, the
   // partials and their pass are saved.
   if (a.share >= 16 * a.cpt)
@@ -471,15 +517,17 @@ template <class V, int P, bool SH> drb_status panel_run(PanelArgs a, cudaStream_
   a.part = nullptr;
   if (cut)
     DRB_TRY(scratch_alloc(&a.part, sizeof(V) * 2 * (size_t)grid * S::BM * S::CP, s));
-  dense_panel<V, P, SH><<<(unsigned)grid, kNT, smem, s>>>(a);
+  cudaError_t e =
+      launch_overlapped(dense_panel<V, P, SH, LONG>, dim3((unsigned)grid), dim3(kNT), smem, s, a);
   note_launch();
-  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && cut) {
+    const bool many = a.cpt > 4 * a.share; // pieces of a tile
+    const int out = many ? 32 : 256;
     const unsigned g = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(148 * 8, (a.m * a.k + 255) / 256));
-    panel_sum<V><<<g, 256, 0, s>>>(a, S::BM, S::CP);
+        1, std::min<int64_t>(148 * 8, (a.m * a.k + out - 1) / out));
+    e = many ? launch_overlapped(panel_sum<V, 8>, dim3(g), dim3(256), 0, s, a, S::BM, S::CP)
+             : launch_overlapped(panel_sum<V, 1>, dim3(g), dim3(256), 0, s, a, S::BM, S::CP);
     note_launch();
-    e = cudaGetLastError();
   }
   if (a.part)
     scratch_free(a.part, s);
@@ -495,7 +543,14 @@ template <class V, int P> drb_status panel_align(const PanelArgs &a, cudaStream_
                        a.lda * sizeof(V) % 16 == 0 &&
                        (a.x_cs != 1 || (reinterpret_cast<uintptr_t>(a.x) % 16 == 0 &&
                                         a.x_js * sizeof(V) % 16 == 0));
-  return aligned ? panel_run<V, P, false>(a, s) : panel_run<V, P, true>(a, s);
+  if constexpr (may_be_long<V, P>()) {
+    // at least kLongShare long chunks for every CTA of the GPU
+    using S = Shape<V, P, false, true>;
+    const int64_t chunks = (a.m + S::BM - 1) / S::BM * ((a.n + S::KC - 1) / S::KC);
+    if (a.n >= 8 * S::KC && chunks >= kLongShare * kCtas * 148)
+      return aligned ? panel_run<V, P, false, true>(a, s) : panel_run<V, P, true, true>(a, s);
+  }
+  return aligned ? panel_run<V, P, false, false>(a, s) : panel_run<V, P, true, false>(a, s);
 }
 
 drb_status panel_cols(const PanelArgs &a, float, cudaStream_t s) {
