@@ -82,6 +82,8 @@ __global__ void __launch_bounds__(kDenseNT)
   constexpr int U = row_unroll<V, VEC>();
   constexpr int NW = kDenseNT / 32;
   __shared__ V s_frag[2 * NW];
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   const uint64_t pol_s = ptx::policy_evict_first();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t r0 = LOCAL ? m * blockIdx.x / gridDim.x : 0;
@@ -155,6 +157,8 @@ __global__ void __launch_bounds__(kDenseNT)
 
 template <class V>
 __global__ void dense_row_join(int64_t steps, int64_t spr, int64_t W, const V *frag, V *y) {
+  ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (w < W)
     join_cut_row<V>(0, steps, spr, w, W, frag, y);
@@ -186,21 +190,21 @@ drb_status dense_row_call(int64_t m, int64_t n, const V *A, int64_t lda, const V
   cudaError_t e;
   if (local) {
     const unsigned g = (unsigned)std::min<int64_t>(full, m);
-    dense_row_kernel<V, VEC, true><<<g, kDenseNT, 0, s>>>(m, n, A, lda, x, y, spr, nullptr);
+    e = launch_overlapped(dense_row_kernel<V, VEC, true>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
+                          lda, x, y, spr, (V *)nullptr);
     note_launch();
-    e = cudaGetLastError();
   } else {
     const unsigned g = (unsigned)std::min<int64_t>(full, (steps + NW - 1) / NW);
     const int64_t W = (int64_t)g * NW;
     V *frag = nullptr;
     DRB_TRY(scratch_alloc(reinterpret_cast<void **>(&frag), sizeof(V) * 2 * (size_t)W, s));
-    dense_row_kernel<V, VEC, false><<<g, kDenseNT, 0, s>>>(m, n, A, lda, x, y, spr, frag);
+    e = launch_overlapped(dense_row_kernel<V, VEC, false>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
+                          lda, x, y, spr, frag);
     note_launch();
-    e = cudaGetLastError();
     if (e == cudaSuccess) {
-      dense_row_join<V><<<(unsigned)((W + 255) / 256), 256, 0, s>>>(steps, spr, W, frag, y);
+      e = launch_overlapped(dense_row_join<V>, dim3((unsigned)((W + 255) / 256)), dim3(256), 0, s,
+                            steps, spr, W, (const V *)frag, y);
       note_launch();
-      e = cudaGetLastError();
     }
     scratch_free(frag, s);
   }
@@ -260,8 +264,10 @@ __global__ void __launch_bounds__(kDotNT)
     dot_kernel(int64_t n, const V *__restrict__ a, const V *__restrict__ b,
                double *partials, int *ticket, double *out) {
   constexpr int PER = 16 / sizeof(V);
-  if (!TICKET)
+  if (!TICKET) {
     ptx::grid_dependents_start();
+    ptx::grid_dependency_wait();
+  }
   const uint64_t pol_s = ptx::policy_evict_first();
   double acc = 0.0;
   const int64_t tid = (int64_t)blockIdx.x * kDotNT + threadIdx.x;
@@ -336,6 +342,7 @@ __global__ void __launch_bounds__(kDotNT)
 
 __global__ void __launch_bounds__(kDotNT)
     dot_finish(const double *partials, int count, double *out) {
+  ptx::grid_dependents_start();
   ptx::grid_dependency_wait();
   const double t = dot_partials_sum(partials, count);
   if (threadIdx.x == 0)
@@ -488,14 +495,14 @@ drb_status dot_launch(int64_t n, const void *a, const void *b, drb_dtype dt,
   if (grid > 1)
     DRB_TRY(scratch_alloc(&scratch, sizeof(double) * kDotGrid, s));
   double *partials = static_cast<double *>(scratch);
+  cudaError_t e;
   if (dt == DRB_F32)
-    dot_kernel<float, false><<<grid, kDotNT, 0, s>>>(n, (const float *)a, (const float *)b,
-                                                     partials, nullptr, out);
+    e = launch_overlapped(dot_kernel<float, false>, dim3(grid), dim3(kDotNT), 0, s, n,
+                          (const float *)a, (const float *)b, partials, (int *)nullptr, out);
   else
-    dot_kernel<double, false><<<grid, kDotNT, 0, s>>>(n, (const double *)a, (const double *)b,
-                                                      partials, nullptr, out);
+    e = launch_overlapped(dot_kernel<double, false>, dim3(grid), dim3(kDotNT), 0, s, n,
+                          (const double *)a, (const double *)b, partials, (int *)nullptr, out);
   note_launch();
-  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && grid > 1) {
     e = launch_overlapped(dot_finish, dim3(1), dim3(kDotNT), 0, s,
                           (const double *)partials, grid, out);

@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(kRedNT)
   using A = typename R::A;
   constexpr int PER = 16 / sizeof(T);
   ptx::grid_dependents_start();
+  ptx::grid_dependency_wait();
   const uint64_t pol = ptx::policy_evict_first();
   A acc = R::id();
   const int64_t tid = (int64_t)blockIdx.x * kRedNT + threadIdx.x;
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(kRedNT)
     reduce_finish(const typename ROp<T, OP>::A *partials, int count, bool has_init, T init,
                   T *out) {
   using R = ROp<T, OP>;
+  ptx::grid_dependents_start();
   ptx::grid_dependency_wait();
   typename R::A s = R::id();
   for (int i = threadIdx.x; i < count; i += kRedNT)
@@ -194,10 +196,11 @@ drb_status reduce_typed(int64_t n, const void *x, const void *init, void *out,
   if (grid > 1)
     DRB_TRY(scratch_alloc(&scratch, sizeof(A) * kRedGrid, s));
   A *partials = static_cast<A *>(scratch);
-  reduce_kernel<T, OP><<<grid, kRedNT, 0, s>>>(n, static_cast<const T *>(x), init != nullptr, iv,
-                                               partials, static_cast<T *>(out));
+  cudaError_t e =
+      launch_overlapped(reduce_kernel<T, OP>, dim3(grid), dim3(kRedNT), 0, s, n,
+                        static_cast<const T *>(x), init != nullptr, iv, partials,
+                        static_cast<T *>(out));
   note_launch();
-  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && grid > 1) {
     e = launch_overlapped(reduce_finish<T, OP>, dim3(1), dim3(kRedNT), 0, s,
                           (const A *)partials, grid, init != nullptr, iv, static_cast<T *>(out));
