@@ -197,13 +197,18 @@ __device__ __forceinline__ int clog2(int x) {
   return ilog2(x) + ((x & (x - 1)) ? 1 : 0);
 }
 
-// X gathers in flight per lane: 4, three CTAs per SM; with five or more lanes per
-// slot, not a power of two (at most six slots, one per row), 8, two CTAs per SM.
-// There rows are long chains of rounds in few slots, and each round waits for
-// its gathers: 0.5M rows of 8..64, f32, k = 28 502 -> 392 us, k = 33 719 -> 543,
-// f64 k = 20 795 -> 755; with fewer lanes a slot more warps do better (f32 k =
-// 12 202 -> 216, k = 16 547 -> 578, k = 8 144 -> 161).  BF16 storage keeps 4, the
-// block of its compensated sums.
+// X gathers in flight per lane: 4, three CTAs per SM; with seven or more lanes per
+// slot, not a power of two (few slots, one per row), 8, two CTAs per SM, and with
+// five or six where X does not stay in L2 either.  There rows are long chains of
+// rounds in few slots, and each round waits for its gathers: rows of 8..64, 0.5M
+// rows f32 k = 28 502 -> 392 us, k = 33 719 -> 543, f64 k = 20 795 -> 755, 1M rows
+// f32 k = 20 (X 80 MB) 738 -> 675; but 1.5M rows of 4..33 over an X of 37 MB, k =
+// 19, 364 -> 382, and with fewer lanes a slot more warps do better (f32 k = 12
+// 202 -> 216, k = 16 547 -> 578, k = 8 144 -> 161), as with vectors of less than
+// 16 bytes (row-major k = 21 963 -> 1122).  Rows shorter than a round repeat
+// their last gather: mean rows of under kWideRow nonzeros keep 4.  BF16 storage
+// keeps 4, the block of its compensated sums.
+constexpr int64_t kWideRow = 8;
 template <class V> constexpr int unroll_of(bool wide) { return wide && sizeof(V) > 2 ? 8 : 4; }
 
 // BF16 storage sums two-sum compensated, per block of the four products a
@@ -1085,7 +1090,15 @@ drb_status make_batch(Batch &B, int32_t count, Csr *const *handles,
   B.KB = B.KP * B.vec;
   B.nkb = (B.ldx + B.KB - 1) / B.KB;
   B.rmax = std::min(kRmax, std::max(1, kYBudget / ((B.KB + 1) * B.abytes)));
-  B.kernel = pick_kernel(B.storage, B.x_f32, B.vec, B.KP >= 5 && (B.KP & (B.KP - 1)));
+  int64_t rows = 0, nnz = 0, xbytes = 0;
+  for (const Csr *A : B.mats) {
+    rows += A->m;
+    nnz += A->nnz;
+    xbytes += A->n * B.ldx * B.xbytes;
+  }
+  const bool wide = B.vec * B.xbytes == 16 && (B.KP & (B.KP - 1)) && nnz >= kWideRow * rows &&
+                    (B.KP >= 7 || (B.KP >= 5 && xbytes > (int64_t)48 << 20));
+  B.kernel = pick_kernel(B.storage, B.x_f32, B.vec, wide);
   if (!B.kernel)
     return fail(DRB_ERR_UNSUPPORTED,
                 "no batch kernel for this type and vector width");
