@@ -23,6 +23,7 @@
 // at its first instruction.  Vectors are the matrix's value type (f32 / f64);
 // the scalars are f64.
 #include <cmath>
+#include <mutex>
 
 #include "cg_state.cuh"
 #include "drb_internal.cuh"
@@ -36,6 +37,7 @@ constexpr int kCgNT = 256;
 constexpr int kCgGrid = 148 * 3;
 constexpr int kCgMinBlocks = 3;
 constexpr int kCgBlock = 8;  // iterations per graph replay
+std::mutex g_resident_mu[64];
 } // namespace
 
 struct CgPlan {
@@ -402,14 +404,21 @@ drb_status solve(Csr &A, const T *b, T *x, int64_t max_iters, double rtol,
   int *ticket = reinterpret_cast<int *>(partials + 2 * kCgGrid);
 
   bool resident = cg_resident_wanted(A);
+  // One such solve at a time on a device: two grids that are each partly
+  // resident would wait for one another.  (Held until the solve has ended; the
+  // call synchronises anyway.)
+  std::unique_lock<std::mutex> alone(g_resident_mu[A.device < 64 ? A.device : 0],
+                                     std::defer_lock);
   if (resident) {
+    alone.lock();
     if (!C.sync.p)
       DRB_TRY(C.sync.alloc(cg_resident_sync_bytes()));
     DRB_TRY(cg_resident_launch<T>(A, b, x, C.r.as<T>(), C.p.as<T>(), C.q.as<T>(), st, C.sync.p,
                                   rtol, max_iters, true, &resident, s));
+    if (resident)
+      return finish_resident<T>(A, C, b, x, rtol, max_iters, info, s);
+    alone.unlock();
   }
-  if (resident)
-    return finish_resident<T>(A, C, b, x, rtol, max_iters, info, s);
   DRB_TRY(fused_scratch(A)); // allocated before any capture
 
   // r = b - A x0, p = r

@@ -28,8 +28,9 @@
 // read; 8 CTAs: 0.9 direct, 1.6 through CTA 0).  Sums are added in CTA order:
 // the same bits everywhere, repeatable.  The barrier is a counter with one
 // polling thread per CTA (1.3 us; a flag per CTA read by all: 5.1).  Every wait
-// gives up after one second of %globaltimer (DRB_ERR_TIMEOUT in the handle's
-// error word) and ends the launch.
+// gives up after ten seconds of %globaltimer (DRB_ERR_TIMEOUT in the handle's
+// error word) and ends the launch: long enough for CTAs that wait for another
+// stream's kernel to leave their SM.
 #include <algorithm>
 
 #include "drb_internal.cuh"
@@ -44,6 +45,7 @@ namespace {
 // 1307 us, 1448 2655 -> 2353; g = 300 726 -> 763).
 constexpr int kResNT = 768, kResNTMany = 1024;
 constexpr int kResManySlices = 64; // slices per CTA from which f32 takes 1024
+constexpr uint64_t kResWaitNs = 10 * tma::kWaitNs;
 constexpr int kResMinSlices = 16;  // slices per CTA at least, for small systems
 constexpr int kResMaxCtas = 256;   // exchange slots
 constexpr int kResDirect = 32;     // CTAs that read each other's sums directly
@@ -109,7 +111,7 @@ template <int NT> struct Grid {
       return false;
     if (spins == 63)
       t0 = tma::globaltimer();
-    else if (tma::globaltimer() - t0 > tma::kWaitNs)
+    else if (tma::globaltimer() - t0 > kResWaitNs)
       atomicExch(err, DRB_ERR_TIMEOUT);
     if (!*(volatile int *)err)
       return false;
