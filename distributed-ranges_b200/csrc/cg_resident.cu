@@ -68,7 +68,7 @@ template <class T> struct ResArgs {
   int cap;   // slices a CTA may own (shared-memory rows = 32 * cap)
   int nres;  // vectors held in shared memory: r, q, x, p in this order
   int first; // this launch starts the solve
-  int keep;  // the matrix stays in L2 between iterations
+  float keep; // share of the matrix that L2 is asked to keep between iterations
 };
 
 __device__ __forceinline__ double warp_down(double v) {
@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(NT, 1) cg_resident(const ResArgs<T> a) {
   for (int i = tid; i <= nsl; i += NT)
     soff[i] = (int)(a.off[s0 + i] - obase);
   Grid<NT> G{a.slots, a.count, a.err, s_red, s_sum, &s_stop};
-  const uint64_t pol = a.keep ? ptx::policy_evict_last() : ptx::policy_evict_first();
+  const uint64_t pol_keep = ptx::policy_evict_last(), pol_pass = ptx::policy_evict_first();
+  const int nkeep = (int)(a.keep * (float)nsl); // the first slices of every CTA
   __syncthreads();
 
   // The matrix runs ahead of its use: a slice's first K entries per row load
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(NT, 1) cg_resident(const ResArgs<T> a) {
   };
   auto fetch = [&](Part &s, int i, int k0) {
     const int o = soff[i], w = ((soff[i + 1] - o) >> 5) - k0;
+    const uint64_t pol = i < nkeep ? pol_keep : pol_pass;
     const T *va = a.vals + obase + o + 32 * k0 + lane;
     const int *ca = a.cols + obase + o + 32 * k0 + lane;
 #pragma unroll
@@ -506,7 +508,7 @@ drb_status cg_resident_launch(Csr &A, const T *b, T *x, T *r, T *p, T *q, CgStat
   a.cap = S.cap;
   a.nres = S.nres;
   a.first = first ? 1 : 0;
-  a.keep = A.sell.padded * (int64_t)(sizeof(T) + 4) <= kResKeepBytes ? 1 : 0;
+  a.keep = resident_keep(A.sell.padded * (int64_t)(sizeof(T) + 4), 4 * A.m * (int64_t)sizeof(T));
   DRB_CUDA_TRY(cudaMemsetAsync(sync, 0, kSyncBytes, s));
   void *args[] = {&a};
   const cudaError_t e = cudaLaunchCooperativeKernel(

@@ -24,10 +24,22 @@ struct CgState {
 // vectors fits the SMs, and three kernels on four CTAs per SM stream as fast: 64
 // iterations on a g x g Laplacian, launch per step / one launch, f64 g = 1900
 // 6013 / 5189 us, f32 1800 3954 / 3677, 2048 4785 / 4779, 2700 7914 / 8748),
-// and the matrix size up to which that launch asks L2 to keep the matrix between
-// iterations.
+// and how much of the matrix it asks L2 to keep between iterations.
 constexpr int64_t kResMaxRows = 3670016;
 constexpr int64_t kResKeepBytes = (int64_t)72 << 20;
+
+// The whole matrix up to kResKeepBytes; above that what the four vectors leave of
+// it, possibly nothing.  64 iterations, f64 g = 1250 / 1448 / 1800 and
+// f32 1448 / 1600 / 1800, with a fixed amount kept of a matrix that does not fit:
+// none 2256 / 3062 / 4719, 2550 / 2984 / 3435 us; 24 MB 2188 / 2986 / 5221, 2451 /
+// 2883 / 3353; 56 MB 2263 / 3163 / 5527, 2383 / 2826 / 3492; 72 MB slower still
+// except where all of it fits (f64 1024: 56 MB 1522, 72 MB 1501).  With the rule
+// 2188 / 3017 / 4722, 2416 / 2857 / 3358.
+inline float resident_keep(int64_t matrix_bytes, int64_t vector_bytes) {
+  if (matrix_bytes <= kResKeepBytes) return 1.0f;
+  const int64_t left = kResKeepBytes - vector_bytes;
+  return left > 0 ? (float)left / (float)matrix_bytes : 0.0f;
+}
 
 bool cg_resident_wanted(const Csr &A);
 size_t cg_resident_sync_bytes();
