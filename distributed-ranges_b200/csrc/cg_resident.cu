@@ -235,8 +235,7 @@ __global__ void __launch_bounds__(NT, 1) cg_resident(const ResArgs<T> a) {
   for (int i = tid; i <= nsl; i += NT)
     soff[i] = (int)(a.off[s0 + i] - obase);
   Grid<NT> G{a.slots, a.count, a.err, s_red, s_sum, &s_stop};
-  const uint64_t pol_keep = ptx::policy_evict_last(), pol_pass = ptx::policy_evict_first();
-  const int nkeep = (int)(a.keep * (float)nsl); // the first slices of every CTA
+  const uint64_t pol = a.keep > 0.0f ? ptx::policy_keep(a.keep) : ptx::policy_evict_first();
   __syncthreads();
 
   // The matrix runs ahead of its use: a slice's first K entries per row load
@@ -249,7 +248,6 @@ __global__ void __launch_bounds__(NT, 1) cg_resident(const ResArgs<T> a) {
   };
   auto fetch = [&](Part &s, int i, int k0) {
     const int o = soff[i], w = ((soff[i + 1] - o) >> 5) - k0;
-    const uint64_t pol = i < nkeep ? pol_keep : pol_pass;
     const T *va = a.vals + obase + o + 32 * k0 + lane;
     const int *ca = a.cols + obase + o + 32 * k0 + lane;
 #pragma unroll

@@ -3,6 +3,8 @@
 // (cg_resident.cu).
 #pragma once
 
+#include <algorithm>
+
 #include "drb_internal.cuh"
 
 namespace drb {
@@ -29,16 +31,16 @@ constexpr int64_t kResMaxRows = 3670016;
 constexpr int64_t kResKeepBytes = (int64_t)72 << 20;
 
 // The whole matrix up to kResKeepBytes; above that what the four vectors leave of
-// it, possibly nothing.  64 iterations, f64 g = 1250 / 1448 / 1800 and
-// f32 1448 / 1600 / 1800, with a fixed amount kept of a matrix that does not fit:
-// none 2256 / 3062 / 4719, 2550 / 2984 / 3435 us; 24 MB 2188 / 2986 / 5221, 2451 /
-// 2883 / 3353; 56 MB 2263 / 3163 / 5527, 2383 / 2826 / 3492; 72 MB slower still
-// except where all of it fits (f64 1024: 56 MB 1522, 72 MB 1501).  With the rule
-// 2188 / 3017 / 4722, 2416 / 2857 / 3358.
+// it, possibly nothing, in the sixteenths of the matrix that a cache policy tells
+// apart (rounded up by the hardware, 0.4% of g = 1530 cost 5%).  64 iterations, us,
+// nothing kept of a matrix that does not fit / this rule: f64 g = 1140
+// 2074 / 1971, 1250 2086 / 1997, 1448 3014 / 2991, 1530 2964 / 2963; f32 1400
+// 2303 / 2104, 1448 2377 / 2202, 1600 2741 / 2610, 1800 3026 / 3005.  A fixed amount
+// fits some sizes only: 40 MB 1893 at g = 1140, but 3522 at 1530 and 5399 (4419) at 1800.
 inline float resident_keep(int64_t matrix_bytes, int64_t vector_bytes) {
   if (matrix_bytes <= kResKeepBytes) return 1.0f;
-  const int64_t left = kResKeepBytes - vector_bytes;
-  return left > 0 ? (float)left / (float)matrix_bytes : 0.0f;
+  const int64_t left = std::max<int64_t>(kResKeepBytes - vector_bytes, 0);
+  return (float)(16 * left / matrix_bytes) / 16.0f;
 }
 
 bool cg_resident_wanted(const Csr &A);

@@ -391,6 +391,12 @@ __device__ __forceinline__ uint64_t policy_evict_last() {
   asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
+// evict-last for a share (0, 1] of the lines, evict-first for the others.
+__device__ __forceinline__ uint64_t policy_keep(float share) {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(p) : "f"(share));
+  return p;
+}
 
 // 16-byte streaming load through the non-coherent path, not allocated in L1.
 __device__ __forceinline__ uint4 ld_stream16(const void *ptr, uint64_t pol) {
