@@ -9,9 +9,9 @@
 // ceil(k / 8) passes over HBM, and rows that do not start on 16 bytes went
 // through single-element loads with few of them in flight.
 //
-// Measured (us): 5003 x 3001 f64 with 20 right-hand sides 246 -> 53, f32 428 -> 44;
-// 8192^2 f32 with 20 336 -> 112, with 8 143 -> 73, with 4 61 -> 57; 4096 x 8192
-// f64 with 32 428 -> 101.  (One CTA of 16 warps per SM with tiles twice as high
+// Measured (us): 5003 x 3001 f64 with 20 right-hand sides 246 -> 48, f32 429 -> 38;
+// 8192^2 f32 with 20 334 -> 94, with 8 136 -> 58, with 4 61 -> 51; 4096 x 8192
+// f64 with 32 429 -> 100.  (One CTA of 16 warps per SM with tiles twice as high
 // ran the f64 case in 57: all warps loaded, waited and multiplied in step.)
 //
 // Tiles and split.  A CTA of 8 warps owns a tile of BM rows and walks along the
@@ -101,6 +101,10 @@ struct PanelArgs {
 // Measured, us, short / long: 8192^2 f32 k = 20 105 / 94, 8191^2 k = 3 83 / 69,
 // 8191 x 4095 f64 k = 5 80 / 70; 16000 x 300 f32 k = 12 9.9 / 11.1, 5003 x 3001
 // f64 k = 20 49.7 / 51.3.
+// f64 keeps three short chunks per CTA in the ring, with more than 24 right-hand
+// sides two (three / two, us: 8192 x 4096 k = 20 66 / 71, k = 32 100 / 95; 8192 x 1024
+// k = 32 38 / 33, 5003 x 3001 k = 32 58 / 57).  Three CTAs of two chunks (8192 x 4096
+// k = 20: 80) and warps of 32 rows (81; k = 32 105) measured slower.
 template <class V, int P, bool SH, bool LONG> struct Shape;
 template <int C, bool SH, bool LONG>
 struct Shape<float, C, SH, LONG> { // C right-hand sides
@@ -112,7 +116,7 @@ template <int NT, bool SH, bool LONG>
 struct Shape<double, NT, SH, LONG> { // 8 NT right-hand sides
   static constexpr int R = 16;
   static constexpr int BM = kWarps / 2 * R, KC = LONG ? 64 : 32, AS = KC + (SH ? 4 : 8), XS = AS;
-  static constexpr int CP = 8 * NT, STAGES = LONG ? 2 : 3;
+  static constexpr int CP = 8 * NT, STAGES = LONG || NT == 4 ? 2 : 3;
   static constexpr int MERGE = BM * CP; // the second half's sums of a tile
 };
 template <class V, int P> constexpr bool may_be_long() { return sizeof(V) == 4 || P <= 2; }
