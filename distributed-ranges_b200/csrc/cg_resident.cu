@@ -14,8 +14,8 @@
 //   p = r + beta p      -> grid barrier (p is gathered by other CTAs next)
 //
 // Measured (64 iterations on a g x g Laplacian, us, launch per step -> here):
-// f64 g = 48 787 -> 491, 512 1455 -> 801, 1024 2386 -> 1343, 1448 3672 -> 3000,
-// 1800 5462 -> 4502; f32 300 1088 -> 720, 1024 2134 -> 1307, 1448 2979 -> 2353.
+// f64 g = 48 787 -> 491, 512 1455 -> 801, 1024 2386 -> 1347, 1448 3672 -> 2991,
+// 1800 5462 -> 4367; f32 300 1088 -> 720, 1024 2134 -> 1307, 1448 2979 -> 2202.
 // What is left at small sizes is the chain of three grid-wide steps (about 5 us
 // of 11 an iteration on all SMs), at large ones the matrix's bytes.
 //

@@ -391,10 +391,13 @@ drb_status drb_fill(int64_t n, void *x, drb_dtype dtype, const void *value,
  *   r = b - A x;  p = r;  rr = r.r
  *   repeat: q = A p;  alpha = rr / p.q;  x += alpha p;  r -= alpha q;
  *           rr' = r.r;  stop if rr' <= rtol^2 b.b;  p = r + (rr'/rr) p
- * The SpMV carries the p.q reduction in its epilogue; the x/r update carries
- * r.r.  Scalars stay in device memory (f64); the loop is replayed from a
- * CUDA graph in blocks of 8 iterations with one small device-to-host read
- * per block, and iterations after convergence return at once.  Stops on
+ * Scalars stay on the device (f64).  A matrix with short, regular rows (a
+ * sliced-ELL copy) and 1024 to 3,670,016 rows is solved by one cooperative
+ * launch per 1024 iterations, which wants every SM: such solves take turns on
+ * a device.  Any other loop is replayed from a CUDA graph in blocks of 8
+ * iterations (the SpMV carries p.q in its epilogue, the x/r update r.r) with
+ * one small device-to-host read per block; iterations after convergence
+ * return at once.  Stops on
  * convergence, at max_iters updates, or on breakdown (p.q <= 0 or not finite:
  * A is not SPD; x is left as it was before that iteration).  The call
  * synchronises `stream`. */
