@@ -41,11 +41,14 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
 // pieces meet in shared memory; else the steps are shared over the whole grid
 // and dense_row_join adds the pieces.  (Whole 32 KB row slabs per warp, the
 // earlier unit, left 8192 rows on 7104 warps: some did two while the others
-// had finished one.  8192^2 f32 53.8 -> 46.8 us = 0.89 of the measured HBM
-// rate, 4001^2 f32, whose rows are not aligned, 73 -> 32.)
-template <class V, bool VEC> constexpr int row_unroll() {
-  return VEC ? (sizeof(V) == 4 ? 4 : 8) : 16;
-}
+// had finished one.  8192^2 f32 54.9 -> 45.2 us = 0.92 of the measured HBM
+// rate, f64 90.9 -> 86, 4001^2 f32, whose rows are not aligned, 73 -> 30; four times
+// as many CTAs' worth of rows hide that: 24000^2 f32 353 -> 356, 32768^2 622 -> 642.)
+// U pieces per lane and step: 8, but 4 for f32 rows under 32 KB, whose last step would
+// be mostly empty (us, U = 4 / 8: 20000 x 500 9.8 / 10.8, 4096^2 14.9 / 15.5;
+// 8192^2 46.3 / 45.6, 24000^2 367 / 361, 8192 x 65536 335 / 328, 32768^2 658 / 648), and 16
+// single elements.
+constexpr int64_t kLongRowBytes = 32768;
 
 struct RowShare { // the steps [s0, s1) of warp w of W over `steps`, from `base`
   int64_t s0, s1;
@@ -74,12 +77,11 @@ __device__ __forceinline__ void join_cut_row(int64_t base, int64_t steps, int64_
   y[row] = s;
 }
 
-template <class V, bool VEC, bool LOCAL>
+template <class V, bool VEC, bool LOCAL, int U>
 __global__ void __launch_bounds__(kDenseNT)
     dense_row_kernel(int64_t m, int64_t n, const V *__restrict__ A, int64_t lda,
                      const V *__restrict__ x, V *__restrict__ y, int64_t spr, V *frag) {
   constexpr int PER = VEC ? 16 / (int)sizeof(V) : 1;
-  constexpr int U = row_unroll<V, VEC>();
   constexpr int NW = kDenseNT / 32;
   __shared__ V s_frag[2 * NW];
   ptx::grid_dependents_start();
@@ -106,21 +108,35 @@ __global__ void __launch_bounds__(kDenseNT)
         V t[PER];
       };
       G16 a[U];
+      if ((q + 1) * (32 * U) <= ng) { // no predicates: all loads go out at once
 #pragma unroll
-      for (int i = 0; i < U; i++) {
-        a[i].u = make_uint4(0, 0, 0, 0);
-        if (g0 + 32 * i < ng)
+        for (int i = 0; i < U; i++)
           a[i].u = ptx::ld_stream16(Ar + (g0 + 32 * i) * PER, pol_s);
-      }
 #pragma unroll
-      for (int i = 0; i < U; i++)
-        if (g0 + 32 * i < ng) {
+        for (int i = 0; i < U; i++) {
           G16 xv;
           xv.u = __ldg(reinterpret_cast<const uint4 *>(x) + g0 + 32 * i);
 #pragma unroll
           for (int e = 0; e < PER; e++)
             acc += a[i].t[e] * xv.t[e];
         }
+      } else {
+#pragma unroll
+        for (int i = 0; i < U; i++) {
+          a[i].u = make_uint4(0, 0, 0, 0);
+          if (g0 + 32 * i < ng)
+            a[i].u = ptx::ld_stream16(Ar + (g0 + 32 * i) * PER, pol_s);
+        }
+#pragma unroll
+        for (int i = 0; i < U; i++)
+          if (g0 + 32 * i < ng) {
+            G16 xv;
+            xv.u = __ldg(reinterpret_cast<const uint4 *>(x) + g0 + 32 * i);
+#pragma unroll
+            for (int e = 0; e < PER; e++)
+              acc += a[i].t[e] * xv.t[e];
+          }
+      }
       if (q + 1 == spr && ng * PER + lane < n) // the elements after the last piece
         acc += Ar[ng * PER + lane] * __ldg(x + ng * PER + lane);
     } else {
@@ -164,11 +180,11 @@ __global__ void dense_row_join(int64_t steps, int64_t spr, int64_t W, const V *f
     join_cut_row<V>(0, steps, spr, w, W, frag, y);
 }
 
-template <class V, bool VEC>
+template <class V, bool VEC, int U>
 drb_status dense_row_call(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, V *y,
                           cudaStream_t s) {
   constexpr int PER = VEC ? 16 / (int)sizeof(V) : 1;
-  constexpr int64_t STEP = 32 * row_unroll<V, VEC>(); // pieces per step
+  constexpr int64_t STEP = 32 * U; // pieces per step
   static int grid_cache[64] = {0};
   int dev = 0;
   DRB_CUDA_TRY(cudaGetDevice(&dev));
@@ -176,7 +192,7 @@ drb_status dense_row_call(int64_t m, int64_t n, const V *A, int64_t lda, const V
   if (full == 0) {
     int occ = 0, sms = 0;
     DRB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &occ, dense_row_kernel<V, VEC, true>, kDenseNT, 0));
+        &occ, dense_row_kernel<V, VEC, true, U>, kDenseNT, 0));
     DRB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     full = std::max(1, occ) * sms;
   }
@@ -190,7 +206,7 @@ drb_status dense_row_call(int64_t m, int64_t n, const V *A, int64_t lda, const V
   cudaError_t e;
   if (local) {
     const unsigned g = (unsigned)std::min<int64_t>(full, m);
-    e = launch_overlapped(dense_row_kernel<V, VEC, true>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
+    e = launch_overlapped(dense_row_kernel<V, VEC, true, U>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
                           lda, x, y, spr, (V *)nullptr);
     note_launch();
   } else {
@@ -198,7 +214,7 @@ drb_status dense_row_call(int64_t m, int64_t n, const V *A, int64_t lda, const V
     const int64_t W = (int64_t)g * NW;
     V *frag = nullptr;
     DRB_TRY(scratch_alloc(reinterpret_cast<void **>(&frag), sizeof(V) * 2 * (size_t)W, s));
-    e = launch_overlapped(dense_row_kernel<V, VEC, false>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
+    e = launch_overlapped(dense_row_kernel<V, VEC, false, U>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
                           lda, x, y, spr, frag);
     note_launch();
     if (e == cudaSuccess) {
@@ -220,8 +236,12 @@ drb_status dense_row(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, 
                      cudaStream_t s) {
   const bool vec = reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(x) % 16 == 0 && lda * sizeof(V) % 16 == 0;
-  return vec ? dense_row_call<V, true>(m, n, A, lda, x, y, s)
-             : dense_row_call<V, false>(m, n, A, lda, x, y, s);
+  if (!vec)
+    return dense_row_call<V, false, 16>(m, n, A, lda, x, y, s);
+  if constexpr (sizeof(V) == 4)
+    if (n * (int64_t)sizeof(V) < kLongRowBytes)
+      return dense_row_call<V, true, 4>(m, n, A, lda, x, y, s);
+  return dense_row_call<V, true, 8>(m, n, A, lda, x, y, s);
 }
 
 // ---- dot -------------------------------------------------------------------------

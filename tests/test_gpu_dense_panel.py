@@ -63,6 +63,7 @@ def test_misaligned_base(mp, dtype, k):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("m,n,lda", [
     (1, 3, 3), (2, 511, 512), (3, 513, 513), (100, 2049, 2052), (889, 1000, 1000),
+    (3, 8191, 8192), (5, 8192, 8192), (700, 8201, 8204), (2, 40003, 40004),
     # over 16 MB with few rows per CTA: rows cut between CTAs
     (5, 1_000_003, 1_000_004), (40, 131_073, 131_073), (1500, 3001, 3001),
     # whole rows per CTA
