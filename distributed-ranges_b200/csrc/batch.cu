@@ -33,6 +33,7 @@
 // rows are padded to a multiple of VEC.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "drb_internal.cuh"
@@ -284,7 +285,11 @@ __device__ __forceinline__ uint64_t x_pair(const XWords<XT, VEC> &o, int p) {
 // The nonzeros [b, e) of one row staged at shared addresses colS/valS (byte
 // address of stage element 0), this lane's VEC sums (and, compensated, their
 // error terms cmp); the lane takes b, b + step, ... with UN gathers in
-// flight.  f32 sums of an even VEC run on packed pairs.
+// flight.  f32 sums of an even VEC run on packed pairs.  Places past the
+// lane's last nonzero multiply a repeated gather by 0, which makes a NaN of a
+// row's infinity: the caller takes plain sums that came out as one again with
+// UN = 1, which has no such places.  (Skipping them here cost 1.6%: rows of 8..64, f32,
+// k = 16 552 -> 561 us, k = 20 676 -> 688.)
 template <class V, class XT, int VEC, int UN, class A>
 __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
                                          int e, const XT *Xl, int ldx,
@@ -398,6 +403,15 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
   }
 }
 
+// Any of a lane's sums is not a number.
+template <int VEC, class A> __device__ __forceinline__ bool any_nan(const A (&acc)[VEC]) {
+  bool r = false;
+#pragma unroll
+  for (int t = 0; t < VEC; t++)
+    r |= acc[t] != acc[t];
+  return r;
+}
+
 // acc += other lane's (acc2, cmp2): compensated when the storage is BF16.
 template <class V, class A>
 __device__ __forceinline__ void merge_sum(A &acc, A &cmp, A acc2, A cmp2) {
@@ -495,31 +509,42 @@ __global__ void __launch_bounds__(256, UN == 4 ? 3 : 2) batch_spmm(const BArgs a
       const uint32_t colP = colS + 4 * (p0 & 3);
       const uint32_t valP = valS + (uint32_t)sizeof(V) * (p0 & VOFF_MASK);
       const uint32_t rsP = wsm + a.rs_off + st * a.rs_stage + 4 * (r0 & 3);
-      for (int i0 = 0; i0 < nrows; i0 += R) {
-        const int i = i0 + grp;
-        A acc[VEC], cmp[VEC];
-#pragma unroll
-        for (int t = 0; t < VEC; t++)
-          acc[t] = cmp[t] = 0;
-        if (con && row_on && i < nrows) {
-          const int b = lds_s32(rsP + 4 * i) - p0, e = lds_s32(rsP + 4 * i + 4) - p0;
-          row_sums<V, XT, VEC, UN, A>(colP, valP, b + gs, e, Xl, ldx, G, acc, cmp);
-        }
-        for (int dd = 1; dd < G; dd <<= 1) {
-#pragma unroll
-          for (int t = 0; t < VEC; t++) {
-            const A a2 = __shfl_xor_sync(0xffffffffu, acc[t], dd * KP);
-            const A c2 = Comp<V>::value ? __shfl_xor_sync(0xffffffffu, cmp[t], dd * KP) : A(0);
-            merge_sum<V>(acc[t], cmp[t], a2, c2);
-          }
-        }
-        if (con && row_on && gs == 0 && i < nrows) {
+      auto rows = [&](auto in_flight) {
+        bool nan = false;
+        for (int i0 = 0; i0 < nrows; i0 += R) {
+          const int i = i0 + grp;
+          A acc[VEC], cmp[VEC];
 #pragma unroll
           for (int t = 0; t < VEC; t++)
-            ytile[i * ystride + jj * VEC + t] = Comp<V>::value ? acc[t] + cmp[t] : acc[t];
+            acc[t] = cmp[t] = 0;
+          if (con && row_on && i < nrows) {
+            const int b = lds_s32(rsP + 4 * i) - p0, e = lds_s32(rsP + 4 * i + 4) - p0;
+            row_sums<V, XT, VEC, in_flight.value, A>(colP, valP, b + gs, e, Xl, ldx, G, acc,
+                                                     cmp);
+          }
+          nan |= any_nan(acc);
+          for (int dd = 1; dd < G; dd <<= 1) {
+#pragma unroll
+            for (int t = 0; t < VEC; t++) {
+              const A a2 = __shfl_xor_sync(0xffffffffu, acc[t], dd * KP);
+              const A c2 =
+                  Comp<V>::value ? __shfl_xor_sync(0xffffffffu, cmp[t], dd * KP) : A(0);
+              merge_sum<V>(acc[t], cmp[t], a2, c2);
+            }
+          }
+          if (con && row_on && gs == 0 && i < nrows) {
+#pragma unroll
+            for (int t = 0; t < VEC; t++)
+              ytile[i * ystride + jj * VEC + t] = Comp<V>::value ? acc[t] + cmp[t] : acc[t];
+          }
         }
-      }
-      __syncwarp();
+        __syncwarp();
+        return nan;
+      };
+      const bool nan = rows(std::integral_constant<int, UN>());
+      if constexpr (!Comp<V>::value)
+        if (__any_sync(0xffffffffu, nan))
+          rows(std::integral_constant<int, 1>());
       // the tile to Y, coalesced: lanes map (row, column) by powers of two
       const int kbv = min(KB, k - jb);
       if (a.row_major) {
@@ -546,22 +571,28 @@ __global__ void __launch_bounds__(256, UN == 4 ? 3 : 2) batch_spmm(const BArgs a
       // ---- one long row, staged cap nonzeros at a time into stage st ----
       const int64_t lo0 = bm->rowptr[r0], hi0 = bm->rowptr[r0 + 1];
       A acc[VEC], cmp[VEC];
+      auto row = [&](auto in_flight) {
 #pragma unroll
-      for (int t = 0; t < VEC; t++)
-        acc[t] = cmp[t] = 0;
-      for (int64_t lo = lo0; lo < hi0; lo += a.cap) {
-        const int len = (int)min((int64_t)a.cap, hi0 - lo);
-        copy16s<int32_t>(colS, bm->colind, lo, len, lane);
-        copy16s<V>(valS, static_cast<const V *>(bm->vals), lo, len, lane);
-        cp_commit();
-        cp_wait<0>();
-        __syncwarp();
-        if (con)
-          row_sums<V, XT, VEC, UN, A>(colS + 4 * (int)(lo & 3),
-                                  valS + (uint32_t)sizeof(V) * (int)(lo & VOFF_MASK),
-                                  slot, len, Xl, ldx, S, acc, cmp);
-        __syncwarp();
-      }
+        for (int t = 0; t < VEC; t++)
+          acc[t] = cmp[t] = 0;
+        for (int64_t lo = lo0; lo < hi0; lo += a.cap) {
+          const int len = (int)min((int64_t)a.cap, hi0 - lo);
+          copy16s<int32_t>(colS, bm->colind, lo, len, lane);
+          copy16s<V>(valS, static_cast<const V *>(bm->vals), lo, len, lane);
+          cp_commit();
+          cp_wait<0>();
+          __syncwarp();
+          if (con)
+            row_sums<V, XT, VEC, in_flight.value, A>(
+                colS + 4 * (int)(lo & 3), valS + (uint32_t)sizeof(V) * (int)(lo & VOFF_MASK),
+                slot, len, Xl, ldx, S, acc, cmp);
+          __syncwarp();
+        }
+      };
+      row(std::integral_constant<int, UN>());
+      if constexpr (!Comp<V>::value)
+        if (__any_sync(0xffffffffu, any_nan(acc)))
+          row(std::integral_constant<int, 1>());
       for (int dd = 1; dd < S; dd <<= 1) {
 #pragma unroll
         for (int t = 0; t < VEC; t++) {

@@ -269,3 +269,30 @@ def test_batch_rejects_mixed_and_misaligned(mp):
         b.gemv()  # nothing bound
     assert e.value.status == capi.DRB_ERR_INVALID_ARG
     b.destroy()
+
+
+@pytest.mark.parametrize("layout", [COL, ROW])
+@pytest.mark.parametrize("dtype,k", [(np.float32, 1), (np.float32, 3), (np.float32, 16),
+                                     (np.float32, 28), (np.float64, 5), (np.float64, 14)])
+def test_infinite_x_stays_infinite(mp, dtype, k, layout):
+    """Rows of every length from 1 to 41 that end on the one column whose x is
+    infinite: each output is that element's product, never a NaN, whatever the
+    row's place in a round of gathers."""
+    rng = np.random.default_rng(5)
+    m, n = 1640, 3000
+    lens = 1 + np.arange(m) % 41
+    rp = np.zeros(m + 1, np.int32)
+    rp[1:] = np.cumsum(lens)
+    ci = np.concatenate([np.append(np.sort(rng.choice(n - 1, int(L) - 1, replace=False)), n - 1)
+                         for L in lens]).astype(np.int32)
+    v = rng.uniform(0.5, 1.0, int(rp[-1])).astype(dtype) * rng.choice([-1, 1], int(rp[-1]))
+    v = v.astype(dtype)
+    x_cm = rng.uniform(-1, 1, n * k).astype(dtype)
+    x_cm.reshape(k, n)[:, n - 1] = np.inf
+    a = mp.distributed_sparse_matrix(mp.csr_matrix_view(v, rp, ci, (m, n)), 0)
+    x = torch.from_numpy(to_layout(x_cm, n, k, layout)).cuda()
+    y = torch.zeros(m * k, dtype=x.dtype, device="cuda")
+    mp.batched_gemv([a], [x], [y], k, layout)
+    got = from_layout(y.cpu().numpy(), m, k, layout).reshape(k, m)
+    want = np.where(v[rp[1:] - 1] > 0, np.inf, -np.inf)
+    assert np.array_equal(got, np.broadcast_to(want, (k, m)))
