@@ -457,17 +457,22 @@ template <class V, class XT, class CI, class RI, int TILE, bool SKEW, bool COMP>
   }
 };
 
-// The last CTA to get here leaves the work counter counters[0] (and its own
-// arrivals, counters[1]) at zero for the next launch: every warp has taken its
-// last batch by then.  (A memset before each launch was a launch of its own
+// The last CTA to get here leaves the work counter counters[0] at zero for the
+// next launch: every warp has taken its last batch by then.  The CTAs' arrivals
+// counters[1] add up to 0 over a whole launch whatever its grid (the last block
+// takes back what the others added) and are never stored to, so that launches
+// of one handle that were wrongly run at the same time leave both words at zero
+// too once all have ended: their own results are lost, the handle is not.  (A
+// memset before each launch was a launch of its own
 // with its gap, and kept the product from starting under its predecessor's
 // tail: power-law rows, f32, 50k rows 27.7 -> 23.1 us with the rest of the
 // launches overlapped too, 0.3M 42.7 -> 39.8, 2M 180.5 -> 178.4.)
 __device__ __forceinline__ void reset_counter(int *counters) {
   __syncthreads();
-  if (threadIdx.x == 0 && atomicAdd(counters + 1, 1) == (int)gridDim.x - 1) {
-    counters[0] = 0;
-    counters[1] = 0;
+  if (threadIdx.x == 0) {
+    const int share = blockIdx.x + 1 < gridDim.x ? 1 : 1 - (int)gridDim.x;
+    if (atomicAdd(counters + 1, share) + share == 0)
+      counters[0] = 0;
   }
 }
 

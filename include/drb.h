@@ -42,7 +42,9 @@
  * DRB_ROW_MAJOR (x[c*k + j], y[r*k + j]) is also accepted.
  *
  * Threads and streams.  Distinct handles may be used concurrently on distinct
- * streams; one handle must not be used by two threads at once.  All compute
+ * streams; one handle must not be used by two threads at once, and its calls
+ * must follow one another in stream order (one stream, or events between
+ * streams): they share the handle's work buffers.  All compute
  * entry points are asynchronous on the given stream (a cudaStream_t passed as
  * void*; NULL = the legacy default stream) except the *_host variants, which
  * synchronise the stream before returning.
