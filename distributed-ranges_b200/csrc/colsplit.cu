@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256)
 constexpr int kCombineRows = 4;
 
 template <class Acc>
-__device__ __forceinline__ void combine4(const Acc *__restrict__ ys, int64_t m, int64_t r,
+__device__ __forceinline__ void combine4(const Acc *ys, int64_t m, int64_t r,
                                          int64_t stride, int64_t r1, int nblk,
                                          Acc (&t)[kCombineRows]) {
 #pragma unroll
@@ -177,7 +177,7 @@ template <class Acc>
 __global__ void split_combine(const Acc *__restrict__ ys, Acc *__restrict__ y, int64_t m,
                               int64_t r0, int64_t r1, int nblk) {
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(ys);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < r1;
        r += kCombineRows * stride) {
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256)
   __shared__ double s_red[8];
   __shared__ int s_last;
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(ys, b);
   double sum = 0.0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;

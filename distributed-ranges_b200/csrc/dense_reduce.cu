@@ -78,14 +78,14 @@ __device__ __forceinline__ void join_cut_row(int64_t base, int64_t steps, int64_
 }
 
 template <class V, bool VEC, bool LOCAL, int U>
-__global__ void __launch_bounds__(kDenseNT)
+__global__ void __launch_bounds__(kDenseNT, 4)
     dense_row_kernel(int64_t m, int64_t n, const V *__restrict__ A, int64_t lda,
                      const V *__restrict__ x, V *__restrict__ y, int64_t spr, V *frag) {
   constexpr int PER = VEC ? 16 / (int)sizeof(V) : 1;
   constexpr int NW = kDenseNT / 32;
   __shared__ V s_frag[2 * NW];
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(A, x);
   const uint64_t pol_s = ptx::policy_evict_first();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t r0 = LOCAL ? m * blockIdx.x / gridDim.x : 0;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kDenseNT)
 #pragma unroll
         for (int i = 0; i < U; i++) {
           G16 xv;
-          xv.u = __ldg(reinterpret_cast<const uint4 *>(x) + g0 + 32 * i);
+          xv.u = reinterpret_cast<const uint4 *>(x)[g0 + 32 * i];
 #pragma unroll
           for (int e = 0; e < PER; e++)
             acc += a[i].t[e] * xv.t[e];
@@ -131,14 +131,14 @@ __global__ void __launch_bounds__(kDenseNT)
         for (int i = 0; i < U; i++)
           if (g0 + 32 * i < ng) {
             G16 xv;
-            xv.u = __ldg(reinterpret_cast<const uint4 *>(x) + g0 + 32 * i);
+            xv.u = reinterpret_cast<const uint4 *>(x)[g0 + 32 * i];
 #pragma unroll
             for (int e = 0; e < PER; e++)
               acc += a[i].t[e] * xv.t[e];
           }
       }
       if (q + 1 == spr && ng * PER + lane < n) // the elements after the last piece
-        acc += Ar[ng * PER + lane] * __ldg(x + ng * PER + lane);
+        acc += Ar[ng * PER + lane] * x[ng * PER + lane];
     } else {
       V a[U];
 #pragma unroll
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kDenseNT)
 #pragma unroll
       for (int i = 0; i < U; i++)
         if (g0 + 32 * i < ng)
-          acc += a[i] * __ldg(x + g0 + 32 * i);
+          acc += a[i] * x[g0 + 32 * i];
     }
     q++;
     if (q == spr || s + 1 == me.s1) {
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kDenseNT)
 template <class V>
 __global__ void dense_row_join(int64_t steps, int64_t spr, int64_t W, const V *frag, V *y) {
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(frag);
   const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (w < W)
     join_cut_row<V>(0, steps, spr, w, W, frag, y);
@@ -247,7 +247,9 @@ drb_status dense_row(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, 
 // ---- dot -------------------------------------------------------------------------
 constexpr int kDotNT = 256;
 constexpr int kDotGrid = 592; // at most; a function of n only: the order must not vary
-constexpr int kDotUnroll = 4; // 16-byte loads in flight per vector per thread
+// 16-byte loads in flight per vector per thread.  (f64, 3 / 4: two vectors of 40 MB
+// 12.5 / 15.3 us, of 240 MB 70.0 / 70.5; f32 16.9 / 13.6 and 74.9 / 71.0.)
+template <class V> constexpr int kDotUnroll = sizeof(V) == 8 ? 3 : 4;
 
 // The CTA's sum of v, in thread 0.
 __device__ __forceinline__ double dot_cta_sum(double v) {
@@ -283,10 +285,10 @@ template <class V, bool TICKET>
 __global__ void __launch_bounds__(kDotNT)
     dot_kernel(int64_t n, const V *__restrict__ a, const V *__restrict__ b,
                double *partials, int *ticket, double *out) {
-  constexpr int PER = 16 / sizeof(V);
+  constexpr int PER = 16 / sizeof(V), U = kDotUnroll<V>;
   if (!TICKET) {
     ptx::grid_dependents_start();
-    ptx::grid_dependency_wait();
+    ptx::grid_dependency_wait(a, b);
   }
   const uint64_t pol_s = ptx::policy_evict_first();
   double acc = 0.0;
@@ -301,34 +303,44 @@ __global__ void __launch_bounds__(kDotNT)
       V t[PER];
     };
     const int64_t nv = n / PER;
-    auto add = [&](const W (&wa)[kDotUnroll], const W (&wb)[kDotUnroll]) {
+    auto add = [&](const W (&wa)[U], const W (&wb)[U]) {
 #pragma unroll
-      for (int u = 0; u < kDotUnroll; u++)
+      for (int u = 0; u < U; u++)
 #pragma unroll
         for (int q = 0; q < PER; q++)
           acc += (double)wa[u].t[q] * (double)wb[u].t[q];
     };
     int64_t i = tid;
-    for (; i + (kDotUnroll - 1) * nth < nv; i += kDotUnroll * nth) {
-      W wa[kDotUnroll], wb[kDotUnroll];
+    if (a == b) { // a squared norm: one stream
+      for (; i + (U - 1) * nth < nv; i += U * nth) {
+        W wa[U];
 #pragma unroll
-      for (int u = 0; u < kDotUnroll; u++)
-        wa[u].u = ptx::ld_stream16(a + (i + u * nth) * PER, pol_s);
+        for (int u = 0; u < U; u++)
+          wa[u].u = ptx::ld_stream16(a + (i + u * nth) * PER, pol_s);
+        add(wa, wa);
+      }
+    } else {
+      for (; i + (U - 1) * nth < nv; i += U * nth) {
+        W wa[U], wb[U];
 #pragma unroll
-      for (int u = 0; u < kDotUnroll; u++)
-        wb[u].u = (a == b) ? wa[u].u : ptx::ld_stream16(b + (i + u * nth) * PER, pol_s);
-      add(wa, wb);
+        for (int u = 0; u < U; u++)
+          wa[u].u = ptx::ld_stream16(a + (i + u * nth) * PER, pol_s);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          wb[u].u = ptx::ld_stream16(b + (i + u * nth) * PER, pol_s);
+        add(wa, wb);
+      }
     }
     if (i < nv) { // the last trip: places past the end count as 0
-      W wa[kDotUnroll], wb[kDotUnroll];
+      W wa[U], wb[U];
 #pragma unroll
-      for (int u = 0; u < kDotUnroll; u++) {
+      for (int u = 0; u < U; u++) {
         const int64_t at = i + u * nth < nv ? i + u * nth : i;
         wa[u].u = ptx::ld_stream16(a + at * PER, pol_s);
         wb[u].u = ptx::ld_stream16(b + at * PER, pol_s);
       }
 #pragma unroll
-      for (int u = 1; u < kDotUnroll; u++)
+      for (int u = 1; u < U; u++)
         if (i + u * nth >= nv)
           wa[u].u = wb[u].u = make_uint4(0, 0, 0, 0);
       add(wa, wb);
@@ -363,7 +375,7 @@ __global__ void __launch_bounds__(kDotNT)
 __global__ void __launch_bounds__(kDotNT)
     dot_finish(const double *partials, int count, double *out) {
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(partials);
   const double t = dot_partials_sum(partials, count);
   if (threadIdx.x == 0)
     *out = t;

@@ -365,9 +365,17 @@ struct drb_csr_matrix : public drb::Csr {};
 namespace drb::ptx {
 
 // Waits until the grids this launch depends on have completed (returns at once
-// for a launch without the programmatic attribute).
-__device__ __forceinline__ void grid_dependency_wait() {
+// for a launch without the programmatic attribute).  The kernel names the
+// const __restrict__ pointers to what those grids may still be writing: a pointer
+// that comes out of the (empty) second asm cannot be used above it, so neither can
+// a load through it.  Their loads are not .nc either: that memory is not
+// read-only while the kernel is resident.  A handle's own arrays (matrix,
+// items, plan) need neither: the kernels that write them never let a dependent
+// start early, so they end before any later launch begins.
+template <class... P> __device__ __forceinline__ void grid_dependency_wait(P &...p) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  auto after = [](auto &q) { asm volatile("" : "+l"(q) : : "memory"); };
+  (after(p), ...);
 }
 // Lets the next kernel of the stream start (it waits for this one's results).
 __device__ __forceinline__ void grid_dependents_start() {
@@ -398,8 +406,17 @@ __device__ __forceinline__ uint64_t policy_keep(float share) {
   return p;
 }
 
-// 16-byte streaming load through the non-coherent path, not allocated in L1.
+// 16-byte streaming loads, not allocated in L1: of a caller's array, and (read-only
+// path) of an array that the handle owns.
 __device__ __forceinline__ uint4 ld_stream16(const void *ptr, uint64_t pol) {
+  uint4 r;
+  asm("ld.global.L1::no_allocate.L2::cache_hint.v4.u32 "
+               "{%0,%1,%2,%3}, [%4], %5;"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(ptr), "l"(pol));
+  return r;
+}
+__device__ __forceinline__ uint4 ld_matrix16(const void *ptr, uint64_t pol) {
   uint4 r;
   asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 "
                "{%0,%1,%2,%3}, [%4], %5;"
@@ -420,14 +437,14 @@ __device__ __forceinline__ void st_hint(double *ptr, double v, uint64_t pol) {
 
 __device__ __forceinline__ float ld_keep(const float *ptr, uint64_t pol) {
   float r;
-  asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;"
+  asm("ld.global.L2::cache_hint.f32 %0, [%1], %2;"
                : "=f"(r)
                : "l"(ptr), "l"(pol));
   return r;
 }
 __device__ __forceinline__ double ld_keep(const double *ptr, uint64_t pol) {
   double r;
-  asm("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;"
+  asm("ld.global.L2::cache_hint.f64 %0, [%1], %2;"
                : "=d"(r)
                : "l"(ptr), "l"(pol));
   return r;
@@ -435,7 +452,7 @@ __device__ __forceinline__ double ld_keep(const double *ptr, uint64_t pol) {
 __device__ __forceinline__ float ld_keep(const __nv_bfloat16 *ptr,
                                          uint64_t pol) {
   unsigned short r;
-  asm("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;"
+  asm("ld.global.L2::cache_hint.u16 %0, [%1], %2;"
                : "=h"(r)
                : "l"(ptr), "l"(pol));
   return __uint_as_float(((unsigned)r) << 16);

@@ -29,7 +29,9 @@ namespace {
 
 constexpr int kRedNT = 256;
 constexpr int kRedGrid = 592; // fixed: the grouping must not depend on the GPU
-constexpr int kRedUnroll = 4; // 16-byte loads in flight per thread
+// 16-byte loads in flight per thread (8-byte types, 3 / 4: a sum of 240 MB 37.8 / 39.2
+// us, f32 42.3 / 38.2)
+template <class T> constexpr int kRedUnroll = sizeof(T) == 8 ? 3 : 4;
 
 template <class T> struct SumAcc { using type = T; };
 template <> struct SumAcc<float> { using type = double; };
@@ -107,9 +109,9 @@ __global__ void __launch_bounds__(kRedNT)
                   typename ROp<T, OP>::A *partials, T *out) {
   using R = ROp<T, OP>;
   using A = typename R::A;
-  constexpr int PER = 16 / sizeof(T);
+  constexpr int PER = 16 / sizeof(T), U = kRedUnroll<T>;
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(x);
   const uint64_t pol = ptx::policy_evict_first();
   A acc = R::id();
   const int64_t tid = (int64_t)blockIdx.x * kRedNT + threadIdx.x;
@@ -126,24 +128,24 @@ __global__ void __launch_bounds__(kRedNT)
       T t[PER];
     };
     int64_t i = tid;
-    for (; i + (kRedUnroll - 1) * nth < nv; i += kRedUnroll * nth) {
-      W w[kRedUnroll];
+    for (; i + (U - 1) * nth < nv; i += U * nth) {
+      W w[U];
 #pragma unroll
-      for (int u = 0; u < kRedUnroll; u++)
+      for (int u = 0; u < U; u++)
         w[u].u = ptx::ld_stream16(xa + (i + u * nth) * PER, pol);
 #pragma unroll
-      for (int u = 0; u < kRedUnroll; u++)
+      for (int u = 0; u < U; u++)
 #pragma unroll
         for (int q = 0; q < PER; q++)
           acc = R::f(acc, R::lift(w[u].t[q]));
     }
     if (i < nv) { // the last trip: places past the end read the first one again
-      W w[kRedUnroll];
+      W w[U];
 #pragma unroll
-      for (int u = 0; u < kRedUnroll; u++)
+      for (int u = 0; u < U; u++)
         w[u].u = ptx::ld_stream16(xa + (i + u * nth < nv ? i + u * nth : i) * PER, pol);
 #pragma unroll
-      for (int u = 0; u < kRedUnroll; u++)
+      for (int u = 0; u < U; u++)
 #pragma unroll
         for (int q = 0; q < PER; q++)
           acc = R::f(acc, i + u * nth < nv ? R::lift(w[u].t[q]) : R::id());
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(kRedNT)
                   T *out) {
   using R = ROp<T, OP>;
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(partials);
   typename R::A s = R::id();
   for (int i = threadIdx.x; i < count; i += kRedNT)
     s = R::f(s, __ldcg(&partials[i]));

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kSellNT)
   __shared__ double s_red[kSellWarps];
   __shared__ int s_last;
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(x);
   if (RESID && ra.stop && *static_cast<const volatile int *>(ra.stop))
     return; // uniform: every CTA reads the same word, written by an earlier launch
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

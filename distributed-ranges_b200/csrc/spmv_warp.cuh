@@ -83,7 +83,7 @@ __device__ __forceinline__ void ld_group(const T *p, T (&out)[G], uint64_t pol) 
 #pragma unroll
   for (int v = 0; v < G / PER; v++) {
     Vec16<T> r;
-    r.u = ptx::ld_stream16(p + v * PER, pol);
+    r.u = ptx::ld_matrix16(p + v * PER, pol);
 #pragma unroll
     for (int i = 0; i < PER; i++)
       out[v * PER + i] = r.t[i];
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ int s_rp[kWarps][kRows + 1];
 
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(x);
   if (RESID && ra.stop && *static_cast<const volatile int *>(ra.stop))
     return; // uniform: every CTA reads the same word, written by an earlier launch
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(kThreads, TILE == 128 ? 4 : 2)
   __shared__ __align__(16) Acc s_prod[kWarps][TILE + TILE / 32];
   __shared__ int s_rp[kWarps][kRows + 1];
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(x);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Kt K{rowptr, colind, vals, x, y, items, nitems, chunks, partials, counters,
        ptx::policy_evict_first(), ptx::policy_evict_last(),
@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(kThreads, TILE == 128 ? 4 : 2)
 // and one dependent load per chunk made it the finishing pass's critical
 // path.
 template <class Acc, bool COMP>
-__device__ __forceinline__ Acc chunk_row_sum(const Acc *__restrict__ pp, int count) {
+__device__ __forceinline__ Acc chunk_row_sum(const Acc *pp, int count) {
   constexpr int kBatch = 16;
   CSum<Acc> sum;
   int i = 0;
@@ -643,7 +643,7 @@ template <class Acc, bool COMP>
 __global__ void chunk_finish(const int4 *__restrict__ splits, int64_t s0, int64_t s1,
                              const Acc *__restrict__ partials, Acc *__restrict__ y) {
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(partials);
   const int64_t nth = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = s0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < s1; i += nth) {
     const int4 sp = splits[i];
@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(kThreads)
   __shared__ double s_red[kWarps];
   __shared__ int s_last;
   ptx::grid_dependents_start();
-  ptx::grid_dependency_wait();
+  ptx::grid_dependency_wait(cpart);
   if (ra.stop && *static_cast<const volatile int *>(ra.stop))
     return;
   const Acc *bvec = static_cast<const Acc *>(ra.b);
