@@ -44,6 +44,10 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
 // had finished one.  8192^2 f32 54.9 -> 45.2 us = 0.92 of the measured HBM
 // rate, f64 90.9 -> 86, 4001^2 f32, whose rows are not aligned, 73 -> 30; four times
 // as many CTAs' worth of rows hide that: 24000^2 f32 353 -> 356, 32768^2 622 -> 642.)
+// A lane sums a step's products (16 to 32) by themselves and adds the steps'
+// sums: one chain over its share of a row grew the error with the row (N(0, 1)
+// rows of 16384 columns, 2-norm over the result's: f32 2.6e-7, f64 4.9e-16, now
+// 1.3e-7 and 2.6e-16).
 // U pieces per lane and step: 8, but 4 for f32 rows under 32 KB, whose last step would
 // be mostly empty (us, U = 4 / 8: 20000 x 500 9.8 / 10.8, 4096^2 14.9 / 15.5;
 // 8192^2 46.3 / 45.6, 24000^2 367 / 361, 8192 x 65536 335 / 328, 32768^2 658 / 648), and 16
@@ -102,6 +106,7 @@ __global__ void __launch_bounds__(kDenseNT, 4)
   for (int64_t s = me.s0; s < me.s1; s++) {
     const V *Ar = A + row * lda;
     const int64_t g0 = q * (32 * U) + lane;
+    V part = 0; // this step's products
     if constexpr (VEC) {
       union G16 {
         uint4 u;
@@ -118,7 +123,7 @@ __global__ void __launch_bounds__(kDenseNT, 4)
           xv.u = reinterpret_cast<const uint4 *>(x)[g0 + 32 * i];
 #pragma unroll
           for (int e = 0; e < PER; e++)
-            acc += a[i].t[e] * xv.t[e];
+            part += a[i].t[e] * xv.t[e];
         }
       } else {
 #pragma unroll
@@ -134,11 +139,11 @@ __global__ void __launch_bounds__(kDenseNT, 4)
             xv.u = reinterpret_cast<const uint4 *>(x)[g0 + 32 * i];
 #pragma unroll
             for (int e = 0; e < PER; e++)
-              acc += a[i].t[e] * xv.t[e];
+              part += a[i].t[e] * xv.t[e];
           }
       }
       if (q + 1 == spr && ng * PER + lane < n) // the elements after the last piece
-        acc += Ar[ng * PER + lane] * x[ng * PER + lane];
+        part += Ar[ng * PER + lane] * x[ng * PER + lane];
     } else {
       V a[U];
 #pragma unroll
@@ -147,8 +152,9 @@ __global__ void __launch_bounds__(kDenseNT, 4)
 #pragma unroll
       for (int i = 0; i < U; i++)
         if (g0 + 32 * i < ng)
-          acc += a[i] * x[g0 + 32 * i];
+          part += a[i] * x[g0 + 32 * i];
     }
+    acc += part;
     q++;
     if (q == spr || s + 1 == me.s1) {
       const V t = warp_sum_d(acc);

@@ -72,6 +72,27 @@ def test_one_rhs(mp, dtype, m, n, lda):
     check(mp, dtype, m, n, 1, lda, 0)
 
 
+@pytest.mark.parametrize("dtype,m,n", [
+    (torch.float32, 4800, 131_072), (torch.float32, 700, 40_001),  # whole rows per CTA
+    (torch.float32, 5, 1_000_003)])
+def test_one_rhs_sums_do_not_drift(mp, dtype, m, n):
+    """Equal products: the additions of one long chain round the same way while
+    the sum is in one binade, so a chain's length shows (0.7 in f32, relative:
+    4e-5 after 4096 terms, 1.6e-4 after 15600)."""
+    A = torch.full((m, n), 0.7, dtype=dtype, device="cuda")
+    x = torch.ones(n, dtype=dtype, device="cuda")
+    y = torch.empty(m, dtype=dtype, device="cuda")
+    mp.dense_gemv(A, x, y, 1, 0)
+    u = 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -53
+    exact = n * float(A[0, 0])
+    # The additions a product passes through: its step's 32, its warp's steps (of 512
+    # elements or more; whole rows, or an equal share for two CTAs per SM), a
+    # tree of 5, the CTA's 8 warps, a lane's share of 592 CTAs and a tree of 5.
+    share = n if m >= 592 else m * n / (2 * 148 * 8) + 512
+    bound = (32 + share / 512 + 2 + 5 + 8 + 19 + 5) * u * exact
+    assert np.all(np.abs(y.double().cpu().numpy() - exact) <= bound)
+
+
 def test_nan_stays_in_its_row_and_column(mp):
     A = torch.randn(70, 200, device="cuda")
     x = torch.randn(3 * 200, device="cuda")
