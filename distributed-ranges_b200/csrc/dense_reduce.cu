@@ -34,16 +34,13 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
 // or x do not start on 16 bytes), 2 KB to 8 KB of a row, so a warp reads long
 // contiguous runs (page locality decides: one row per warp with 2 KB steps
 // streams at 6.9 TB/s on 32768^2 f32, four rows of 512 bytes at 4.9).
-// Warps take equal consecutive shares of the steps; a row that falls to one
-// warp goes straight to y, the pieces of a row cut between warps to frag
-// (slot 0: the piece does not start its row; slot 1: it does), added in step
-// order.  With LOCAL a CTA owns whole rows, its warps share them, and the
-// pieces meet in shared memory; else the steps are shared over the whole grid
-// and dense_row_join adds the pieces.  (Whole 32 KB row slabs per warp, the
-// earlier unit, left 8192 rows on 7104 warps: some did two while the others
-// had finished one.  8192^2 f32 54.9 -> 45.2 us = 0.92 of the measured HBM
-// rate, f64 90.9 -> 86, 4001^2 f32, whose rows are not aligned, 73 -> 30; four times
-// as many CTAs' worth of rows hide that: 24000^2 f32 353 -> 356, 32768^2 622 -> 642.)
+// CTAs take equal consecutive shares of the steps (LOCAL: of the rows), their
+// warps equal shares of those.  A row that falls to one warp goes straight to y,
+// the parts of a row cut between warps meet in shared memory in step order, and
+// the parts of a row cut between CTAs go to frag (slot 0: the part does not start
+// its row; slot 1: it does), which dense_row_join adds, a warp per row.  (Whole
+// 32 KB row slabs per warp, the earlier unit, left 8192 rows on 7104 warps: some
+// did two while the others had finished one.)
 // A lane sums a step's products (16 to 32) by themselves and adds the steps'
 // sums: one chain over its share of a row grew the error with the row (N(0, 1)
 // rows of 16384 columns, 2-norm over the result's: f32 2.6e-7, f64 4.9e-16, now
@@ -53,33 +50,13 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
 // 8192^2 46.3 / 45.6, 24000^2 367 / 361, 8192 x 65536 335 / 328, 32768^2 658 / 648), and 16
 // single elements.
 constexpr int64_t kLongRowBytes = 32768;
+constexpr int64_t kUneven = 48 * 1024;
 
-struct RowShare { // the steps [s0, s1) of warp w of W over `steps`, from `base`
+struct RowShare { // the steps [s0, s1) of share w of W over `steps`, from `base`
   int64_t s0, s1;
   __device__ RowShare(int64_t base, int64_t steps, int64_t w, int64_t W)
       : s0(base + steps * w / W), s1(base + steps * (w + 1) / W) {}
 };
-
-// The row that warp w started and did not finish: its pieces in step order.
-template <class V>
-__device__ __forceinline__ void join_cut_row(int64_t base, int64_t steps, int64_t spr, int64_t w,
-                                             int64_t W, const V *frag, V *y) {
-  const RowShare me(base, steps, w, W);
-  const int64_t row = me.s1 / spr;
-  if (me.s1 % spr == 0 || row * spr < me.s0)
-    return;
-  V s = frag[2 * w + 1];
-  for (int64_t v = w + 1;; v++) {
-    const RowShare o(base, steps, v, W);
-    if (o.s0 >= (row + 1) * spr)
-      break;
-    if (o.s1 > o.s0)
-      s += frag[2 * v];
-    if (v + 1 == W)
-      break;
-  }
-  y[row] = s;
-}
 
 template <class V, bool VEC, bool LOCAL, int U>
 __global__ void __launch_bounds__(kDenseNT, 4)
@@ -92,16 +69,13 @@ __global__ void __launch_bounds__(kDenseNT, 4)
   ptx::grid_dependency_wait(A, x);
   const uint64_t pol_s = ptx::policy_evict_first();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t r0 = LOCAL ? m * blockIdx.x / gridDim.x : 0;
-  const int64_t r1 = LOCAL ? m * (blockIdx.x + 1) / gridDim.x : m;
-  const int64_t base = r0 * spr, steps = (r1 - r0) * spr;
-  const int64_t w = LOCAL ? warp : (int64_t)blockIdx.x * NW + warp;
-  const int64_t W = LOCAL ? NW : (int64_t)gridDim.x * NW;
-  const RowShare me(base, steps, w, W);
-  V *fr = LOCAL ? s_frag : frag;
+  const RowShare cta = LOCAL ? RowShare(0, m, blockIdx.x, gridDim.x)
+                             : RowShare(0, m * spr, blockIdx.x, gridDim.x);
+  const int64_t c0 = LOCAL ? cta.s0 * spr : cta.s0, c1 = LOCAL ? cta.s1 * spr : cta.s1;
+  const RowShare me(c0, c1 - c0, warp, NW);
   const int64_t ng = n / PER; // whole pieces of a row
   int64_t row = me.s0 / spr, q = me.s0 - row * spr;
-  bool inside = q != 0; // the current piece does not start its row
+  bool inside = q != 0; // the current part does not start its row
   V acc = 0;
   for (int64_t s = me.s0; s < me.s1; s++) {
     const V *Ar = A + row * lda;
@@ -162,7 +136,7 @@ __global__ void __launch_bounds__(kDenseNT, 4)
         if (q == spr && !inside)
           y[row] = t;
         else
-          fr[2 * w + (inside ? 0 : 1)] = t;
+          s_frag[2 * warp + (inside ? 0 : 1)] = t;
       }
       acc = 0;
       row++;
@@ -170,20 +144,55 @@ __global__ void __launch_bounds__(kDenseNT, 4)
       inside = false;
     }
   }
-  if (LOCAL) {
-    __syncthreads();
-    if (threadIdx.x < NW)
-      join_cut_row<V>(base, steps, spr, threadIdx.x, NW, s_frag, y);
+  __syncthreads();
+  if (threadIdx.x >= NW)
+    return;
+  // what the CTA's warps have of the row up to step `end`, from warp v on
+  auto rest = [&](int v, int64_t end, V sum) {
+    for (; v < NW; v++) {
+      const RowShare o(c0, c1 - c0, v, NW);
+      if (o.s0 >= end)
+        break;
+      if (o.s1 > o.s0)
+        sum += s_frag[2 * v];
+    }
+    return sum;
+  };
+  const RowShare mine(c0, c1 - c0, threadIdx.x, NW);
+  const int64_t cut = mine.s1 / spr; // the row that this warp started and did not finish
+  if (mine.s1 % spr != 0 && cut * spr >= mine.s0) {
+    const V sum = rest(threadIdx.x + 1, (cut + 1) * spr, s_frag[2 * threadIdx.x + 1]);
+    if (LOCAL || (cut + 1) * spr <= c1)
+      y[cut] = sum;
+    else
+      frag[2 * blockIdx.x + 1] = sum;
   }
+  if (!LOCAL && threadIdx.x == 0 && c0 % spr != 0) // the row that an earlier CTA started
+    frag[2 * blockIdx.x] = rest(0, (c0 / spr + 1) * spr, V(0));
 }
 
+// The rows cut between the G CTAs: a warp per CTA that started one and did not
+// finish it adds its part and the later CTAs'.
 template <class V>
-__global__ void dense_row_join(int64_t steps, int64_t spr, int64_t W, const V *frag, V *y) {
+__global__ void __launch_bounds__(kDenseNT)
+    dense_row_join(int64_t steps, int64_t spr, int64_t G, const V *frag, V *y) {
   ptx::grid_dependents_start();
   ptx::grid_dependency_wait(frag);
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w < W)
-    join_cut_row<V>(0, steps, spr, w, W, frag, y);
+  const int lane = threadIdx.x & 31;
+  const int64_t b = ((int64_t)blockIdx.x * kDenseNT + threadIdx.x) >> 5;
+  if (b >= G)
+    return;
+  const RowShare me(0, steps, b, G);
+  const int64_t row = me.s1 / spr;
+  if (me.s1 % spr == 0 || row * spr < me.s0)
+    return;
+  const int64_t last = ((row + 1) * spr * G - 1) / steps; // the CTA of the row's last step
+  V s = 0;
+  for (int64_t v = b + 1 + lane; v <= last; v += 32)
+    s += frag[2 * v];
+  s = warp_sum_d(s);
+  if (lane == 0)
+    y[row] = frag[2 * b + 1] + s;
 }
 
 template <class V, bool VEC, int U>
@@ -205,27 +214,29 @@ drb_status dense_row_call(int64_t m, int64_t n, const V *A, int64_t lda, const V
   const int64_t spr = std::max<int64_t>(1, (n / PER + STEP - 1) / STEP);
   const int64_t steps = m * spr;
   constexpr int NW = kDenseNT / 32;
-  // Whole rows per CTA, unless there are so few of them per CTA (under 4) that
-  // the rounding idles warps for longer than the second launch takes (A over
-  // 16 MB).
-  const bool local = m >= 4 * (int64_t)full || m * n * (int64_t)sizeof(V) < ((int64_t)16 << 20);
+  const int64_t gl = std::min<int64_t>(full, m), gs = std::min<int64_t>(full, (steps + NW - 1) / NW);
+  // Whole rows per CTA, unless the CTA with the most rows then reads more than
+  // kUneven bytes above an equal share: that takes longer than the second launch
+  // and its scratch do.  (us, whole rows / shared steps, f32: 1 row of 0.25 MB
+  // 7.4 / 4.5, of 4 MB 184 / 6.1; 4 rows of 64 KB 3.6 / 4.7; 32 rows, 2 MB 5.9 / 5.8,
+  // 4 MB 9.2 / 6.0; 100 rows, 8 MB 7.7 / 6.3; 148 rows, 8 MB 6.2 / 6.4; 592 rows,
+  // 16 MB 6.0 / 7.8.  The slab kernel that came before: 1 row of 4 MB 22.)
+  const int64_t row_bytes = n * (int64_t)sizeof(V);
+  const bool local = (m + gl - 1) / gl * row_bytes - m * row_bytes / full <= kUneven;
   cudaError_t e;
   if (local) {
-    const unsigned g = (unsigned)std::min<int64_t>(full, m);
-    e = launch_overlapped(dense_row_kernel<V, VEC, true, U>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
-                          lda, x, y, spr, (V *)nullptr);
+    e = launch_overlapped(dense_row_kernel<V, VEC, true, U>, dim3((unsigned)gl), dim3(kDenseNT), 0,
+                          s, m, n, A, lda, x, y, spr, (V *)nullptr);
     note_launch();
   } else {
-    const unsigned g = (unsigned)std::min<int64_t>(full, (steps + NW - 1) / NW);
-    const int64_t W = (int64_t)g * NW;
     V *frag = nullptr;
-    DRB_TRY(scratch_alloc(reinterpret_cast<void **>(&frag), sizeof(V) * 2 * (size_t)W, s));
-    e = launch_overlapped(dense_row_kernel<V, VEC, false, U>, dim3(g), dim3(kDenseNT), 0, s, m, n, A,
-                          lda, x, y, spr, frag);
+    DRB_TRY(scratch_alloc(reinterpret_cast<void **>(&frag), sizeof(V) * 2 * (size_t)gs, s));
+    e = launch_overlapped(dense_row_kernel<V, VEC, false, U>, dim3((unsigned)gs), dim3(kDenseNT),
+                          0, s, m, n, A, lda, x, y, spr, frag);
     note_launch();
     if (e == cudaSuccess) {
-      e = launch_overlapped(dense_row_join<V>, dim3((unsigned)((W + 255) / 256)), dim3(256), 0, s,
-                            steps, spr, W, (const V *)frag, y);
+      e = launch_overlapped(dense_row_join<V>, dim3((unsigned)((gs + NW - 1) / NW)),
+                            dim3(kDenseNT), 0, s, steps, spr, gs, (const V *)frag, y);
       note_launch();
     }
     scratch_free(frag, s);

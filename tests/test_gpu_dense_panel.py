@@ -74,7 +74,8 @@ def test_one_rhs(mp, dtype, m, n, lda):
 
 @pytest.mark.parametrize("dtype,m,n", [
     (torch.float32, 4800, 131_072), (torch.float32, 700, 40_001),  # whole rows per CTA
-    (torch.float32, 5, 1_000_003)])
+    (torch.float32, 1, 4_000_000), (torch.float32, 3, 1 << 20), (torch.float32, 2, 700_003),
+    (torch.float32, 1, 40_000_000), (torch.float64, 1, 4_000_000), (torch.float64, 3, 700_003)])
 def test_one_rhs_sums_do_not_drift(mp, dtype, m, n):
     """Equal products: the additions of one long chain round the same way while
     the sum is in one binade, so a chain's length shows (0.7 in f32, relative:
