@@ -45,12 +45,18 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
 // sums: one chain over its share of a row grew the error with the row (N(0, 1)
 // rows of 16384 columns, 2-norm over the result's: f32 2.6e-7, f64 4.9e-16, now
 // 1.3e-7 and 2.6e-16).
-// U pieces per lane and step: 8, but 4 for f32 rows under 32 KB, whose last step would
-// be mostly empty (us, U = 4 / 8: 20000 x 500 9.8 / 10.8, 4096^2 14.9 / 15.5;
-// 8192^2 46.3 / 45.6, 24000^2 367 / 361, 8192 x 65536 335 / 328, 32768^2 658 / 648), and 16
-// single elements.
-constexpr int64_t kLongRowBytes = 32768;
+// U pieces per lane and step: 8, but 4 for f32 rows under 32 KB and f64 rows under 4
+// KB, whose last step would be mostly empty (us, U = 4 / 8: f32 20000 x 500 9.8 /
+// 10.8, 4096^2 14.9 / 15.5, 8192^2 46.3 / 45.6, 24000^2 367 / 361, 32768^2 658 / 648;
+// f64 10000 x 500 10.0 / 10.8, 16384 x 128 5.7 / 7.6), and 16 single elements.
+template <class V> constexpr int64_t kLongRowBytes = sizeof(V) == 4 ? 32768 : 4096;
 constexpr int64_t kUneven = 48 * 1024;
+// CTAs per SM: as many as leave the registers for a step's loads to go out at once.
+// Rows of 16-byte pieces, us, 4 / 3 / 2: f32 8192^2 45.0 / 43.1 / 41.9 (0.99 of the
+// measured HBM rate; the slab kernel 53.5), 32768^2 656 / 617 / 604 (slabs 626), f64
+// 8192^2 91.3 / 84.4 / 81.9, 20000^2 509 / 476 / 460.  Single elements: f32 4001^2 15.8
+// / 16.3 with 4 / 3 CTAs, f64 5003 x 3001 23.9 / 22.4.
+template <class V, bool VEC> constexpr int kRowCtas = VEC ? 2 : sizeof(V) == 4 ? 4 : 3;
 
 struct RowShare { // the steps [s0, s1) of share w of W over `steps`, from `base`
   int64_t s0, s1;
@@ -59,7 +65,7 @@ struct RowShare { // the steps [s0, s1) of share w of W over `steps`, from `base
 };
 
 template <class V, bool VEC, bool LOCAL, int U>
-__global__ void __launch_bounds__(kDenseNT, 4)
+__global__ void __launch_bounds__(kDenseNT, kRowCtas<V, VEC>)
     dense_row_kernel(int64_t m, int64_t n, const V *__restrict__ A, int64_t lda,
                      const V *__restrict__ x, V *__restrict__ y, int64_t spr, V *frag) {
   constexpr int PER = VEC ? 16 / (int)sizeof(V) : 1;
@@ -255,9 +261,8 @@ drb_status dense_row(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, 
                    reinterpret_cast<uintptr_t>(x) % 16 == 0 && lda * sizeof(V) % 16 == 0;
   if (!vec)
     return dense_row_call<V, false, 16>(m, n, A, lda, x, y, s);
-  if constexpr (sizeof(V) == 4)
-    if (n * (int64_t)sizeof(V) < kLongRowBytes)
-      return dense_row_call<V, true, 4>(m, n, A, lda, x, y, s);
+  if (n * (int64_t)sizeof(V) < kLongRowBytes<V>)
+    return dense_row_call<V, true, 4>(m, n, A, lda, x, y, s);
   return dense_row_call<V, true, 8>(m, n, A, lda, x, y, s);
 }
 
