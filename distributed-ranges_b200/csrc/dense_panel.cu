@@ -9,9 +9,9 @@
 // ceil(k / 8) passes over HBM, and rows that do not start on 16 bytes went
 // through single-element loads with few of them in flight.
 //
-// Measured (us): 5003 x 3001 f64 with 20 right-hand sides 246 -> 48, f32 429 -> 38;
-// 8192^2 f32 with 20 334 -> 94, with 8 136 -> 58, with 4 61 -> 51; 4096 x 8192
-// f64 with 32 429 -> 100.  (One CTA of 16 warps per SM with tiles twice as high
+// Measured (us), a gemv repeated over column blocks -> here: 5003 x 3001 f64 with 20
+// right-hand sides 253 -> 50, f32 445 -> 38; 8192^2 f32 with 20 342 -> 102, with 8
+// 138 -> 61, with 4 63 -> 53; 4096 x 8192 f64 with 32 437 -> 106.  (One CTA of 16 warps per SM with tiles twice as high
 // ran the f64 case in 57: all warps loaded, waited and multiplied in step.)
 //
 // Tiles and split.  A CTA of 8 warps owns a tile of BM rows and walks along the
@@ -101,6 +101,15 @@ struct PanelArgs {
 // Measured, us, short / long: 8192^2 f32 k = 20 105 / 94, 8191^2 k = 3 83 / 69,
 // 8191 x 4095 f64 k = 5 80 / 70; 16000 x 300 f32 k = 12 9.9 / 11.1, 5003 x 3001
 // f64 k = 20 49.7 / 51.3.
+// FOLD chunks: a sum runs over 32 products (a lane's in f32, a warp's mma chain in
+// f64) before it joins the tile's, since one chain over a whole tile grew its error
+// with the row: N(0, 1) entries, 2-norm over the result's, blocks of columns before /
+// one chain / folded: 16384 x 4096, k = 20, f32 2.1e-7 / 2.4e-7 / 1.3e-7, k = 32 2.1e-7 /
+// 2.7e-7 / 1.3e-7, f64 3.0e-16 / 1.2e-15 / 3.0e-16; 16384 x 1024 f32 1.20e-7 / 1.30e-7 /
+// 1.14e-7, f64 2.2e-16 / 6.0e-16 / 2.4e-16.  (Under 512 columns the shorter trees
+// leave it 1.13 times the old one in f32, 1.45 in f64, whose chains of 16 would be
+// 1.2.)  It costs, us: 5003 x 3001 k = 20 f64 48.2 -> 49.8, f32 37.3 -> 37.5; 8192^2 k = 20
+// f32 92.6 -> 101.7, f64 122 -> 138; 8192 x 4096 k = 32 f32 78.7 -> 82.1, f64 93.3 -> 100.1.
 // f64 keeps three short chunks per CTA in the ring, with more than 24 right-hand
 // sides two (three / two, us: 8192 x 4096 k = 20 66 / 71, k = 32 100 / 95; 8192 x 1024
 // k = 32 38 / 33, 5003 x 3001 k = 32 58 / 57).  Three CTAs of two chunks (8192 x 4096
@@ -110,7 +119,7 @@ template <int C, bool SH, bool LONG>
 struct Shape<float, C, SH, LONG> { // C right-hand sides
   static constexpr int R = C <= 20 ? 8 : 4;
   static constexpr int BM = kWarps * R, KC = LONG ? 128 : 64, AS = KC + 4, XS = KC + 16, CP = C;
-  static constexpr int STAGES = LONG ? 2 : 4, MERGE = 0;
+  static constexpr int STAGES = LONG ? 2 : 4, MERGE = 0, FOLD = 32 * 16 / KC;
 };
 template <int NT, bool SH, bool LONG>
 struct Shape<double, NT, SH, LONG> { // 8 NT right-hand sides
@@ -118,6 +127,7 @@ struct Shape<double, NT, SH, LONG> { // 8 NT right-hand sides
   static constexpr int BM = kWarps / 2 * R, KC = LONG ? 64 : 32, AS = KC + (SH ? 4 : 8), XS = AS;
   static constexpr int CP = 8 * NT, STAGES = LONG || NT == 4 ? 2 : 3;
   static constexpr int MERGE = BM * CP; // the second half's sums of a tile
+  static constexpr int FOLD = LONG ? 1 : 2;
 };
 template <class V, int P> constexpr bool may_be_long() { return sizeof(V) == 4 || P <= 2; }
 template <class V, int P, bool SH, bool LONG> constexpr size_t panel_smem() {
@@ -266,8 +276,8 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
   // this thread's sums of the current tile
   constexpr int R = S::R;
   constexpr int NACC = sizeof(V) == 4 ? R * CP / 2 : 2 * (CP / 8);
-  float accf[sizeof(V) == 4 ? NACC : 1];
-  double accd[sizeof(V) == 8 ? NACC : 1][2];
+  float accf[sizeof(V) == 4 ? NACC : 1], sumf[sizeof(V) == 4 ? NACC / 16 : 1];
+  double accd[sizeof(V) == 8 ? NACC : 1][2], sumd[sizeof(V) == 8 ? NACC : 1][2];
   auto clear = [&]() {
     if constexpr (sizeof(V) == 4) {
 #pragma unroll
@@ -279,7 +289,47 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
         accd[i][0] = accd[i][1] = 0.0;
     }
   };
-  auto compute = [&](int st) {
+  auto clear_sums = [&]() {
+    if constexpr (sizeof(V) == 4) {
+#pragma unroll
+      for (int i = 0; i < NACC / 16; i++)
+        sumf[i] = 0.0f;
+    } else {
+#pragma unroll
+      for (int i = 0; i < NACC; i++)
+        sumd[i][0] = sumd[i][1] = 0.0;
+    }
+  };
+  // The sums since the last fold join the tile's.  f32: the 16 lanes' sums
+  // meet in a halving tree, which leaves a sixteenth of them in each lane.
+  auto fold = [&]() {
+    if constexpr (sizeof(V) == 4) {
+      constexpr int N = NACC;
+      static_assert(N % 16 == 0, "the halving tree needs a multiple of 16 sums");
+      // each step a lane keeps one half of its sums and passes the other on
+#pragma unroll
+      for (int s = 0; s < 4; s++) {
+        const int off = 8 >> s, h = N >> (s + 1);
+        const bool up = lane & off;
+#pragma unroll
+        for (int i = 0; i < N / 2; i++)
+          if (i < h) {
+            const float keep = up ? accf[i + h] : accf[i], send = up ? accf[i] : accf[i + h];
+            accf[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < N / 16; i++)
+        sumf[i] += accf[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < NACC; i++) {
+        sumd[i][0] += accd[i][0];
+        sumd[i][1] += accd[i][1];
+      }
+    }
+  };
+  auto compute = [&](int st, bool fold_first) {
     const V *As = sa + (size_t)st * BM * AS + wr * AS;
     const V *Xs = sx + (size_t)st * CP * XS;
     if constexpr (sizeof(V) == 4) {
@@ -325,6 +375,10 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
           else
             bv[t] = *reinterpret_cast<const double2 *>(Xp + t * 8 * XS + c);
         }
+        if (c == 0 && fold_first) {
+          fold();
+          clear();
+        }
 #pragma unroll
         for (int i = 0; i < 2; i++)
 #pragma unroll
@@ -353,19 +407,6 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
     };
     if constexpr (sizeof(V) == 4) {
       constexpr int CH = CP / 2, N = R * CH;
-      static_assert(N % 16 == 0, "the halving tree needs a multiple of 16 sums");
-      // each step a lane keeps one half of its sums and passes the other on
-#pragma unroll
-      for (int s = 0; s < 4; s++) {
-        const int off = 8 >> s, h = N >> (s + 1);
-        const bool up = lane & off;
-#pragma unroll
-        for (int i = 0; i < N / 2; i++)
-          if (i < h) {
-            const float keep = up ? accf[i + h] : accf[i], send = up ? accf[i] : accf[i + h];
-            accf[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-          }
-      }
       int f0 = 0;
 #pragma unroll
       for (int s = 0; s < 4; s++)
@@ -373,7 +414,7 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
           f0 += N >> (s + 1);
 #pragma unroll
       for (int i = 0; i < N / 16; i++)
-        put(wr + (f0 + i) / CH, (lane >> 4) + 2 * ((f0 + i) % CH), accf[i]);
+        put(wr + (f0 + i) / CH, (lane >> 4) + 2 * ((f0 + i) % CH), sumf[i]);
     } else {
       // the second half's warps hand their sums over
       constexpr int NT = CP / 8;
@@ -387,7 +428,7 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
 #pragma unroll
           for (int t = 0; t < NT; t++)
             *reinterpret_cast<double2 *>(mine + at(i, t, 0)) =
-                make_double2(accd[i * NT + t][0], accd[i * NT + t][1]);
+                make_double2(sumd[i * NT + t][0], sumd[i * NT + t][1]);
       }
       __syncthreads();
       if (!kh) {
@@ -398,13 +439,17 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
 #pragma unroll
             for (int e = 0; e < 2; e++)
               put(wr + i * 8 + (lane >> 2), t * 8 + 2 * (lane & 3) + e,
-                  accd[i * NT + t][e] + mine[at(i, t, e)]);
+                  sumd[i * NT + t][e] + mine[at(i, t, e)]);
       }
     }
   };
 
   int64_t ct = c0 / cpt;                      // current tile
   int left = cpt - (int)(c0 - ct * cpt);      // chunks left in it
+  if (c1 - c0 < left)
+    left = (int)(c1 - c0); // (of this CTA's)
+  int run = min(left, S::FOLD); // chunks until the next fold
+  bool fold_next = false; // f64: fold in the next chunk, behind whose loads the adds hide
 #pragma unroll
   for (int s = 0; s < ST - 1; s++) {
     if (c0 + s < c1)
@@ -412,6 +457,7 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
     cp_commit();
   }
   clear();
+  clear_sums();
   int st = 0;
   for (int64_t q = c0; q < c1; q++) {
     cp_wait<ST - 2>();
@@ -420,12 +466,23 @@ __global__ void __launch_bounds__(kNT, kCtas) dense_panel(const PanelArgs a) {
     if (q + ST - 1 < c1)
       load(fill);
     cp_commit();
-    compute(st);
-    if (--left == 0 || q + 1 == c1) {
-      emit(ct);
-      clear();
-      left = cpt;
-      ct++;
+    compute(st, fold_next);
+    left--;
+    fold_next = false;
+    if (--run == 0) {
+      if (sizeof(V) == 4 || left == 0) {
+        fold();
+        clear();
+      } else {
+        fold_next = true;
+      }
+      if (left == 0) {
+        emit(ct);
+        clear_sums();
+        left = (int)min((int64_t)cpt, c1 - q - 1);
+        ct++;
+      }
+      run = min(left, S::FOLD);
     }
     st = st + 1 == ST ? 0 : st + 1;
   }

@@ -105,3 +105,22 @@ def test_nan_stays_in_its_row_and_column(mp):
     want[:, 5] = True
     want[1, :] = True
     assert torch.equal(bad, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("k", [3, 20, 32])
+def test_panel_sums_do_not_drift(mp, dtype, k):
+    """Equal products, as in test_one_rhs_sums_do_not_drift, in tiles that no
+    CTA boundary cuts (more tiles than CTAs)."""
+    m, n = 19_000, 16_384
+    A = torch.full((m, n), 0.7, dtype=dtype, device="cuda")
+    x = torch.ones(n * k, dtype=dtype, device="cuda")
+    y = torch.empty(m * k, dtype=dtype, device="cuda")
+    mp.dense_gemv(A, x, y, k, 0)
+    u = 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -53
+    exact = n * float(A[0, 0])
+    # The additions a product passes through: 32 until a fold (a lane's in f32, one of
+    # two warps' in f64), the folds of the row (512 columns each, or 64), a tree.
+    folds = n / 512 if dtype == torch.float32 else n / 64
+    bound = (32 + folds + 8) * u * exact
+    assert np.all(np.abs(y.double().cpu().numpy() - exact) <= bound)
