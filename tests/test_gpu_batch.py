@@ -146,6 +146,17 @@ def test_batch_f64(mp, k):
 
 
 @pytest.mark.parametrize("layout", [COL, ROW])
+@pytest.mark.parametrize("dtype,k,tol", [(np.float32, 28, 1e-5), (np.float32, 36, 1e-5),
+                                         (np.float64, 14, 1e-12), (np.float64, 20, 1e-12)])
+def test_batch_eight_gathers_in_flight(mp, dtype, k, tol, layout):
+    """Seven or more lanes per slot, not a power of two, rows of eight or more."""
+    mats_np = mixed_batch(dtype)
+    assert sum(m[4].size for m in mats_np) >= 8 * sum(m[0] for m in mats_np)
+    _, xs, ys, _ = run_batch(mp, mats_np, k, layout)
+    check_against_oracle(mats_np, xs, ys, k, layout, tol)
+
+
+@pytest.mark.parametrize("layout", [COL, ROW])
 @pytest.mark.parametrize("k", [1, 16, 33])
 def test_batch_bf16(mp, k, layout):
     mats_np = mixed_batch()

@@ -124,3 +124,16 @@ def test_panel_sums_do_not_drift(mp, dtype, k):
     folds = n / 512 if dtype == torch.float32 else n / 64
     bound = (32 + folds + 8) * u * exact
     assert np.all(np.abs(y.double().cpu().numpy() - exact) <= bound)
+
+
+@pytest.mark.parametrize("dtype,m,n,k,lda,layout", [
+    # long chunks (a ring of two): 16-byte rows and shifted ones, both layouts
+    (torch.float32, 4100, 4096, 3, 4096, 0), (torch.float32, 4100, 4099, 12, 4099, 1),
+    (torch.float32, 4100, 4099, 20, 4100, 0), (torch.float32, 2100, 4099, 25, 4101, 0),
+    (torch.float32, 2100, 4096, 32, 4104, 1), (torch.float64, 4097, 4095, 5, 4095, 0),
+    (torch.float64, 4097, 4096, 13, 4098, 1), (torch.float64, 4097, 4095, 16, 4097, 0),
+    # shares of many tiles, rounded up to whole tiles
+    (torch.float32, 310_001, 40, 3, 40, 0), (torch.float32, 155_003, 50, 30, 51, 1),
+    (torch.float64, 310_001, 30, 2, 31, 0)])
+def test_panel_long_chunks_and_many_tiles(mp, dtype, m, n, k, lda, layout):
+    check(mp, dtype, m, n, k, lda, layout)

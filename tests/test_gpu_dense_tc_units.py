@@ -58,3 +58,30 @@ def test_units(mp, shapes, k, layout, variant):
         # exact products; every accumulation step rounds (or truncates) once: 2^-23
         assert np.all(np.abs(got - ref) <= (n + 8) * 2.0 ** -23 * den)
     P.destroy()
+
+
+@pytest.mark.parametrize("shapes,k,layout", [
+    ([(100, 16000)], 200, COL), ([(513, 6001), (2, 9000)], 128, ROW), ([(300, 8192)], 3, COL),
+    ([(257, 5000)], 40, ROW), ([(129, 1023)], 32, COL), ([(128, 1088)], 32, COL)])
+def test_every_column_counts_once(mp, shapes, k, layout):
+    """Small integers: every sum is exact in FP32, so a column that a cut along K
+    drops or takes twice shows."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    As, xs, ys, want = [], [], [], []
+    for m, n in shapes:
+        lda = (n + 7) // 8 * 8
+        A = torch.randint(-8, 9, (m, lda), device="cuda", generator=g).bfloat16()
+        if lda > n:
+            A[:, n:] = float("nan")
+        X = torch.randint(-8, 9, (k, n), device="cuda", generator=g).bfloat16()
+        assert n * 64 < 2 ** 24
+        As.append(A[:, :n])
+        xs.append((X if layout == COL else X.t()).contiguous().view(-1))
+        ys.append(torch.full((m * k,), float("nan"), device="cuda"))
+        want.append((A[:, :n].double() @ X.double().t()).float())
+    P = mp.dense_batch(As, xs, ys, k, layout)
+    P.gemv()
+    P.check()
+    for (m, _), y, w in zip(shapes, ys, want):
+        assert torch.equal(y.view(m, k) if layout == ROW else y.view(k, m).t(), w)
+    P.destroy()
