@@ -437,29 +437,30 @@ template <class T> struct ResShape {
 };
 
 template <class T, int NT> drb_status res_shape(const Csr &A, ResShape<T> &S) {
-  static int limits[64][2]; // SMs, shared memory of a CTA (0: not read yet)
-  const int d = A.device < 64 ? A.device : 0;
-  if (limits[d][0] == 0 || A.device >= 64) {
-    int sms = 0, optin = 0;
-    DRB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, A.device));
+  static std::atomic<unsigned long long> allowed[64];
+  static std::atomic<int> dyn_of[64]; // shared memory that a CTA may have
+  std::atomic<int> &dyn = dyn_of[A.device < 64 ? A.device : 0];
+  int sms = 0;
+  DRB_TRY(device_sms(A.device, &sms));
+  DRB_TRY(once_per_context(allowed, A.device, [&]() -> drb_status {
+    int optin = 0;
     DRB_CUDA_TRY(
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, A.device));
     cudaFuncAttributes fa;
     DRB_CUDA_TRY(cudaFuncGetAttributes(&fa, cg_resident<T, NT>));
-    const int dyn = optin - (int)fa.sharedSizeBytes;
-    DRB_CUDA_TRY(cudaFuncSetAttribute(cg_resident<T, NT>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-    limits[d][1] = dyn;
-    limits[d][0] = sms;
-  }
+    dyn.store(optin - (int)fa.sharedSizeBytes);
+    DRB_CUDA_TRY(cudaFuncSetAttribute(
+        cg_resident<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn.load()));
+    return DRB_OK;
+  }));
   const int64_t ns = A.sell.nslices;
   S.kernel = reinterpret_cast<const void *>(cg_resident<T, NT>);
   S.threads = NT;
   S.grid = (int)std::max<int64_t>(
-      1, std::min<int64_t>(std::min(limits[d][0], kResMaxCtas), ns / kResMinSlices));
+      1, std::min<int64_t>(std::min(sms, kResMaxCtas), ns / kResMinSlices));
   S.cap = (int)((ns + S.grid - 1) / S.grid);
   const int64_t vec = 32 * (int64_t)S.cap * (int64_t)sizeof(T);
-  const int64_t room = limits[d][1] - 4 * ((int64_t)S.cap + 1);
+  const int64_t room = dyn.load() - 4 * ((int64_t)S.cap + 1);
   S.nres = (int)std::max<int64_t>(0, std::min<int64_t>(4, room / vec));
   S.smem = (size_t)(S.nres * vec + 4 * ((int64_t)S.cap + 1));
   return DRB_OK;

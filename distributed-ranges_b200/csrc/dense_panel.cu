@@ -551,15 +551,15 @@ template <class V, int P, bool SH, bool LONG>
 drb_status panel_run(PanelArgs a, cudaStream_t s) {
   using S = Shape<V, P, SH, LONG>;
   constexpr size_t smem = panel_smem<V, P, SH, LONG>();
-  static int sm_count[64] = {0}; // 0: this device has not run the kernel yet
-  int dev = 0;
+  static std::atomic<unsigned long long> allowed[64];
+  int dev = 0, sms = 0;
   DRB_CUDA_TRY(cudaGetDevice(&dev));
-  int &sms = sm_count[dev < 64 ? dev : 0];
-  if (sms == 0 || dev >= 64) {
+  DRB_TRY(device_sms(dev, &sms));
+  DRB_TRY(once_per_context(allowed, dev, [&]() -> drb_status {
     DRB_CUDA_TRY(cudaFuncSetAttribute(dense_panel<V, P, SH, LONG>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    DRB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  }
+    return DRB_OK;
+  }));
   const int64_t tiles = (a.m + S::BM - 1) / S::BM;
   a.cpt = (a.n + S::KC - 1) / S::KC;
   a.chunks = tiles * a.cpt;
@@ -585,7 +585,7 @@ drb_status panel_run(PanelArgs a, cudaStream_t s) {
     const bool many = a.cpt > 4 * a.share; // pieces of a tile
     const int out = many ? 32 : 256;
     const unsigned g = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(148 * 8, (a.m * a.k + out - 1) / out));
+        1, std::min<int64_t>(8 * (int64_t)sms, (a.m * a.k + out - 1) / out));
     e = many ? launch_overlapped(panel_sum<V, 8>, dim3(g), dim3(256), 0, s, a, S::BM, S::CP)
              : launch_overlapped(panel_sum<V, 1>, dim3(g), dim3(256), 0, s, a, S::BM, S::CP);
     note_launch();
@@ -606,9 +606,12 @@ template <class V, int P> drb_status panel_align(const PanelArgs &a, cudaStream_
                                         a.x_js * sizeof(V) % 16 == 0));
   if constexpr (may_be_long<V, P>()) {
     // at least kLongShare long chunks for every CTA of the GPU
+    int dev = 0, sms = 0;
+    DRB_CUDA_TRY(cudaGetDevice(&dev));
+    DRB_TRY(device_sms(dev, &sms));
     using S = Shape<V, P, false, true>;
     const int64_t chunks = (a.m + S::BM - 1) / S::BM * ((a.n + S::KC - 1) / S::KC);
-    if (a.n >= 8 * S::KC && chunks >= kLongShare * kCtas * 148)
+    if (a.n >= 8 * S::KC && chunks >= kLongShare * kCtas * sms)
       return aligned ? panel_run<V, P, false, true>(a, s) : panel_run<V, P, true, true>(a, s);
   }
   return aligned ? panel_run<V, P, false, false>(a, s) : panel_run<V, P, true, false>(a, s);

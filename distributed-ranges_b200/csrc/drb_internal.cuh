@@ -90,6 +90,26 @@ struct DeviceGuard {
 // Stream-ordered per-call scratch from a library-private pool that keeps its
 // memory mapped (util.cu); release with scratch_free on the same stream.
 drb_status scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+// Id of the calling thread's current context (unique for the life of the
+// process: a context created again, e.g. after cudaDeviceReset, gets a new
+// id), or 0 when none is current.  What the runtime keeps per context (memory
+// pools, kernels' attributes) is remembered under it.
+drb_status current_context(unsigned long long *id);
+// Calls `setup` in each context of device `dev` before what needs it first;
+// done: zero-initialised, one per setup.
+template <class F>
+drb_status once_per_context(std::atomic<unsigned long long> (&done)[64], int dev, F setup) {
+  unsigned long long id = 0;
+  DRB_TRY(current_context(&id));
+  if (dev < 64 && id != 0 && done[dev].load(std::memory_order_acquire) == id)
+    return DRB_OK;
+  DRB_TRY(setup()); // (makes the context)
+  DRB_TRY(current_context(&id));
+  if (dev < 64)
+    done[dev].store(id, std::memory_order_release);
+  return DRB_OK;
+}
+drb_status device_sms(int dev, int *sms);
 void scratch_free(void *p, cudaStream_t s);
 
 // ---- device buffers ----------------------------------------------------------

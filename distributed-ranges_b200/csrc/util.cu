@@ -1,6 +1,10 @@
 // util.cu -- small device kernels: layout transposes and element conversions
 // used at upload time and around multi-RHS calls.
+#include <cuda.h> // CUcontext, CUresult: types only; the library does not link libcuda
+
+#include <atomic>
 #include <cstdint>
+#include <map>
 #include <mutex>
 
 #include "drb_internal.cuh"
@@ -16,8 +20,54 @@ namespace drb {
 // largest scratch in flight (a few MB) and is kept until process exit.
 namespace {
 std::mutex g_pool_mu;
-cudaMemPool_t g_pool[64];
+std::map<unsigned long long, cudaMemPool_t> g_pool[64]; // per device, by context
+
+// The driver's context queries, through the runtime's entry-point lookup (the
+// library does not link libcuda itself).
+struct ContextQueries {
+  CUresult (*current)(CUcontext *) = nullptr;
+  CUresult (*id)(CUcontext, unsigned long long *) = nullptr;
+  ContextQueries() {
+    void *f1 = nullptr, *f2 = nullptr;
+    cudaDriverEntryPointQueryResult q1, q2;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f1, 12000, cudaEnableDefault,
+                                         &q1) != cudaSuccess ||
+        cudaGetDriverEntryPointByVersion("cuCtxGetId", &f2, 12000, cudaEnableDefault, &q2) !=
+            cudaSuccess ||
+        q1 != cudaDriverEntryPointSuccess || q2 != cudaDriverEntryPointSuccess)
+      return;
+    current = reinterpret_cast<decltype(current)>(f1);
+    id = reinterpret_cast<decltype(id)>(f2);
+  }
+};
 } // namespace
+
+drb_status current_context(unsigned long long *id) {
+  static const ContextQueries q;
+  if (!q.current || !q.id) {
+    set_error("the driver does not provide cuCtxGetCurrent/cuCtxGetId");
+    return DRB_ERR_CUDA;
+  }
+  CUcontext c = nullptr;
+  *id = 0;
+  if (q.current(&c) != CUDA_SUCCESS || !c)
+    return DRB_OK;
+  if (q.id(c, id) != CUDA_SUCCESS)
+    *id = 0;
+  return DRB_OK;
+}
+
+drb_status device_sms(int dev, int *sms) {
+  static std::atomic<int> known[64];
+  int n = dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (n == 0) {
+    DRB_CUDA_TRY(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    if (dev < 64)
+      known[dev].store(n, std::memory_order_relaxed);
+  }
+  *sms = n;
+  return DRB_OK;
+}
 
 drb_status scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
   int dev = 0;
@@ -29,7 +79,10 @@ drb_status scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
   cudaMemPool_t pool;
   {
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    if (!g_pool[dev]) {
+    unsigned long long ctx = 0;
+    DRB_TRY(current_context(&ctx));
+    auto known = ctx ? g_pool[dev].find(ctx) : g_pool[dev].end();
+    if (known == g_pool[dev].end()) {
       cudaMemPoolProps props = {};
       props.allocType = cudaMemAllocationTypePinned;
       props.location.type = cudaMemLocationTypeDevice;
@@ -38,9 +91,10 @@ drb_status scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
       DRB_CUDA_TRY(cudaMemPoolCreate(&created, &props));
       uint64_t keep = UINT64_MAX;
       DRB_CUDA_TRY(cudaMemPoolSetAttribute(created, cudaMemPoolAttrReleaseThreshold, &keep));
-      g_pool[dev] = created;
+      DRB_TRY(current_context(&ctx));
+      known = g_pool[dev].insert_or_assign(ctx, created).first;
     }
-    pool = g_pool[dev];
+    pool = known->second;
   }
   DRB_CUDA_TRY(cudaMallocFromPoolAsync(p, bytes ? bytes : 16, pool, s));
   return DRB_OK;
