@@ -973,6 +973,17 @@ drb_status drb_csr_cg(drb_csr_t A, const void *b, void *x, int64_t max_iters, do
   return cg_solve(*A, b, x, max_iters, rtol, info, static_cast<cudaStream_t>(stream));
 }
 
+drb_status drb_csr_cg_set_wait(drb_csr_t A, uint64_t start_ns, int32_t stall_cta) {
+  clear_error();
+  if (!A)
+    return invalid("A is NULL");
+  if (stall_cta < -1)
+    return invalid("stall_cta < -1");
+  A->cg_start_ns = start_ns ? start_ns : kCgStartNs;
+  A->cg_stall_cta = stall_cta;
+  return DRB_OK;
+}
+
 drb_status drb_dot(int64_t n, const void *a, const void *b, drb_dtype dtype,
                    double *out, void *stream) {
   clear_error();

@@ -23,6 +23,7 @@
 // at its first instruction.  Vectors are the matrix's value type (f32 / f64);
 // the scalars are f64.
 #include <cmath>
+#include <condition_variable>
 #include <mutex>
 
 #include "cg_state.cuh"
@@ -37,7 +38,41 @@ constexpr int kCgNT = 256;
 constexpr int kCgGrid = 148 * 3;
 constexpr int kCgMinBlocks = 3;
 constexpr int kCgBlock = 8;  // iterations per graph replay
-std::mutex g_resident_mu[64];
+
+// One-launch solves of a device run at the same time while their CTAs fit its
+// SMs, one each, in the order of the calls: two grids that are each partly
+// resident would wait for one another.
+struct Turns {
+  std::mutex mu;
+  std::condition_variable freed;
+  uint64_t next = 0, serving = 0;
+  int used = 0; // CTAs of the solves that run
+};
+Turns g_turns[64];
+
+class Turn { // held while a solve is on the GPU
+public:
+  Turn(Turns &t, int ctas, int sms) : t_(t), ctas_(ctas) {
+    std::unique_lock<std::mutex> lock(t_.mu);
+    const uint64_t mine = t_.next++;
+    t_.freed.wait(lock,
+                  [&] { return t_.serving == mine && (t_.used == 0 || t_.used + ctas <= sms); });
+    t_.serving++;
+    t_.used += ctas;
+    t_.freed.notify_all();
+  }
+  ~Turn() {
+    std::lock_guard<std::mutex> lock(t_.mu);
+    t_.used -= ctas_;
+    t_.freed.notify_all();
+  }
+  Turn(const Turn &) = delete;
+  Turn &operator=(const Turn &) = delete;
+
+private:
+  Turns &t_;
+  int ctas_;
+};
 } // namespace
 
 struct CgPlan {
@@ -348,13 +383,36 @@ void report(const CgState &h, drb_cg_info *info) {
   info->breakdown = h.done == kBreakdown;
 }
 
-// Waits for the one-launch loop, whose first launch is queued, and launches it
-// again while the solve runs.
+// The solve in launches of the one-launch loop, until it has ended or one of them
+// could not run (*done = kRunning; *started: the state, x, r and p are those of
+// an iteration's start, else as before the call).
 template <class T>
-drb_status finish_resident(Csr &A, CgPlan &C, const T *b, T *x, double rtol, int64_t max_iters,
-                           drb_cg_info *info, cudaStream_t s) {
+drb_status solve_resident(Csr &A, CgPlan &C, const T *b, T *x, double rtol, int64_t max_iters,
+                          int *done, bool *started, cudaStream_t s) {
   auto *st = C.state.as<CgState>();
+  *done = kRunning;
+  *started = false;
+  int ctas = 0, sms = 0;
+  DRB_TRY(cg_resident_grid<T>(A, &ctas));
+  DRB_TRY(device_sms(A.device, &sms));
+  if (!C.sync.p)
+    DRB_TRY(C.sync.alloc(cg_resident_sync_bytes()));
+  // earlier work of the stream is waited for before the turn is taken, not
+  // during it (the call synchronises anyway)
+  const cudaError_t e = cudaStreamQuery(s);
+  if (e == cudaErrorNotReady) {
+    cudaGetLastError();
+    DRB_CUDA_TRY(cudaStreamSynchronize(s));
+  } else {
+    DRB_CUDA_TRY(e);
+  }
+  Turn turn(g_turns[A.device < 64 ? A.device : 0], ctas, sms);
   for (;;) {
+    bool launched = false;
+    DRB_TRY(cg_resident_launch<T>(A, b, x, C.r.as<T>(), C.p.as<T>(), C.q.as<T>(), st, C.sync.p,
+                                  rtol, max_iters, !*started, &launched, s));
+    if (!launched)
+      return DRB_OK;
     // one host round trip: the state and the error word behind the launch
     int *err = reinterpret_cast<int *>(&C.host[1]);
     DRB_CUDA_TRY(cudaMemcpyAsync(&C.host[0], st, sizeof(CgState), cudaMemcpyDeviceToHost, s));
@@ -363,17 +421,18 @@ drb_status finish_resident(Csr &A, CgPlan &C, const T *b, T *x, double rtol, int
     DRB_CUDA_TRY(cudaStreamSynchronize(s));
     if (*err != 0)
       return pipe_check(A, s); // reports and clears it
+    if (C.host[0].done == kNotStarted) {
+      if (*started) { // the loop that goes on reads the word
+        const int running = kRunning;
+        DRB_CUDA_TRY(cudaMemcpy(&st->done, &running, sizeof(int), cudaMemcpyHostToDevice));
+      }
+      return DRB_OK;
+    }
+    *started = true;
     if (C.host[0].done != kRunning)
       break;
-    bool launched = false;
-    DRB_TRY(cg_resident_launch<T>(A, b, x, C.r.as<T>(), C.p.as<T>(), C.q.as<T>(), st, C.sync.p,
-                                  rtol, max_iters, false, &launched, s));
-    if (!launched) {
-      set_error("drb_csr_cg: the grid no longer fits the device");
-      return DRB_ERR_CUDA;
-    }
   }
-  report(C.host[0], info);
+  *done = C.host[0].done;
   return DRB_OK;
 }
 
@@ -403,30 +462,25 @@ drb_status solve(Csr &A, const T *b, T *x, int64_t max_iters, double rtol,
   double *partials = C.scratch.as<double>();
   int *ticket = reinterpret_cast<int *>(partials + 2 * kCgGrid);
 
-  bool resident = cg_resident_wanted(A);
-  // One such solve at a time on a device: two grids that are each partly
-  // resident would wait for one another.  (Held until the solve has ended; the
-  // call synchronises anyway.)
-  std::unique_lock<std::mutex> alone(g_resident_mu[A.device < 64 ? A.device : 0],
-                                     std::defer_lock);
-  if (resident) {
-    alone.lock();
-    if (!C.sync.p)
-      DRB_TRY(C.sync.alloc(cg_resident_sync_bytes()));
-    DRB_TRY(cg_resident_launch<T>(A, b, x, C.r.as<T>(), C.p.as<T>(), C.q.as<T>(), st, C.sync.p,
-                                  rtol, max_iters, true, &resident, s));
-    if (resident)
-      return finish_resident<T>(A, C, b, x, rtol, max_iters, info, s);
-    alone.unlock();
+  bool started = false;
+  if (cg_resident_wanted(A)) {
+    int done = kRunning;
+    DRB_TRY(solve_resident<T>(A, C, b, x, rtol, max_iters, &done, &started, s));
+    if (done != kRunning) {
+      report(C.host[0], info);
+      return DRB_OK;
+    }
   }
   DRB_TRY(fused_scratch(A)); // allocated before any capture
 
-  // r = b - A x0, p = r
-  DRB_TRY(spmv_pipe_launch(A, x, C.q.p, s));
-  cg_init<T><<<cg_grid(n), kCgNT, 0, s>>>(n, b, C.q.as<T>(), C.r.as<T>(), C.p.as<T>(), st,
-                                          rtol, max_iters, partials, ticket);
-  note_launch();
-  DRB_CUDA_TRY(cudaGetLastError());
+  if (!started) {
+    // r = b - A x0, p = r
+    DRB_TRY(spmv_pipe_launch(A, x, C.q.p, s));
+    cg_init<T><<<cg_grid(n), kCgNT, 0, s>>>(n, b, C.q.as<T>(), C.r.as<T>(), C.p.as<T>(), st,
+                                            rtol, max_iters, partials, ticket);
+    note_launch();
+    DRB_CUDA_TRY(cudaGetLastError());
+  }
   if (C.gx != x || C.gen != A.pipe.gen || !C.exec)
     DRB_TRY(capture_block<T>(A, C, x));
 

@@ -27,10 +27,19 @@
 // measured 3.9 us a sum, 1.9 through CTA 0, 2.3 by a counter and a second
 // read; 8 CTAs: 0.9 direct, 1.6 through CTA 0).  Sums are added in CTA order:
 // the same bits everywhere, repeatable.  The barrier is a counter with one
-// polling thread per CTA (1.3 us; a flag per CTA read by all: 5.1).  Every wait
-// gives up after ten seconds of %globaltimer (DRB_ERR_TIMEOUT in the handle's
-// error word) and ends the launch: long enough for CTAs that wait for another
-// stream's kernel to leave their SM.
+// polling thread per CTA (1.3 us; a flag per CTA read by all: 5.1).
+//
+// The CTAs wait for one another, so all have to be resident: a cooperative launch,
+// which was seen to start only when all its CTAs fit beside the kernels of other
+// streams.  Should some start without the others all the same (other processes
+// under MPS), until the first exchange ends, which changes nothing that counts,
+// a wait of more than start_ns (100 ms) ends the launch, and the host goes on
+// with a kernel per step.  All CTAs agree
+// on it through one word: each counts itself in as it starts, and giving up is a
+// compare-and-swap that succeeds only while the count is short; a CTA that starts
+// after it leaves at once.  From then on all CTAs run, and a wait that takes ten
+// seconds of %globaltimer all the same is an error (DRB_ERR_TIMEOUT in the
+// handle's error word).
 #include <algorithm>
 
 #include "drb_internal.cuh"
@@ -69,7 +78,11 @@ template <class T> struct ResArgs {
   int nres;  // vectors held in shared memory: r, q, x, p in this order
   int first; // this launch starts the solve
   float keep; // share of the matrix that L2 is asked to keep between iterations
+  unsigned *start;   // CTAs that started; kGaveUp
+  uint64_t start_ns; // limit of the wait for them
+  int stall_cta;     // failure-detection hook: this CTA stays away (-1: none)
 };
+constexpr unsigned kGaveUp = 0x80000000u;
 
 __device__ __forceinline__ double warp_down(double v) {
 #pragma unroll
@@ -103,16 +116,50 @@ template <int NT> struct Grid {
   double *s_red;  // [W]
   double *s_sum;  // [kResMaxCtas / 32]
   int *s_stop;
+  unsigned *start;
+  uint64_t start_ns;
+  CgState *st;
   unsigned epoch = 0, arrived = 0; // exchanges, barrier arrivals so far
 
+  // Thread 0 counts the CTA in as it starts (the answer, in `ticket`, is not
+  // waited for until the first exchange) ...
+  unsigned ticket = 0;
+  __device__ void enter() { ticket = atomicAdd(start, 1u); }
+  // ... and before it takes part in one finds out: false, the others have given up.
+  __device__ bool entered() {
+    const bool in = !(ticket & kGaveUp);
+    __threadfence(); // counted before its sum can be seen
+    return in;
+  }
+  // After start_ns without all CTAs: true when the launch is given up.
+  __device__ bool give_up() {
+    unsigned v = atomicAdd(start, 0u);
+    while (!(v & kGaveUp) && v < gridDim.x) {
+      const unsigned was = atomicCAS(start, v, v | kGaveUp);
+      if (was == v) {
+        st->done = kNotStarted;
+        v |= kGaveUp;
+      } else {
+        v = was;
+      }
+    }
+    return v & kGaveUp;
+  }
   // One step of a wait: true when it has to be given up.
   __device__ bool expired(uint64_t &t0, int spins) {
     if ((spins & 63) != 63) // (reading the timer takes as long as a poll)
       return false;
-    if (spins == 63)
+    if (spins == 63) {
       t0 = tma::globaltimer();
-    else if (tma::globaltimer() - t0 > kResWaitNs)
-      atomicExch(err, DRB_ERR_TIMEOUT);
+    } else {
+      const uint64_t waited = tma::globaltimer() - t0;
+      if (epoch == 1 && waited > start_ns && give_up()) {
+        *s_stop = 1;
+        return true;
+      }
+      if (waited > kResWaitNs)
+        atomicExch(err, DRB_ERR_TIMEOUT);
+    }
     if (!*(volatile int *)err)
       return false;
     *s_stop = 1;
@@ -158,8 +205,10 @@ template <int NT> struct Grid {
       if (lane == 0) {
         if (G == 1)
           s_sum[0] = t;
-        else
+        else if (epoch > 1 || entered())
           publish(slot + blockIdx.x, t, epoch);
+        else
+          *s_stop = 1;
       }
     }
     const bool reads = G > 1 && (G <= kResDirect || blockIdx.x == 0);
@@ -175,13 +224,14 @@ template <int NT> struct Grid {
       s_sum[0] = collect(copies + (blockIdx.x % kResCopies) * 8);
     }
     __syncthreads();
+    const bool complete = *(volatile int *)s_stop == 0; // (else there is no total)
     double t = 0.0;
     for (int i = 0; i < np; i++)
       t += s_sum[i];
     total = t;
-    if (G > kResDirect && blockIdx.x == 0 && threadIdx.x < kResCopies)
+    if (G > kResDirect && blockIdx.x == 0 && threadIdx.x < kResCopies && complete)
       publish(copies + threadIdx.x * 8, t, epoch);
-    return *(volatile int *)s_stop == 0;
+    return complete;
   }
 
   // Global writes of every thread before are seen by every thread after.
@@ -230,13 +280,20 @@ __global__ void __launch_bounds__(NT, 1) cg_resident(const ResArgs<T> a) {
   T *const pg = a.p + row0;
   T *const vp = a.nres > 3 ? sm + 3 * vs : pg;
   const int64_t obase = a.off[s0];
-  if (tid == 0)
-    s_stop = 0;
+  Grid<NT> G{a.slots, a.count, a.err, s_red, s_sum, &s_stop, a.start, a.start_ns, a.st};
+  if (tid == 0) {
+    s_stop = (int)blockIdx.x == a.stall_cta;
+    if (!s_stop)
+      G.enter();
+    else if (gridDim.x == 1)
+      a.st->done = kNotStarted;
+  }
   for (int i = tid; i <= nsl; i += NT)
     soff[i] = (int)(a.off[s0 + i] - obase);
-  Grid<NT> G{a.slots, a.count, a.err, s_red, s_sum, &s_stop};
   const uint64_t pol = a.keep > 0.0f ? ptx::policy_keep(a.keep) : ptx::policy_evict_first();
   __syncthreads();
+  if (s_stop)
+    return;
 
   // The matrix runs ahead of its use: a slice's first K entries per row load
   // while the previous slice's gathers are in flight, those of the warp's first
@@ -428,7 +485,7 @@ __global__ void __launch_bounds__(NT, 1) cg_resident(const ResArgs<T> a) {
 }
 
 constexpr size_t kSyncBytes =
-    (2 * kResMaxCtas + 2 * kResCopies * 8) * sizeof(ulonglong2) + sizeof(unsigned);
+    (2 * kResMaxCtas + 2 * kResCopies * 8) * sizeof(ulonglong2) + 2 * sizeof(unsigned);
 
 template <class T> struct ResShape {
   const void *kernel = nullptr;
@@ -477,16 +534,30 @@ bool cg_resident_wanted(const Csr &A) {
 
 size_t cg_resident_sync_bytes() { return kSyncBytes; }
 
+template <class T> drb_status shape_of(const Csr &A, ResShape<T> &S) {
+  DRB_TRY((res_shape<T, kResNT>(A, S)));
+  if constexpr (sizeof(T) == 4)
+    if (S.cap >= kResManySlices)
+      DRB_TRY((res_shape<T, kResNTMany>(A, S)));
+  return DRB_OK;
+}
+
+template <class T> drb_status cg_resident_grid(const Csr &A, int *ctas) {
+  ResShape<T> S;
+  DRB_TRY(shape_of<T>(A, S));
+  *ctas = S.grid;
+  return DRB_OK;
+}
+template drb_status cg_resident_grid<float>(const Csr &, int *);
+template drb_status cg_resident_grid<double>(const Csr &, int *);
+
 template <class T>
 drb_status cg_resident_launch(Csr &A, const T *b, T *x, T *r, T *p, T *q, CgState *st,
                               void *sync, double rtol, int64_t max_iters, bool first,
                               bool *launched, cudaStream_t s) {
   *launched = false;
   ResShape<T> S;
-  DRB_TRY((res_shape<T, kResNT>(A, S)));
-  if constexpr (sizeof(T) == 4)
-    if (S.cap >= kResManySlices)
-      DRB_TRY((res_shape<T, kResNTMany>(A, S)));
+  DRB_TRY(shape_of<T>(A, S));
   ResArgs<T> a;
   a.vals = A.sell.vals.as<T>();
   a.cols = A.sell.cols.as<int>();
@@ -501,6 +572,9 @@ drb_status cg_resident_launch(Csr &A, const T *b, T *x, T *r, T *p, T *q, CgStat
   a.st = st;
   a.slots = static_cast<ulonglong2 *>(sync);
   a.count = reinterpret_cast<unsigned *>(a.slots + 2 * kResMaxCtas + 2 * kResCopies * 8);
+  a.start = a.count + 1;
+  a.start_ns = A.cg_start_ns;
+  a.stall_cta = A.cg_stall_cta;
   a.err = A.pipe.err.as<int>();
   a.rtol = rtol;
   a.max_iters = max_iters;

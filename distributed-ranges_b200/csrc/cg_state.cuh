@@ -9,7 +9,13 @@
 
 namespace drb {
 
-enum : int { kRunning = 0, kConverged = 1, kBreakdown = 2, kMaxIters = 3 };
+enum : int {
+  kRunning = 0,
+  kConverged = 1,
+  kBreakdown = 2,
+  kMaxIters = 3,
+  kNotStarted = 4, // one-launch loop: its CTAs did not all get an SM; nothing has changed
+};
 
 struct CgState {
   double rr;   // r.r of the current residual
@@ -44,11 +50,15 @@ inline float resident_keep(int64_t matrix_bytes, int64_t vector_bytes) {
 }
 
 bool cg_resident_wanted(const Csr &A);
+// CTAs of such a launch (all of them want an SM at once).
+template <class T> drb_status cg_resident_grid(const Csr &A, int *ctas);
 size_t cg_resident_sync_bytes();
 // One launch of the loop (at most 1024 iterations; `first`: from x, else from
 // the state, r and p that the previous launch left).  *launched = false when
 // the grid cannot be resident at once.  sync: cg_resident_sync_bytes() of
-// device memory.  A device-side timeout is left in the handle's error word.
+// device memory.  A device-side timeout is left in the handle's error word;
+// kNotStarted in the state: CTAs that started waited CgWait::start_ns for others
+// that other kernels kept from an SM, and the launch ended without an effect.
 template <class T>
 drb_status cg_resident_launch(Csr &A, const T *b, T *x, T *r, T *p, T *q, CgState *st,
                               void *sync, double rtol, int64_t max_iters, bool first,

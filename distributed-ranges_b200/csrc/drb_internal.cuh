@@ -238,11 +238,17 @@ struct BatchDeleter {
   void operator()(Batch *p) const;
 };
 
+// How long the CTAs of a one-launch conjugate-gradient solve wait for all of them
+// to be on the GPU (cg_resident.cu).
+constexpr uint64_t kCgStartNs = 100000000;
+
 struct Csr {
   int device = 0;
   int64_t m = 0, n = 0, nnz = 0;
   int64_t max_row = 0; // nonzeros in the longest row
   int64_t long_nnz = 0; // nonzeros in rows longer than kLongRowNnz
+  uint64_t cg_start_ns = kCgStartNs; // drb_csr_cg_set_wait
+  int cg_stall_cta = -1;
   drb_dtype value_type = DRB_F32; // caller's element type
   drb_dtype storage = DRB_F32;    // device element type
   int cbytes = 4, rbytes = 4;     // stored index widths

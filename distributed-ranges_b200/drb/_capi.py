@@ -123,6 +123,7 @@ DRB_SYMBOLS = [
     ("drb_reduce", _st, [_i64, _vp, _i32, _i32, _vp, _vp, _vp]),
     ("drb_iota", _st, [_i64, _vp, _i32, _i64, _vp]),
     ("drb_fill", _st, [_i64, _vp, _i32, _vp, _vp]),
+    ("drb_csr_cg_set_wait", _st, [_vp, C.c_uint64, _i32]),
     ("drb_csr_cg", _st, [_vp, _vp, _vp, _i64, C.c_double, C.POINTER(CgInfo), _vp]),
     ("drb_read_matrix_market", _st, [C.c_char_p, _i32, C.POINTER(CsrHost)]),
     ("drb_csr_host_free", None, [C.POINTER(CsrHost)]),

@@ -394,15 +394,21 @@ drb_status drb_fill(int64_t n, void *x, drb_dtype dtype, const void *value,
  *   repeat: q = A p;  alpha = rr / p.q;  x += alpha p;  r -= alpha q;
  *           rr' = r.r;  stop if rr' <= rtol^2 b.b;  p = r + (rr'/rr) p
  * Scalars stay on the device (f64).  A matrix with short, regular rows (a
- * sliced-ELL copy) and 1024 to 3,670,016 rows is solved by one cooperative
- * launch per 1024 iterations, which wants every SM: such solves take turns on
- * a device.  Any other loop is replayed from a CUDA graph in blocks of 8
- * iterations (the SpMV carries p.q in its epilogue, the x/r update r.r) with
- * one small device-to-host read per block; iterations after convergence
- * return at once.  Stops on
- * convergence, at max_iters updates, or on breakdown (p.q <= 0 or not finite:
- * A is not SPD; x is left as it was before that iteration).  The call
- * synchronises `stream`. */
+ * sliced-ELL copy) and 993 (32 slices of 32) to 3,670,016 rows is solved by one
+ * cooperative launch per 1024 iterations, of one CTA per SM or, under 75,776
+ * rows, per 512 rows.  Such solves run at the same time as far as
+ * their CTAs fit the SMs and else take turns, in the order of the calls, once
+ * earlier work of their streams is done.  A solve starts when all its CTAs fit beside
+ * other streams' kernels; should CTAs be kept from an SM by more than 100 ms after the
+ * first, the solve goes on as any other does.  That is a CUDA
+ * graph of 8 iterations, replayed (the SpMV carries p.q in its epilogue, the
+ * x/r update r.r) with one small device-to-host read per block; iterations
+ * after convergence return at once.  Both forms are repeatable, but add p.q and
+ * r.r in different orders, so their last bits differ.  Stops on convergence, at
+ * max_iters updates, or on breakdown (p.q <= 0 or not finite: A is not SPD; x
+ * is left as it was before that iteration).  DRB_ERR_TIMEOUT: CTAs that all ran
+ * waited ten seconds for one another; x is then part way through an update.  The
+ * call synchronises `stream`. */
 typedef struct {
   int64_t iterations;   /* updates applied to x                    */
   double residual_norm; /* ||r|| of the recurrence at exit          */
@@ -412,6 +418,11 @@ typedef struct {
 } drb_cg_info;
 drb_status drb_csr_cg(drb_csr_t A, const void *b, void *x, int64_t max_iters,
                       double rtol, drb_cg_info *info, void *stream);
+/* Failure detection (no counterpart in the reference).  Later one-launch solves
+ * of the handle wait start_ns nanoseconds for all CTAs (0 = the default, 100
+ * ms), and with stall_cta >= 0 that CTA stays away, so the wait runs out.
+ * stall_cta = -1 restores normal launches. */
+drb_status drb_csr_cg_set_wait(drb_csr_t A, uint64_t start_ns, int32_t stall_cta);
 
 /* ---- ingest ----------------------------------------------------------------
  * drb_read_matrix_market replaces dr::read_csr<T, I>(path, one_indexed)
