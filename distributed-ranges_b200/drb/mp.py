@@ -405,10 +405,11 @@ class distributed_sparse_matrix:
                                     capi.DRB_COL_MAJOR, _stream(stream)))
         if y is res:
             return
-        if isinstance(res, np.ndarray) and res.dtype == _NP_OF_TORCH[y.dtype] and \
+        if type(res) is np.ndarray and res.dtype == _NP_OF_TORCH[y.dtype] and \
                 res.flags.c_contiguous and res.flags.writeable and \
                 res.size == m * width > 0:
-            # straight into res, with no host tensor in between
+            # straight into res, with no host tensor in between (subclasses, masked
+            # arrays for one, have assignments of their own)
             st = _stream(stream)
             check(capi.lib.drb_memcpy(_ptr(res), _ptr(y), res.nbytes, 1, st))
             check(capi.lib.drb_stream_synchronize(st))

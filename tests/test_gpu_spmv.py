@@ -851,3 +851,18 @@ def test_sell_autotune_keeps_a_valid_choice(mp):
     a.gemv_device(xt, yt)
     y64 = oracle.gemv_row(rp, ci, v, x, m, m, 1, oracle.ACC_LD)
     assert rel_err(yt.cpu().numpy(), y64, oracle.absdot(rp, ci, v, x, m, m)) <= 1e-12
+
+
+def test_result_into_a_masked_array_is_assigned(mp):
+    """Assigning to a masked array unmasks it: a result written past that
+    assignment would stay masked."""
+    import drb
+    rp, ci, v = drb.gen.uniform_rows_csr(50, 50, lo=1, hi=5, seed=1, value_dtype=np.float64)
+    a = mp.distributed_sparse_matrix(mp.csr_matrix_view(v, rp, ci, (50, 50)), 0)
+    b = mp.broadcasted_vector()
+    b.broadcast_data(50, 0, np.ones(50))
+    plain = np.zeros(50)
+    mp.gemv(0, plain, a, b)
+    masked = np.ma.masked_array(np.zeros(50), mask=np.arange(50) % 2 == 0)
+    mp.gemv(0, masked, a, b)
+    assert not np.ma.getmaskarray(masked).any() and np.array_equal(masked.data, plain)
