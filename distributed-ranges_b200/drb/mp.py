@@ -44,13 +44,20 @@ _STORAGE_TORCH = {capi.DRB_F32: torch.float32, capi.DRB_F64: torch.float64,
 # The wrappers below run on every call of kernels that take a few microseconds,
 # so they pass plain integers for pointers and streams (ctypes converts them by
 # the argument types) and read torch's current stream without building a Stream
-# object: 6 us less of host time a call.
+# object: 6 us less of host time a call.  The two calls for that are private to
+# torch: without them, the public one.
+_RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_DEVICE = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream(stream=None) -> int:
     if stream is not None:
         return stream.cuda_stream
+    if _RAW_STREAM is None or _DEVICE is None:
+        return torch.cuda.current_stream().cuda_stream
     if not torch.cuda.is_initialized():
         torch.cuda.init()
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return _RAW_STREAM(_DEVICE())
 
 
 def _ptr(t):

@@ -132,3 +132,13 @@ def test_dense_products_and_reductions_feed_one_another(mp, dtype, n, k):
             mp.reduce(top, 0.0, max, out=last)
         return [x[0], x[1], dots, top, last], 40, one
     same_chained_and_paused(make)
+
+
+def test_current_stream_without_the_private_calls(mp, monkeypatch):
+    side = torch.cuda.Stream()
+    for stream in (torch.cuda.default_stream(), side):
+        with torch.cuda.stream(stream):
+            fast = mp._stream()
+            with monkeypatch.context() as patch:
+                patch.setattr(mp, "_RAW_STREAM", None)
+                assert mp._stream() == fast == stream.cuda_stream
