@@ -369,7 +369,8 @@ drb_status build_typed(Csr &A, cudaStream_t s) {
                                cudaMemcpyDeviceToHost, s));
   DRB_CUDA_TRY(cudaStreamSynchronize(s));
   keys_out.release();
-  T.long_nnz = long_row_nnz(T.m, cp.data(), sizeof(RI));
+  int64_t longest = 0;
+  row_lengths(T.m, cp.data(), sizeof(RI), &longest, &T.long_nnz);
   DRB_TRY(build_plan(T.plan, T.m, cp.data(), sizeof(RI),
                      plan_group(dtype_bytes(T.storage), T.cbytes), 0, 0, 0));
   DRB_TRY(build_pipe_plan(T.pipe, T.m, cp.data(), sizeof(RI),

@@ -334,9 +334,7 @@ drb_status drb_csr_create(drb_csr_t *out, int64_t m, int64_t n, int64_t nnz,
   DRB_TRY(upload(A->vals.p, vb, values, vb_in, nnz, on_dev,
                  storage == DRB_BF16, s));
   DRB_CUDA_TRY(cudaStreamSynchronize(s));
-  for (int64_t i = 0; i < m; i++)
-    A->max_row = std::max(A->max_row, rp_at(rp_h, ib, i + 1) - rp_at(rp_h, ib, i));
-  A->long_nnz = long_row_nnz(m, rp_h, ib);
+  row_lengths(m, rp_h, ib, &A->max_row, &A->long_nnz);
   DRB_TRY(build_plan(A->plan, m, rp_h, ib, plan_group(vb, A->cbytes), 0, 0, 0));
   DRB_TRY(build_pipe_plan(A->pipe, m, rp_h, ib, plan_group(vb, A->cbytes),
                           default_pipe_variant(*A), 0));

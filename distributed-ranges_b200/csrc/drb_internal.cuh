@@ -205,7 +205,8 @@ drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
 // autotuned, by its type, size and share of nonzeros in long rows.
 int default_pipe_variant(const Csr &A);
 constexpr int64_t kLongRowNnz = 256;
-int64_t long_row_nnz(int64_t m, const void *rowptr_host, int rbytes);
+void row_lengths(int64_t m, const void *rowptr_host, int rbytes, int64_t *longest,
+                 int64_t *long_nnz);
 // Elements per 16-byte vector group of a plan over values of vbytes and
 // column indices of cbytes.
 int plan_group(int vbytes, int cbytes);

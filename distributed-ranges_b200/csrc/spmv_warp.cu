@@ -60,16 +60,78 @@ int default_pipe_variant(const Csr &A) {
   return 256 | 1;
 }
 
-int64_t long_row_nnz(int64_t m, const void *rowptr_host, int rbytes) {
+namespace {
+
+template <class RI> void row_lengths(int64_t m, const RI *rowptr, int64_t *longest, int64_t *long_nnz) {
+  RI top = 0;
   int64_t total = 0;
   for (int64_t r = 0; r < m; r++) {
-    const int64_t len = rbytes == 4 ? (int64_t)((const int32_t *)rowptr_host)[r + 1] -
-                                          ((const int32_t *)rowptr_host)[r]
-                                    : ((const int64_t *)rowptr_host)[r + 1] -
-                                          ((const int64_t *)rowptr_host)[r];
-    total += len > kLongRowNnz ? len : 0;
+    const RI len = rowptr[r + 1] - rowptr[r];
+    top = std::max(top, len);
+    total += len > (RI)kLongRowNnz ? (int64_t)len : 0;
   }
-  return total;
+  *longest = (int64_t)top;
+  *long_nnz = total;
+}
+
+// Row r's range as build_pipe_plan cuts it: items of up to `tile` nonzeros from
+// an aligned start, wider rows in chunks.
+template <class RI>
+void cut_items(int64_t m, const RI *rowptr, int64_t G, int tile, int rows, std::vector<Item> &longi,
+               std::vector<Item> &tiles, std::vector<Chunk> &chunks, std::vector<int4> &splits) {
+  // about a quarter of an item stays empty at its end
+  tiles.reserve((size_t)((rowptr[m] - rowptr[0]) / tile * 5 / 4 + m / rows + 64));
+  int64_t r = 0;
+  while (r < m) {
+    const int64_t p0 = (int64_t)rowptr[r], a0 = p0 & ~(G - 1), p1 = (int64_t)rowptr[r + 1];
+    if (p1 - a0 > tile) {
+      // a row wider than one item: aligned chunks of `tile` elements
+      const int64_t nch = (p1 - a0 + tile - 1) / tile;
+      const int first = (int)chunks.size();
+      for (int64_t i = 0; i < nch; i++) {
+        Chunk c;
+        c.p0 = std::max(p0, a0 + i * tile);
+        c.p1 = std::min(p1, a0 + (i + 1) * tile);
+        c.row = (int32_t)r;
+        c.first = first;
+        c.count = (int32_t)nch;
+        c.counter = (int32_t)splits.size();
+        chunks.push_back(c);
+        Item it{};
+        it.p0 = c.p0;
+        it.len = (int32_t)(c.p1 - c.p0);
+        it.r0 = (int32_t)r;
+        it.nrows = 0;
+        it.chunk = first + (int32_t)i;
+        longi.push_back(it);
+      }
+      splits.push_back(make_int4((int)r, first, (int)nch, 0));
+      r++;
+      continue;
+    }
+    const int64_t end = std::min(m, r + rows);
+    int64_t r1 = r + 1;
+    while (r1 < end && (int64_t)rowptr[r1 + 1] - a0 <= tile)
+      r1++;
+    Item it{};
+    it.p0 = p0;
+    it.len = (int32_t)((int64_t)rowptr[r1] - p0);
+    it.r0 = (int32_t)r;
+    it.nrows = (int32_t)(r1 - r);
+    it.chunk = -1;
+    tiles.push_back(it);
+    r = r1;
+  }
+}
+
+} // namespace
+
+void row_lengths(int64_t m, const void *rowptr_host, int rbytes, int64_t *longest,
+                 int64_t *long_nnz) {
+  if (rbytes == 4)
+    row_lengths(m, static_cast<const int32_t *>(rowptr_host), longest, long_nnz);
+  else
+    row_lengths(m, static_cast<const int64_t *>(rowptr_host), longest, long_nnz);
 }
 
 drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
@@ -92,60 +154,23 @@ drb_status build_pipe_plan(PipePlan &plan, int64_t m, const void *rowptr_host,
   plan.tile = tile;
   plan.rows = rows;
   plan.group = group;
-  auto RP = [&](int64_t i) -> int64_t {
-    return rbytes == 4 ? (int64_t)((const int32_t *)rowptr_host)[i]
-                       : ((const int64_t *)rowptr_host)[i];
-  };
-  const int64_t G = group;
   std::vector<Item> longi, tiles;
   std::vector<Chunk> chunks;
   std::vector<int4> splits;
-  int64_t nsplit = 0;
-  int64_t r = 0;
-  while (r < m) {
-    const int64_t p0 = RP(r), a0 = p0 & ~(G - 1), p1 = RP(r + 1);
-    if (p1 - a0 > tile) {
-      // a row wider than one item: aligned chunks of `tile` elements
-      const int64_t nch = (p1 - a0 + tile - 1) / tile;
-      const int first = (int)chunks.size();
-      for (int64_t i = 0; i < nch; i++) {
-        Chunk c;
-        c.p0 = std::max(p0, a0 + i * tile);
-        c.p1 = std::min(p1, a0 + (i + 1) * tile);
-        c.row = (int32_t)r;
-        c.first = first;
-        c.count = (int32_t)nch;
-        c.counter = (int32_t)nsplit;
-        chunks.push_back(c);
-        Item it{};
-        it.p0 = c.p0;
-        it.len = (int32_t)(c.p1 - c.p0);
-        it.r0 = (int32_t)r;
-        it.nrows = 0;
-        it.chunk = first + (int32_t)i;
-        longi.push_back(it);
-      }
-      splits.push_back(make_int4((int)r, first, (int)nch, 0));
-      nsplit++;
-      r++;
-      continue;
-    }
-    int64_t r1 = r + 1;
-    while (r1 < m && r1 - r < rows && RP(r1 + 1) - a0 <= tile)
-      r1++;
-    Item it{};
-    it.p0 = p0;
-    it.len = (int32_t)(RP(r1) - p0);
-    it.r0 = (int32_t)r;
-    it.nrows = (int32_t)(r1 - r);
-    it.chunk = -1;
-    tiles.push_back(it);
-    r = r1;
-  }
+  if (rbytes == 4)
+    cut_items(m, static_cast<const int32_t *>(rowptr_host), group, tile, rows, longi, tiles, chunks,
+              splits);
+  else
+    cut_items(m, static_cast<const int64_t *>(rowptr_host), group, tile, rows, longi, tiles, chunks,
+              splits);
+  const int64_t nsplit = (int64_t)splits.size();
   // Interleave chunk items with whole-row items so every warp's share mixes
   // both kinds.
   std::vector<Item> all;
-  all.reserve(longi.size() + tiles.size());
+  if (longi.empty())
+    all.swap(tiles);
+  else
+    all.reserve(longi.size() + tiles.size());
   size_t a = 0, b = 0;
   const double ratio = tiles.empty() ? 0.0 : (double)longi.size() / (double)tiles.size();
   double acc = 0.0;
