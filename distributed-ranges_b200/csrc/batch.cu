@@ -287,9 +287,13 @@ __device__ __forceinline__ uint64_t x_pair(const XWords<XT, VEC> &o, int p) {
 // error terms cmp); the lane takes b, b + step, ... with UN gathers in
 // flight.  f32 sums of an even VEC run on packed pairs.  Places past the
 // lane's last nonzero multiply a repeated gather by 0, which makes a NaN of a
-// row's infinity: the caller takes plain sums that came out as one again with
-// UN = 1, which has no such places.  (Skipping them here cost 1.6%: rows of 8..64, f32,
-// k = 16 552 -> 561 us, k = 20 676 -> 688.)
+// row's infinity.  So f64 skips them, and f32 sums that came out as one are taken
+// again with UN = 1, which has no such places (kRepeats).  (Skipping cost f32 1.6%:
+// rows of 8..64, k = 16 552 -> 561 us, k = 20 676 -> 688; a second form of the
+// rows beside the first cost f64 up to 18%: 34 matrices of 4090 rows of 12..60,
+// k = 16, 151 -> 185 us.)  Compensated sums add 0 x: an infinity ends in their
+// error terms as NaN in any case.
+template <class V> constexpr bool kRepeats = sizeof(V) == 4;
 template <class V, class XT, int VEC, int UN, class A>
 __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
                                          int e, const XT *Xl, int ldx,
@@ -395,6 +399,8 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
     } else {
 #pragma unroll
       for (int u = 0; u < UN; u++) {
+        if (u > 0 && sizeof(A) == 8 && q + u * step >= e)
+          continue; // f64 skips them
 #pragma unroll
         for (int t = 0; t < VEC; t++)
           acc[t] = fma(vv[u], (x_at<XT, VEC, A>(xv[u], t)), acc[t]);
@@ -404,7 +410,7 @@ __device__ __forceinline__ void row_sums(uint32_t colS, uint32_t valS, int b,
 }
 
 // Any of a lane's sums is not a number.
-template <int VEC, class A> __device__ __forceinline__ bool any_nan(const A (&acc)[VEC]) {
+template <class A, int VEC> __device__ __forceinline__ bool any_nan(const A (&acc)[VEC]) {
   bool r = false;
 #pragma unroll
   for (int t = 0; t < VEC; t++)
@@ -425,6 +431,49 @@ __device__ __forceinline__ void merge_sum(A &acc, A &cmp, A acc2, A cmp2) {
   }
 }
 
+// The whole rows of one work item, R at a time, G slots each.
+template <class XT, class A> struct ShortUnit {
+  uint32_t colP, valP, rsP; // shared addresses of the columns, values, row offsets
+  int p0, nrows, R, grp, gs, G, KP, ldx;
+  bool active; // this lane has a slot and columns
+  const XT *Xl;
+  A *ytile; // this lane's first column of the item's tile of Y
+  int ystride;
+};
+
+// The rows' sums to the tile; true: one of this lane's is not a number.
+template <class V, class XT, int VEC, int UN, class A>
+__device__ __forceinline__ bool short_rows(const ShortUnit<XT, A> &w) {
+  bool nan = false;
+  for (int i0 = 0; i0 < w.nrows; i0 += w.R) {
+    const int i = i0 + w.grp;
+    A acc[VEC], cmp[VEC];
+#pragma unroll
+    for (int t = 0; t < VEC; t++)
+      acc[t] = cmp[t] = 0;
+    if (w.active && i < w.nrows) {
+      const int b = lds_s32(w.rsP + 4 * i) - w.p0, e = lds_s32(w.rsP + 4 * i + 4) - w.p0;
+      row_sums<V, XT, VEC, UN, A>(w.colP, w.valP, b + w.gs, e, w.Xl, w.ldx, w.G, acc, cmp);
+    }
+    if constexpr (kRepeats<V>)
+      nan |= any_nan(acc);
+    for (int dd = 1; dd < w.G; dd <<= 1) {
+#pragma unroll
+      for (int t = 0; t < VEC; t++) {
+        const A a2 = __shfl_xor_sync(0xffffffffu, acc[t], dd * w.KP);
+        const A c2 = Comp<V>::value ? __shfl_xor_sync(0xffffffffu, cmp[t], dd * w.KP) : A(0);
+        merge_sum<V>(acc[t], cmp[t], a2, c2);
+      }
+    }
+    if (w.active && w.gs == 0 && i < w.nrows) {
+#pragma unroll
+      for (int t = 0; t < VEC; t++)
+        w.ytile[i * w.ystride + t] = Comp<V>::value ? acc[t] + cmp[t] : acc[t];
+    }
+  }
+  __syncwarp();
+  return nan;
+}
 template <class V, class XT, int VEC, int UN>
 __global__ void __launch_bounds__(256, UN == 4 ? 3 : 2) batch_spmm(const BArgs a) {
   using A = typename AccOf<V>::type;
@@ -509,42 +558,12 @@ __global__ void __launch_bounds__(256, UN == 4 ? 3 : 2) batch_spmm(const BArgs a
       const uint32_t colP = colS + 4 * (p0 & 3);
       const uint32_t valP = valS + (uint32_t)sizeof(V) * (p0 & VOFF_MASK);
       const uint32_t rsP = wsm + a.rs_off + st * a.rs_stage + 4 * (r0 & 3);
-      auto rows = [&](auto in_flight) {
-        bool nan = false;
-        for (int i0 = 0; i0 < nrows; i0 += R) {
-          const int i = i0 + grp;
-          A acc[VEC], cmp[VEC];
-#pragma unroll
-          for (int t = 0; t < VEC; t++)
-            acc[t] = cmp[t] = 0;
-          if (con && row_on && i < nrows) {
-            const int b = lds_s32(rsP + 4 * i) - p0, e = lds_s32(rsP + 4 * i + 4) - p0;
-            row_sums<V, XT, VEC, in_flight.value, A>(colP, valP, b + gs, e, Xl, ldx, G, acc,
-                                                     cmp);
-          }
-          nan |= any_nan(acc);
-          for (int dd = 1; dd < G; dd <<= 1) {
-#pragma unroll
-            for (int t = 0; t < VEC; t++) {
-              const A a2 = __shfl_xor_sync(0xffffffffu, acc[t], dd * KP);
-              const A c2 =
-                  Comp<V>::value ? __shfl_xor_sync(0xffffffffu, cmp[t], dd * KP) : A(0);
-              merge_sum<V>(acc[t], cmp[t], a2, c2);
-            }
-          }
-          if (con && row_on && gs == 0 && i < nrows) {
-#pragma unroll
-            for (int t = 0; t < VEC; t++)
-              ytile[i * ystride + jj * VEC + t] = Comp<V>::value ? acc[t] + cmp[t] : acc[t];
-          }
-        }
-        __syncwarp();
-        return nan;
-      };
-      const bool nan = rows(std::integral_constant<int, UN>());
-      if constexpr (!Comp<V>::value)
+      const ShortUnit<XT, A> unit{colP, valP, rsP, p0, nrows, R, grp, gs, G, KP, ldx,
+                                  con && row_on, Xl, ytile + jj * VEC, ystride};
+      const bool nan = short_rows<V, XT, VEC, UN, A>(unit);
+      if constexpr (kRepeats<V>)
         if (__any_sync(0xffffffffu, nan))
-          rows(std::integral_constant<int, 1>());
+          short_rows<V, XT, VEC, 1, A>(unit);
       // the tile to Y, coalesced: lanes map (row, column) by powers of two
       const int kbv = min(KB, k - jb);
       if (a.row_major) {
@@ -590,7 +609,7 @@ __global__ void __launch_bounds__(256, UN == 4 ? 3 : 2) batch_spmm(const BArgs a
         }
       };
       row(std::integral_constant<int, UN>());
-      if constexpr (!Comp<V>::value)
+      if constexpr (kRepeats<V>)
         if (__any_sync(0xffffffffu, any_nan(acc)))
           row(std::integral_constant<int, 1>());
       for (int dd = 1; dd < S; dd <<= 1) {
