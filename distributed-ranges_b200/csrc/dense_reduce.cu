@@ -29,9 +29,8 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
 
 // One right-hand side: HBM-bound, A streamed once.  The work is cut into
 // steps of one row x 32 * U pieces (16 bytes, or single elements where A's rows
-// or x do not start on 16 bytes), 2 KB to 8 KB of a row, so a warp reads long
-// contiguous runs (page locality decides: one row per warp with 2 KB steps
-// streams at 6.9 TB/s on 32768^2 f32, four rows of 512 bytes at 4.9).
+// or x do not start on 16 bytes), 2 KB or 4 KB of a row, so a warp reads long
+// contiguous runs.
 // CTAs take equal consecutive shares of the steps (LOCAL: of the rows), their
 // warps equal shares of those.  A row that falls to one warp goes straight to y,
 // the parts of a row cut between warps meet in shared memory in step order, and
@@ -43,11 +42,11 @@ template <class V> __device__ __forceinline__ V warp_sum_d(V v) {
 // sums: one chain over its share of a row grew the error with the row (N(0, 1)
 // rows of 16384 columns, 2-norm over the result's: f32 2.6e-7, f64 4.9e-16, now
 // 1.3e-7 and 2.6e-16).
-// U pieces per lane and step: 8, but 4 for f32 rows under 32 KB and f64 rows under 4
-// KB, whose last step would be mostly empty (us, U = 4 / 8: f32 20000 x 500 9.8 /
-// 10.8, 4096^2 14.9 / 15.5, 8192^2 46.3 / 45.6, 24000^2 367 / 361, 32768^2 658 / 648;
-// f64 10000 x 500 10.0 / 10.8, 16384 x 128 5.7 / 7.6), and 16 single elements.
-template <class V> constexpr int64_t kLongRowBytes = sizeof(V) == 4 ? 32768 : 4096;
+// U pieces per lane and step: 8, but 4 for rows under 8 KB, whose last step would be
+// mostly empty (us, U = 4 / 8: f32 20000 x 500 10.2 / 11.7, 10000 x 2000 16.3 / 16.1, 4096^2
+// 13.2 / 12.6, 8192^2 43.3 / 42.5, 32768^2 622 / 606; f64 16384 x 128 6.3 / 7.9, 10000 x 500
+// 10.5 / 11.8, 16384 x 1000 23.7 / 24.0, 5000 x 4000 28.4 / 27.5), and 16 single elements.
+constexpr int64_t kLongRowBytes = 8192;
 constexpr int64_t kUneven = 48 * 1024;
 // CTAs per SM: as many as leave the registers for a step's loads to go out at once.
 // Rows of 16-byte pieces, us, 4 / 3 / 2: f32 8192^2 45.0 / 43.1 / 41.9 (0.99 of the
@@ -259,7 +258,7 @@ drb_status dense_row(int64_t m, int64_t n, const V *A, int64_t lda, const V *x, 
                    reinterpret_cast<uintptr_t>(x) % 16 == 0 && lda * sizeof(V) % 16 == 0;
   if (!vec)
     return dense_row_call<V, false, 16>(m, n, A, lda, x, y, s);
-  if (n * (int64_t)sizeof(V) < kLongRowBytes<V>)
+  if (n * (int64_t)sizeof(V) < kLongRowBytes)
     return dense_row_call<V, true, 4>(m, n, A, lda, x, y, s);
   return dense_row_call<V, true, 8>(m, n, A, lda, x, y, s);
 }
