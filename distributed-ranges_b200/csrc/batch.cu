@@ -203,8 +203,10 @@ __device__ __forceinline__ int clog2(int x) {
 // five or six where X does not stay in L2 either.  There rows are long chains of
 // rounds in few slots, and each round waits for its gathers: rows of 8..64, 0.5M
 // rows f32 k = 28 502 -> 392 us, k = 33 719 -> 543, f64 k = 20 795 -> 755, 1M rows
-// f32 k = 20 (X 80 MB) 738 -> 675; but 1.5M rows of 4..33 over an X of 37 MB, k =
-// 19, 364 -> 382, and with fewer lanes a slot more warps do better (f32 k = 12
+// f32 k = 20 (X 80 MB) 738 -> 675.  Five lanes, rows of 8..64, k = 20, by the size of X:
+// 36 MB 236 -> 231, 44 MB 275 -> 288, 52 MB 371 -> 365, 60 MB 478 -> 448; 37 MB with rows of
+// 4..33, k = 19, 364 -> 382; six lanes (k = 24), 44 MB 278 -> 266, 52 MB 337 -> 347, 60 MB
+// 457 -> 433.  And with fewer lanes a slot more warps do better (f32 k = 12
 // 202 -> 216, k = 16 547 -> 578, k = 8 144 -> 161), as with vectors of less than
 // 16 bytes (row-major k = 21 963 -> 1122).  Rows shorter than a round repeat
 // their last gather: mean rows of under kWideRow nonzeros keep 4.  BF16 storage

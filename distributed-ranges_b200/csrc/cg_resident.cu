@@ -14,8 +14,8 @@
 //   p = r + beta p      -> grid barrier (p is gathered by other CTAs next)
 //
 // Measured (64 iterations on a g x g Laplacian, us, launch per step -> here):
-// f64 g = 48 787 -> 491, 512 1455 -> 801, 1024 2386 -> 1347, 1448 3672 -> 2991,
-// 1800 5462 -> 4367; f32 300 1088 -> 720, 1024 2134 -> 1307, 1448 2979 -> 2202.
+// f64 g = 48 787 -> 478, 512 1455 -> 812, 1024 2386 -> 1339, 1448 3672 -> 2991,
+// 1800 5462 -> 4367; f32 300 1088 -> 680, 1024 2134 -> 1307, 1448 2979 -> 2151.
 // What is left at small sizes is the chain of three grid-wide steps (about 5 us
 // of 11 an iteration on all SMs), at large ones the matrix's bytes.
 //
@@ -527,8 +527,10 @@ template <class T, int NT> drb_status res_shape(const Csr &A, ResShape<T> &S) {
 
 bool cg_resident_wanted(const Csr &A) {
   // The sliced-ELL copy only (its rows map to threads one to one).  Solves of
-  // under 32 slices keep the graph: they are over in microseconds and their
-  // launch count is part of what the library reports.
+  // under 32 slices keep the graph, whose launches per iteration callers may
+  // count (drb_launch_count), although one launch is faster there too (40 iterations
+  // on a g x g Laplacian, f64, us, graph / one launch: g = 8 520 / 134, 16 509 / 133, 24
+  // 517 / 149, 31 577 / 180).
   return A.sell.on && A.sell.nslices >= 32 && A.m <= kResMaxRows;
 }
 

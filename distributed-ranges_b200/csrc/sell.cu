@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kSellNT)
 
 // The grid for `need` CTAs of work: all resident, the same number on every SM (the
 // slices are shared evenly whatever the grid).  With the launch overlapped, 131072
-// rows of 16, f32, 12.3 -> 10.3 us; 256 CTAs on 148 SMs had left most of them
+// rows of 16, f32, 12.3 -> 10.2 us; 256 CTAs on 148 SMs had left most of them
 // with one.
 template <class V, bool RESID, int NS, int K> int sell_grid(int dev, int64_t need) {
   static int cache[64][2];

@@ -34,7 +34,9 @@ using warpk::WarpResid;
 //   rows of 1..95, FP32, 1M rows 210 / 235; rows of 1..21, FP32, 0.8M rows, residual
 //     and backward 164 / 180.
 // 256 also stays for FP64 where x is in L2 and the matrix fills the GPU either
-// way (1.5M rows 167 / 166, 5M 490 / 505), for compensated sums (143 / 145) and
+// way (mean 20, 6M nonzeros 51.6 / 48.2, 10M 72.7 / 67.6, 12M 79.5 / 75.6, 15M 90.6 /
+// 90.8, 20M 115.5 / 113.6, 30M 161 / 163, 100M 490 / 505: the line at 12M lies at the end
+// of the gain), for compensated sums (143 / 145) and
 // for FP64 handles with an adjoint, whose abar runs on the same items (1.5M rows,
 // residual and backward 525 / 537; 6M 1894 / 1990).  The environment variable
 // DRB_SPMV_VARIANT="tile,skew" (e.g. "512,0") overrides it for handles

@@ -1,7 +1,7 @@
 """Dense gemv paths against the oracle at the edges of their tiles: the multi-RHS
-panel kernel (tiles of 64 or 32 rows x 128 columns in FP32, 128 x 32 in FP64,
-tiles cut between CTAs, 16-byte and single-element loads, blocks of at most 32
-right-hand sides) and the one-RHS row kernel (rows cut between warps and CTAs)."""
+panel kernel (tiles of 64 or 32 rows in FP32, 64 in FP64; chunks of 64 or 128
+columns in FP32, 32 or 64 in FP64; tiles cut between CTAs, aligned and shifted rows,
+blocks of at most 32 right-hand sides) and the one-RHS row kernel (rows cut between warps and CTAs)."""
 import numpy as np
 import pytest
 import torch
