@@ -82,7 +82,9 @@ template <class RI>
 void cut_items(int64_t m, const RI *rowptr, int64_t G, int tile, int rows, std::vector<Item> &longi,
                std::vector<Item> &tiles, std::vector<Chunk> &chunks, std::vector<int4> &splits) {
   // about a quarter of an item stays empty at its end
-  tiles.reserve((size_t)((rowptr[m] - rowptr[0]) / tile * 5 / 4 + m / rows + 64));
+  // (rows that were not validated: the count may be anything)
+  const int64_t nnz = std::max<int64_t>(0, (int64_t)rowptr[m] - (int64_t)rowptr[0]);
+  tiles.reserve((size_t)(nnz / tile * 5 / 4 + m / rows + 64));
   int64_t r = 0;
   while (r < m) {
     const int64_t p0 = (int64_t)rowptr[r], a0 = p0 & ~(G - 1), p1 = (int64_t)rowptr[r + 1];
